@@ -1,179 +1,567 @@
 // Symmetric eigensolver for one matrix per CTA (n <= kMaxN), replacing the reference's faer
 // `self_adjoint_eigen` (pm3-rs src/linalg.rs:221-263) on the SCF path:
-//   1. Householder reduction to tridiagonal form, the matrix held as a packed lower triangle
-//      (row-major: element (r, c), r >= c, at r(r+1)/2 + c) in shared memory (or global memory
-//      when it does not fit), a power-of-two group of threads per remaining row. Reflectors stay
-//      in the strictly-lower part of column i.
+//   1. Householder reduction to tridiagonal form with the matrix in registers (`tridiagonalize`).
+//      The reflectors go to global memory, one row of `V` per reduced column.
 //   2. Eigenvalues of the tridiagonal T by Sturm-count multisection, a group of lanes per
 //      eigenvalue, started from the previous SCF iteration's eigenvalues when given.
 //   3. Eigenvectors of T by twisted (N_r D_r N_r^T) factorisation, one thread per vector,
 //      on the unreduced block holding the eigenvalue (T is split where |e_i| <= 1000 eps ||T||,
 //      which separates exact degeneracies); members of a within-block cluster (gap below
 //      1e-7 ||T||) after the first are redone by inverse iteration with re-orthogonalisation.
-//   4. Back-transformation Z = Q Y, one warp per 2, 4 or 8 vectors held in registers (fewer rows
-//      per lane for smaller bases, more vectors).
+//   4. Back-transformation Z = Q Y, a group of lanes per 1 to 3 vectors held in registers, the
+//      reflectors staged through shared memory.
 // Only the eigenpairs the SCF needs are formed (the occupied block, plus one more value for
 // the frontier gap). Eigenvalues come out ascending, as the reference requires.
 #pragma once
+#include <type_traits>
+
 #include "cta_blas.cuh"
 
 namespace pm3gpu {
 
 constexpr int kMaxN = 256;          // largest basis handled by the per-CTA path
-constexpr int kRowT = kMaxN / 32;   // rows per lane in warp-per-row loops
 
-__device__ __forceinline__ int tri(int r) { return r * (r + 1) / 2; }
-__device__ __forceinline__ double ap_get(const double* A, int r, int c) { return r >= c ? A[tri(r) + c] : A[tri(c) + r]; }
+// The same shared-memory address, expressed from the shared window so that the compiler emits shared
+// accesses: the scratch pointers reach these functions through memory, where their address space is lost, and
+// generic loads and stores cost more (a reduced column of a 112 x 112 matrix 3.5k cycles against 2.4k).
+template <class T>
+__device__ __forceinline__ T* in_shared(T* p) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int off = (int)__cvta_generic_to_shared(p) - (int)__cvta_generic_to_shared(smem);
+  return reinterpret_cast<T*>(smem + off);
+}
 
 struct EigenScratch {
   double* d;     // [n] diagonal of T
   double* e;     // [n] off-diagonal of T (e[i] couples i, i+1); zeroed where T splits
   double* e2;    // [n] e^2
   double* tau;   // [n] reflector scales
-  double* v;     // [n] current reflector
-  double* p;     // [n] symv result
+  double* v;     // [n] eigenvector scratch (norm parts)
+  double* p;     // [n] eigenvector scratch (norm parts)
   double* lam;   // [n] eigenvalues (ascending)
   int* blk;      // [n+1] block starts (blk[0] = 0, ..., blk[nb] = n)
   int* nblk;     // [1]
-  int* vinfo;    // [n] per eigenvector: its block index
+  int* vinfo;    // [n] per eigenvector: its block index, and the twist index in the upper 16 bits
   double* red;   // reduction scratch (>= 8 * kWarps)
   double* misc;  // [8] broadcast scalars
+  double* sh;    // shared scratch: reduction vectors, then memory blocks, then staged reflectors
+  int sh_doubles;
 };
 
 // ---------------------------------------------------------------- 1. tridiagonalisation
-// Sum over the CTA with one barrier: `red` holds two alternating kWarps buffers, so a call may
-// overwrite the buffer two calls back without waiting (the previous call's barrier separates them).
-__device__ __forceinline__ double block_sum_alt(double v, double* red, int& parity) {
-  v = warp_sum(v);
-  double* buf = red + parity * kWarps;
-  parity ^= 1;
-  if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
+// Householder reduction with the matrix in registers. The matrix sits at the end of a frame of
+// 16 x 16 blocks (rows padded in front, so the columns retire from the first block on); thread
+// (ty, tx) of the 16 x 16 thread grid owns element (16 I + ty, 16 J + tx) of every lower block
+// (I >= J; a diagonal block holds both triangles). The last kRegB block columns live in registers;
+// the block columns before them (n > 16 kRegB only) live in private memory slots, shared memory
+// first, and are reduced by the same steps.
+// The reflector of column i is H = I - tau v v^T with v = x - beta e_{i+1}, x the column below the diagonal
+// (not scaled to v_{i+1} = 1): then A v = A x - beta A e_{i+1}, and the product A x needs neither the norm
+// nor the square root and division that beta and tau take, which overlap with it.
+// Two barriers per column. Between them one thread per row adds up the row's and the column
+// partial sums of A x, forms w, and applies the column's update to the next column in advance (its
+// old values were published with the partial sums), so that the next reflector is known when the
+// rest of the matrix is updated.
+// What bounds it: the chain of two barriers, shuffles and shared-memory round trips up to
+// n = 64 or so (about 1500 cycles a column), FP64 issue above (4 FMAs per element and column).
+constexpr int kRegB = 7;                        // block columns held in registers: 28 values a thread
+constexpr int kRegRows = 16 * kRegB;
+__host__ __device__ constexpr int frame_rows(int n) { return n <= kRegRows ? kRegRows : (n + 15) / 16 * 16; }
+// doubles of shared scratch `tridiagonalize` needs for bases up to n (vectors; memory blocks go after them)
+__host__ __device__ constexpr int tri_scratch(int n) { return 15 * frame_rows(n); }
+
+constexpr int kPart = 10;
+struct TriCtx {
+  double *xs, *vs, *ws, *raw, *rsum;  // [M] each
+  double *cpart;                      // [M][kPart]: column sums by warp (16-byte rows, no bank conflicts)
+  double *npart, *dpart;              // [kWarps]: squared norm of the next column, x^T A x
+  double *d, *e, *tau, *V;
+  int n, M, off;                         // basis size, frame rows, first used row of the frame
+};
+
+__device__ __forceinline__ constexpr int rblk(int I, int J) { return I * (I + 1) / 2 + J; }
+
+// Sums 8 values over the 16 lanes of a half-warp; lane l ends with the total of value l >> 1.
+__device__ __forceinline__ double sum16_of8(double (&v)[8], int lane) {
 #pragma unroll
-  for (int i = 0; i < kWarps; ++i) t += buf[i];
-  return t;
+  for (int k = 0; k < 4; ++k) {
+    const double send = (lane & 8) ? v[k] : v[k + 4], keep = (lane & 8) ? v[k + 4] : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double send = (lane & 4) ? v[k] : v[k + 2], keep = (lane & 4) ? v[k + 2] : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  }
+  const double send = (lane & 2) ? v[0] : v[1], keep = (lane & 2) ? v[1] : v[0];
+  const double r = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+__device__ __forceinline__ double sum16_of2(double (&v)[2], int lane) {  // lane l: value l >> 3
+  const double send = (lane & 8) ? v[0] : v[1], keep = (lane & 8) ? v[1] : v[0];
+  double r = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  r += __shfl_xor_sync(0xffffffffu, r, 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+// The same for 4 values: lane l ends with the total of value l >> 2.
+__device__ __forceinline__ double sum16_of4(double (&v)[4], int lane) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double send = (lane & 8) ? v[k] : v[k + 2], keep = (lane & 8) ? v[k + 2] : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const double send = (lane & 4) ? v[0] : v[1], keep = (lane & 4) ? v[1] : v[0];
+  double r = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
 }
 
-// Householder reduction (n <= kThreads). For column i, the m = n - i - 1 trailing rows get T
-// threads each (T the largest power of two with T m <= kThreads, at most a warp), so that late
-// columns, with few rows left, still keep the CTA busy. The T threads of row r split the
-// matrix-vector product (its row segment c <= r, then the column below it) and the rank-2
-// update of its row segment by interleaved columns, and combine the product by shuffles; the
-// first of them contributes its element of the next column to the next reflector's norm.
-// Three barriers per column. This sweep reduces columns [0, i_stop) of the n x n matrix and, with
-// `close`, writes the last diagonal and off-diagonal entries; d, e, tau are indexed from the
-// matrix's first row.
-__device__ __forceinline__ void householder_columns(int n, double* __restrict__ A, double* v, double* p, double* red, double* tau_out,
-                                    double* e_out, double* d_out, int i_stop, bool close) {
-  // scratch pointers in registers: the stores below go through generic pointers, which
-  // would otherwise force them to be re-read after every store
-  struct {
-    double *v, *p, *red, *tau, *e, *d;
-  } s = {v, p, red, tau_out, e_out, d_out};
-  const int t = threadIdx.x;
-  int parity = 0;
-  double xn2 = block_sum_alt(t >= 2 && t < n ? A[tri(t)] * A[tri(t)] : 0.0, s.red, parity);
-  for (int i = 0; i < i_stop; ++i) {
-    const double alpha = A[tri(i + 1) + i];
-    double beta = alpha, tau = 0.0, scal = 0.0;
-    if (xn2 > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-      tau = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
+// p[0] + ... + p[7], p 16-byte aligned
+__device__ __forceinline__ double sum8(const double* p) {
+  static_assert(kWarps == 8, "one term per warp");
+  const double2* q = reinterpret_cast<const double2*>(p);
+  const double2 a = q[0], b = q[1], c = q[2], d = q[3];
+  return ((a.x + a.y) + (b.x + b.y)) + ((c.x + c.y) + (d.x + d.y));
+}
+
+// 1 / sqrt(x) and 1 / x for normal x > 0 by Newton's iteration from the hardware's approximations (PTX
+// rsqrt.approx.ftz.f64, rcp.approx.ftz.f64), without the branches of the library functions, so that the
+// compiler can interleave the chain with the products around it. Two steps square an error of at most
+// 2^-19 twice: within 2 ulp.
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+#pragma unroll
+  for (int k = 0; k < 2; ++k) r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
+  return r;
+}
+__device__ __forceinline__ double rcp_newton(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+#pragma unroll
+  for (int k = 0; k < 2; ++k) r = fma(r, fma(-x, r, 1.0), r);
+  return r;
+}
+
+struct Refl {
+  double beta, tau, v1;  // v1 = alpha - beta, the reflector's first element
+};
+// The reflector of the published column i: s = |x|^2, beta = -sign(alpha) |x|, tau = 2 / v^T v.
+// A column below 1e-120 counts as reduced already (tau = 0).
+__device__ __forceinline__ Refl reflector(const TriCtx& c, int i) {
+  const double alpha = c.xs[i + 1], xn2 = sum8(c.npart), s = fma(alpha, alpha, xn2);
+  const bool zero = !(xn2 > 1.0e-240);
+  const double ss = zero ? 1.0 : s, nrm = ss * rsqrt_newton(ss);
+  const double t = rcp_newton(fma(fabs(alpha), nrm, ss));
+  Refl h;
+  h.beta = zero ? alpha : -copysign(nrm, alpha);
+  h.tau = zero ? 0.0 : t;
+  h.v1 = alpha - h.beta;
+  return h;
+}
+
+// Between the barriers of column i: thread t owns frame row p = first + t (rows below `first` are done).
+// Completes y = A v, forms w = tau y + a2 v, and publishes v, w and the updated next column.
+__device__ __forceinline__ void tri_rows(const TriCtx& c, int first, int i, const Refl& h) {
+  const int t = threadIdx.x, p = first + t;
+  double part = 0.0;
+  if (p < c.M) {
+    const double z1 = c.rsum[i + 1] + sum8(c.cpart + (i + 1) * kPart), raw1 = c.raw[i + 1];
+    const double z = c.rsum[p] + sum8(c.cpart + p * kPart), raw = c.raw[p], x0 = c.xs[p];
+    const double q = sum8(c.dpart);
+    const double y1 = fma(-h.beta, raw1, z1), y = fma(-h.beta, raw, z);
+    const double vav = fma(-h.beta, z1 + y1, q);  // x^T A x - 2 beta (A x)_{i+1} + beta^2 A_{i+1,i+1}
+    const double a2 = -0.5 * h.tau * h.tau * vav;
+    const double v = p == i + 1 ? h.v1 : x0;      // x is zero up to i
+    const double w = p > i ? fma(h.tau, y, a2 * v) : 0.0;
+    const double w1 = fma(h.tau, y1, a2 * h.v1);
+    const double x = raw - fma(v, w1, w * h.v1);
+    const double xn = p > i + 1 ? x : 0.0;
+    c.xs[p] = xn;
+    c.ws[p] = w;
+    c.vs[p] = v;
+    if (p > i + 2) part = x * x;
+    if (p == i + 1) {
+      c.d[p - c.off] = x;
+      c.e[i - c.off] = h.beta;
+      c.tau[i - c.off] = h.tau;
     }
-    if (t == 0) {
-      s.tau[i] = tau;
-      s.e[i] = beta;
-      s.d[i] = A[tri(i) + i];
-    }
-    if (xn2 == 0.0) {  // column already reduced (uniform): only the next norm is needed
-      xn2 = block_sum_alt(t >= i + 3 && t < n ? A[tri(t) + i + 1] * A[tri(t) + i + 1] : 0.0, s.red, parity);
-      continue;
-    }
-    if (t > i && t < n) {  // reflector: one thread per row
-      double vr = 1.0;
-      if (t > i + 1) {
-        vr = A[tri(t) + i] * scal;
-        A[tri(t) + i] = vr;
+  }
+  if (first + (t & ~31) < c.M) part = warp_sum(part);
+  if ((t & 31) == 0) c.npart[t >> 5] = part;
+}
+
+// After the second barrier: reflector i to global memory.
+__device__ __forceinline__ void store_reflector(const TriCtx& c, int first, int i) {
+  const int p = first + threadIdx.x;
+  if (p > i && p < c.M) c.V[(i - c.off) * c.n + (p - c.off)] = c.vs[p];
+}
+
+// Columns of block column kRegB - NB of the register frame (frame rows base + 16 (kRegB - NB) ..),
+// from frame row i on; returns the first column not done.
+template <int NB>
+__device__ __forceinline__ int tri_cols(double (&a)[kRegB * (kRegB + 1) / 2], const TriCtx& c, int base, int i) {
+  constexpr int B0 = kRegB - NB;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
+  const int end = min(base + 16 * (B0 + 1), c.M - 2);
+  for (; i < end; ++i) {
+    const Refl h = reflector(c, i);
+    constexpr int R = NB > 3 ? 8 : (NB > 1 ? 4 : 2);  // row sums and, in the last place, v^T A v
+    {
+      double vc[NB], pc[NB], py[R], dot = 0.0;
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        vc[k] = c.xs[base + 16 * (B0 + k) + tx];
+        pc[k] = 0.0;
       }
-      s.v[t] = vr;
+#pragma unroll
+      for (int I = 0; I < NB; ++I) {
+        const double vr = c.xs[base + 16 * (B0 + I) + ty];
+        double acc = 0.0;
+#pragma unroll
+        for (int J = 0; J <= I; ++J) {
+          const double x = a[rblk(B0 + I, B0 + J)];
+          acc = fma(x, vc[J], acc);
+          if (J < I) pc[J] = fma(x, vr, pc[J]);
+        }
+        dot = fma(acc, vr, dot);
+        py[I] = acc;
+      }
+#pragma unroll
+      for (int J = 0; J < NB; ++J) dot = fma(pc[J], vc[J], dot);
+#pragma unroll
+      for (int I = NB; I < R - 1; ++I) py[I] = 0.0;
+      py[R - 1] = dot;
+      // the next column's present values
+      if (tx == ((i + 1) & 15)) {
+        const bool nextb = tx == 0;
+#pragma unroll
+        for (int I = 0; I < NB; ++I) {
+          double x = a[rblk(B0 + I, B0)];
+          if (I > 0) x = nextb ? a[rblk(B0 + I, B0 + (I > 0 ? 1 : 0))] : x;
+          c.raw[base + 16 * (B0 + I) + ty] = x;
+        }
+      }
+      // column sums over this warp's two rows of threads, then one partial per warp
+#pragma unroll
+      for (int J = 0; J < NB; ++J) pc[J] += __shfl_xor_sync(0xffffffffu, pc[J], 16);
+      if (lane < 16) {
+#pragma unroll
+        for (int J = 0; J < NB; ++J) c.cpart[(base + 16 * (B0 + J) + tx) * kPart + (tid >> 5)] = pc[J];
+      }
+      // row sums over the 16 lanes of a row
+      double sum;
+      if constexpr (R == 8) sum = sum16_of8(py, lane);
+      else if constexpr (R == 4) sum = sum16_of4(py, lane);
+      else sum = sum16_of2(py, lane);
+      constexpr int S = 16 / R;  // lanes that share a sum
+      const int I = (lane & 15) / S;
+      const double both = sum + __shfl_xor_sync(0xffffffffu, sum, 16);
+      if ((lane & (S - 1)) == 0) {
+        if (I < NB) c.rsum[base + 16 * (B0 + I) + ty] = sum;
+        if (I == R - 1 && lane < 16) c.dpart[tid >> 5] = both;
+      }
     }
     __syncthreads();
-    const int m = n - i - 1;
-    const int lg = min(5, 31 - __clz(kThreads / m));
-    const int T = 1 << lg, k = t & (T - 1), r = i + 1 + (t >> lg);
-    const bool mine = r < n;
-    const int tr = mine ? tri(r) : 0;
-    // y_r = sum_{c > i} A(r, c) v_c; four independent accumulators per thread
-    double y = 0.0;
-    if (mine) {
-      double y0 = 0.0, y1 = 0.0, y2 = 0.0, y3 = 0.0;
-      const double* row = A + tr;
-      int c = i + 1 + k;
-      for (; c + 3 * T <= r; c += 4 * T) {
-        y0 = fma(row[c], s.v[c], y0);
-        y1 = fma(row[c + T], s.v[c + T], y1);
-        y2 = fma(row[c + 2 * T], s.v[c + 2 * T], y2);
-        y3 = fma(row[c + 3 * T], s.v[c + 3 * T], y3);
+    tri_rows(c, base + 16 * B0, i, h);
+    __syncthreads();
+    store_reflector(c, base + 16 * B0, i);
+    {
+      double wr[NB], vr[NB];
+#pragma unroll
+      for (int I = 0; I < NB; ++I) {
+        wr[I] = c.ws[base + 16 * (B0 + I) + ty];
+        vr[I] = c.vs[base + 16 * (B0 + I) + ty];
       }
-      for (; c <= r; c += T) y0 = fma(row[c], s.v[c], y0);
-      for (; c + 3 * T < n; c += 4 * T) {
-        y0 = fma(A[tri(c) + r], s.v[c], y0);
-        y1 = fma(A[tri(c + T) + r], s.v[c + T], y1);
-        y2 = fma(A[tri(c + 2 * T) + r], s.v[c + 2 * T], y2);
-        y3 = fma(A[tri(c + 3 * T) + r], s.v[c + 3 * T], y3);
-      }
-      for (; c < n; c += T) y1 = fma(A[tri(c) + r], s.v[c], y1);
-      y = (y0 + y1) + (y2 + y3);
-    }
-    for (int o = T >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    y *= tau;
-    const double vr = mine ? s.v[r] : 0.0;
-    if (mine && k == 0) s.p[r] = y;
-    const double a2 = -0.5 * tau * block_sum_alt(mine && k == 0 ? y * vr : 0.0, s.red, parity);
-    // A22 -= v w^T + w v^T (w = p + a2 v) on the row segments, keeping the next column's norm part
-    double part = 0.0;
-    if (mine) {
-      const double wr = y + a2 * vr;
-      double* row = A + tr;
-      int c = i + 1 + k;
-      for (; c + 3 * T <= r; c += 4 * T) {
-        const double v0 = s.v[c], v1 = s.v[c + T], v2 = s.v[c + 2 * T], v3 = s.v[c + 3 * T];
-        const double w0 = s.p[c] + a2 * v0, w1 = s.p[c + T] + a2 * v1, w2 = s.p[c + 2 * T] + a2 * v2,
-                     w3 = s.p[c + 3 * T] + a2 * v3;
-        const double a0 = row[c], a1 = row[c + T], a2_ = row[c + 2 * T], a3 = row[c + 3 * T];
-        row[c] = a0 - (vr * w0 + wr * v0);
-        row[c + T] = a1 - (vr * w1 + wr * v1);
-        row[c + 2 * T] = a2_ - (vr * w2 + wr * v2);
-        row[c + 3 * T] = a3 - (vr * w3 + wr * v3);
-      }
-      for (; c <= r; c += T) {
-        const double vc = s.v[c], wc = s.p[c] + a2 * vc;
-        row[c] -= vr * wc + wr * vc;
-      }
-      if (k == 0 && r >= i + 3) {
-        const double x = row[i + 1];
-        part = x * x;
+#pragma unroll
+      for (int J = 0; J < NB; ++J) {
+        const double wc = c.ws[base + 16 * (B0 + J) + tx], vc = c.vs[base + 16 * (B0 + J) + tx];
+#pragma unroll
+        for (int I = J; I < NB; ++I) {
+          double& x = a[rblk(B0 + I, B0 + J)];
+          x = fma(-wr[I], vc, fma(-vr[I], wc, x));
+        }
       }
     }
-    xn2 = block_sum_alt(part, s.red, parity);
   }
-  if (close && t == 0) {
-    if (n >= 2) {
-      s.d[n - 2] = A[tri(n - 2) + n - 2];
-      s.e[n - 2] = A[tri(n - 1) + n - 2];
-      s.tau[n - 2] = 0.0;
-    }
-    s.d[n - 1] = A[tri(n - 1) + n - 1];
-    s.e[n - 1] = 0.0;
-  }
-  __syncthreads();
+  return i;
 }
 
-// Householder reduction of the packed n x n matrix A (shared or global memory).
-__device__ void tridiagonalize(int n, double* __restrict__ A, const EigenScratch& s) {
-  householder_columns(n, A, s.v, s.p, s.red, s.tau, s.e, s.d, n - 2, true);
+// Private slot of this thread for block (I, J) of the memory columns (later columns, which live
+// longer, come first and so stay in shared memory longest).
+struct TriMem {
+  double *sm, *gm;
+  int cap, nbt, mb;  // slots in shared memory, blocks per frame side, memory block columns
+  __device__ __forceinline__ double* at(int I, int J) const {
+    // columns J+1 .. mb-1 hold nbt - J' blocks each
+    const int k = mb - 1 - J;
+    const int idx = k * (nbt - mb) + k * (k + 1) / 2, end = idx + nbt - J;  // a column is in one of the two
+    return (end <= cap ? sm : gm) + (size_t)(idx + I - J) * kThreads + threadIdx.x;
+  }
+  __device__ __forceinline__ double* next(double* q) const { return q + kThreads; }  // the block below
+};
+
+// The columns of the memory block columns (n > kRegRows): the register blocks take part in every step.
+__device__ __forceinline__ int tri_mem_cols(double (&a)[kRegB * (kRegB + 1) / 2], const TriCtx& c, const TriMem& m, int i) {
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
+  const int mb = m.mb, base = 16 * mb;
+  for (; i < base; ++i) {
+    const int B = i >> 4;
+    const Refl h = reflector(c, i);
+    double py[8];
+    double dot = 0.0;
+    {
+      double vc[kRegB], pc[kRegB];
+#pragma unroll
+      for (int k = 0; k < kRegB; ++k) {
+        vc[k] = c.xs[base + 16 * k + tx];
+        pc[k] = 0.0;
+      }
+#pragma unroll
+      for (int I = 0; I < kRegB; ++I) {
+        const double vr = c.xs[base + 16 * I + ty];
+        double acc = 0.0;
+#pragma unroll
+        for (int J = 0; J <= I; ++J) {
+          const double x = a[rblk(I, J)];
+          acc = fma(x, vc[J], acc);
+          if (J < I) pc[J] = fma(x, vr, pc[J]);
+        }
+        py[I] = acc;
+      }
+#pragma unroll
+      for (int J = 0; J < kRegB; ++J) {
+        dot = fma(pc[J], vc[J], dot);
+        pc[J] += __shfl_xor_sync(0xffffffffu, pc[J], 16);
+      }
+      if (lane < 16) {
+#pragma unroll
+        for (int J = 0; J < kRegB; ++J) c.cpart[(base + 16 * J + tx) * kPart + (tid >> 5)] = pc[J];
+      }
+    }
+    double vr[kRegB];
+#pragma unroll
+    for (int k = 0; k < kRegB; ++k) vr[k] = c.xs[base + 16 * k + ty];
+    for (int J = B; J < mb; ++J) {
+      const double vcj = c.xs[16 * J + tx];
+      double pcj = 0.0;
+      for (int I = J + 1; I < mb; ++I) pcj = fma(*m.at(I, J), c.xs[16 * I + ty], pcj);
+      const double* q = m.at(mb, J);
+#pragma unroll
+      for (int k = 0; k < kRegB; ++k, q += kThreads) {
+        const double x = *q;
+        py[k] = fma(x, vcj, py[k]);
+        pcj = fma(x, vr[k], pcj);
+      }
+      dot = fma(pcj, vcj, dot);
+      const double s = pcj + __shfl_xor_sync(0xffffffffu, pcj, 16);
+      if (lane < 16) c.cpart[(16 * J + tx) * kPart + (tid >> 5)] = s;
+    }
+    for (int I = B; I < mb; ++I) {
+      double acc = 0.0;
+      for (int J = B; J <= I; ++J) acc = fma(*m.at(I, J), c.xs[16 * J + tx], acc);
+      dot = fma(acc, c.xs[16 * I + ty], dot);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if ((lane & 15) == 0) c.rsum[16 * I + ty] = acc;
+    }
+#pragma unroll
+    for (int I = 0; I < kRegB; ++I) dot = fma(py[I], vr[I], dot);
+    py[7] = dot;
+    {
+      const double s = sum16_of8(py, lane);
+      const int I = (lane & 15) >> 1;
+      const double both = s + __shfl_xor_sync(0xffffffffu, s, 16);
+      if (!(lane & 1)) {
+        if (I < kRegB) c.rsum[base + 16 * I + ty] = s;
+        else if (lane < 16) c.dpart[tid >> 5] = both;
+      }
+    }
+    if (tx == ((i + 1) & 15)) {
+      const int Bn = (i + 1) >> 4;
+      if (Bn < mb) {
+        for (int I = Bn; I < m.nbt; ++I) c.raw[16 * I + ty] = *m.at(I, Bn);
+      } else {
+#pragma unroll
+        for (int I = 0; I < kRegB; ++I) c.raw[base + 16 * I + ty] = a[rblk(I, 0)];
+      }
+    }
+    __syncthreads();
+    tri_rows(c, 16 * B, i, h);
+    __syncthreads();
+    store_reflector(c, 16 * B, i);
+    double wr[kRegB];
+#pragma unroll
+    for (int k = 0; k < kRegB; ++k) {
+      wr[k] = c.ws[base + 16 * k + ty];
+      vr[k] = c.vs[base + 16 * k + ty];
+    }
+#pragma unroll
+    for (int J = 0; J < kRegB; ++J) {
+      const double wcj = c.ws[base + 16 * J + tx], vcj = c.vs[base + 16 * J + tx];
+#pragma unroll
+      for (int I = J; I < kRegB; ++I) a[rblk(I, J)] = fma(-wr[I], vcj, fma(-vr[I], wcj, a[rblk(I, J)]));
+    }
+    for (int J = B; J < mb; ++J) {
+      const double vcj = c.vs[16 * J + tx], wcj = c.ws[16 * J + tx];
+      for (int I = J; I < mb; ++I) {
+        double* q = m.at(I, J);
+        *q = fma(-c.ws[16 * I + ty], vcj, fma(-c.vs[16 * I + ty], wcj, *q));
+      }
+      double* q = m.at(mb, J);
+#pragma unroll
+      for (int k = 0; k < kRegB; ++k, q = m.next(q)) *q = fma(-wr[k], vcj, fma(-vr[k], wcj, *q));
+    }
+  }
+  return i;
+}
+
+// The symmetric matrix to diagonalise: X, or (len > 0) sum_l coef[l] H_l over the accelerator's history
+// matrices H_l = hist + ((head + l) % depth) stride; plus shift (I - proj). Lower triangles are read.
+struct SymInput {
+  const double* X;
+  const double* hist;
+  const double* coef;
+  int head, len, depth;
+  size_t stride;
+  const double* proj;
+  double shift;
+  __device__ __forceinline__ double at(size_t ix, bool diag) const {
+    double v = 0.0;
+    if (len == 0) v = X[ix];
+    for (int l = 0; l < len; ++l) v = fma(coef[l], hist[(size_t)((head + l) % depth) * stride + ix], v);
+    if (shift != 0.0) v += shift * ((diag ? 1.0 : 0.0) - proj[ix]);
+    return v;
+  }
+};
+
+// Householder reduction of the n x n symmetric matrix: diagonals to s.d, s.e,
+// reflector scales to s.tau, reflector i to V[i n + r] (r > i).
+// `gmem` holds the memory blocks that do not fit shared memory.
+__device__ __noinline__ void tridiagonalize(int n, const SymInput& in, double* V, double* gmem, const EigenScratch& s) {
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  TriCtx c;
+  c.n = n;
+  c.M = frame_rows(n);
+  c.off = c.M - n;
+  c.xs = in_shared(s.sh);
+  c.vs = c.xs + c.M;
+  c.ws = c.vs + c.M;
+  c.raw = c.ws + c.M;
+  c.rsum = c.raw + c.M;
+  c.cpart = c.rsum + c.M;  // M is even and sh 16-byte aligned: rows of kPart stay aligned
+  c.npart = in_shared(s.red);
+  c.dpart = c.npart + kWarps;
+  c.d = in_shared(s.d);
+  c.e = in_shared(s.e);
+  c.tau = in_shared(s.tau);
+  c.V = V;
+  const int off = c.off, M = c.M, nbt = M / 16, mb = nbt - kRegB, base = 16 * mb;
+  TriMem m;
+  m.sm = s.sh + 15 * M;
+  m.gm = gmem;
+  m.cap = max(0, (s.sh_doubles - 15 * M) / kThreads);
+  m.nbt = nbt;
+  m.mb = mb;
+  // element (row, col) of a block at this thread, as an index into the lower triangle; -1 in the padding
+  auto index = [&](int I, int J) -> int {
+    const int r = 16 * I + ty - off, q = 16 * J + tx - off;
+    return min(r, q) >= 0 ? max(r, q) * n + min(r, q) : -1;
+  };
+  double a[kRegB * (kRegB + 1) / 2];
+#pragma unroll
+  for (int k = 0; k < kRegB * (kRegB + 1) / 2; ++k) a[k] = 0.0;
+  // history matrices in groups, with all the group's loads in flight: four at a time when a thread has at
+  // most 6 elements, else one (28 loads of one matrix)
+  auto load = [&](auto first, auto group) {
+    constexpr int F = decltype(first)::value, U = decltype(group)::value;
+    const int terms = max(in.len, 1);
+    for (int l0 = 0; l0 < terms; l0 += U) {
+      const double* src[U];
+      double cf[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int l = min(l0 + u, terms - 1);
+        src[u] = in.len ? in.hist + (size_t)((in.head + l) % in.depth) * in.stride : in.X;
+        cf[u] = l0 + u >= terms ? 0.0 : (in.len ? in.coef[l] : 1.0);
+      }
+#pragma unroll
+      for (int I = F; I < kRegB; ++I)
+#pragma unroll
+        for (int J = F; J <= I; ++J) {
+          const int ix = index(mb + I, mb + J);
+          if (ix >= 0) {
+            double x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[u] = src[u][ix];
+#pragma unroll
+            for (int u = 0; u < U; ++u) a[rblk(I, J)] = fma(cf[u], x[u], a[rblk(I, J)]);
+          }
+        }
+    }
+  };
+  if (off >= 16 * (kRegB - 3)) load(std::integral_constant<int, kRegB - 3>{}, std::integral_constant<int, 4>{});
+  else load(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
+  if (in.shift != 0.0) {
+#pragma unroll
+    for (int I = 0; I < kRegB; ++I)
+#pragma unroll
+      for (int J = 0; J <= I; ++J) {
+        const int ix = index(mb + I, mb + J);
+        if (ix >= 0) a[rblk(I, J)] += in.shift * ((I == J && tx == ty ? 1.0 : 0.0) - in.proj[ix]);
+      }
+  }
+  for (int J = 0; J < mb; ++J)
+    for (int I = J; I < nbt; ++I) {
+      const int ix = index(I, J);
+      *m.at(I, J) = ix >= 0 ? in.at(ix, I == J && tx == ty) : 0.0;
+    }
+  // publish the first column
+  const int B = off >> 4;
+  if (tx == (off & 15)) {
+    if (B < mb) {
+      for (int I = B; I < nbt; ++I) c.raw[16 * I + ty] = *m.at(I, B);
+    } else {
+#pragma unroll
+      for (int J = 0; J < kRegB; ++J)
+        if (J == B - mb) {
+#pragma unroll
+          for (int I = J; I < kRegB; ++I) c.raw[base + 16 * I + ty] = a[rblk(I, J)];
+        }
+    }
+  }
+  __syncthreads();
+  double part = 0.0;
+  if (tid < M) {
+    const double x = tid > off ? c.raw[tid] : 0.0;
+    c.xs[tid] = x;
+    if (tid == off) c.d[0] = c.raw[tid];
+    if (tid > off + 1) part = x * x;
+  }
+  part = warp_sum(part);
+  if ((tid & 31) == 0) c.npart[tid >> 5] = part;
+  __syncthreads();
+  int i = off;
+  if (mb > 0) i = tri_mem_cols(a, c, m, i);
+  switch (mb > 0 ? kRegB : kRegB - (off >> 4)) {
+    case 7: i = tri_cols<7>(a, c, base, i); [[fallthrough]];
+    case 6: i = tri_cols<6>(a, c, base, i); [[fallthrough]];
+    case 5: i = tri_cols<5>(a, c, base, i); [[fallthrough]];
+    case 4: i = tri_cols<4>(a, c, base, i); [[fallthrough]];
+    case 3: i = tri_cols<3>(a, c, base, i); [[fallthrough]];
+    case 2: i = tri_cols<2>(a, c, base, i); [[fallthrough]];
+    default: tri_cols<1>(a, c, base, i);
+  }
+  if (tid == 0) {
+    if (n >= 2) {
+      c.e[n - 2] = c.xs[M - 1];
+      c.tau[n - 2] = 0.0;
+    }
+    c.e[n - 1] = 0.0;
+  }
+  if (n >= 2 && tid == kThreads - 1) c.d[n - 1] = a[rblk(kRegB - 1, kRegB - 1)];
+  __syncthreads();
 }
 
 // ------------------------------------------------------------- 2. split + eigenvalues
@@ -255,40 +643,44 @@ __device__ void tridiag_eigenvalues(int n, int kval, const EigenScratch& s_, con
   struct {
     double *d, *e, *e2, *misc, *lam;
     int *blk, *nblk;
-  } s = {s_.d, s_.e, s_.e2, s_.misc, s_.lam, s_.blk, s_.nblk};
+  } s = {in_shared(s_.d), in_shared(s_.e), in_shared(s_.e2), in_shared(s_.misc), in_shared(s_.lam), in_shared(s_.blk),
+         in_shared(s_.nblk)};
   const int tid = threadIdx.x;
   constexpr double eps = 2.220446049250313e-16;
-  if (tid == 0) {
+  {
     // Gershgorin bounds of the unsplit T, then split where |e_i| <= 1000 eps ||T||: an
     // absolute criterion, so exactly degenerate eigenvalues (which Householder leaves joined
-    // by couplings of a few eps ||T||) land in separate blocks.
-    double gl = s.d[0], gu = s.d[0];
-    for (int i = 0; i < n; ++i) {
-      const double rad = (i + 1 < n ? fabs(s.e[i]) : 0.0) + (i > 0 ? fabs(s.e[i - 1]) : 0.0);
-      gl = fmin(gl, s.d[i] - rad);
-      gu = fmax(gu, s.d[i] + rad);
-    }
+    // by couplings of a few eps ||T||) land in separate blocks. One row per thread (n <= kThreads).
+    const bool row = tid < n;
+    const double ei = tid + 1 < n ? s.e[tid] : 0.0;
+    const double rad = fabs(ei) + (row && tid > 0 ? fabs(s.e[tid - 1]) : 0.0);
+    const double gl = -block_max(row ? rad - s.d[tid] : -INFINITY, s_.red);
+    const double gu = block_max(row ? s.d[tid] + rad : -INFINITY, s_.red);
     const double tnorm = fmax(fabs(gl), fabs(gu));
-    const double cut = 1000.0 * eps * tnorm;
-    int nb = 0;
-    s.blk[0] = 0;
-    double emax = 0.0;
-    for (int i = 0; i < n; ++i) {
-      double ei = (i + 1 < n) ? s.e[i] : 0.0;
-      if (i + 1 < n && fabs(ei) <= cut) {
-        ei = 0.0;
-        s.e[i] = 0.0;
-        s.blk[++nb] = i + 1;
+    const bool cut = tid + 1 < n && fabs(ei) <= 1000.0 * eps * tnorm;
+    if (row) s.e2[tid] = cut ? 0.0 : ei * ei;
+    const double emax = block_max(row && !cut ? ei * ei : 0.0, s_.red);
+    if (cut) s.e[tid] = 0.0;
+    if (__syncthreads_or(cut)) {
+      if (tid == 0) {
+        int nb = 0;
+        s.blk[0] = 0;
+        for (int i = 0; i + 1 < n; ++i)
+          if (s.e[i] == 0.0) s.blk[++nb] = i + 1;
+        s.blk[++nb] = n;
+        *s.nblk = nb;
       }
-      s.e2[i] = ei * ei;
-      emax = fmax(emax, ei * ei);
+    } else if (tid == 0) {
+      s.blk[0] = 0;
+      s.blk[1] = n;
+      *s.nblk = 1;
     }
-    s.blk[++nb] = n;
-    *s.nblk = nb;
-    s.misc[0] = 2.2250738585072014e-308 * fmax(1.0, emax);  // pivmin
-    s.misc[1] = tnorm;
-    s.misc[2] = gl - 4.0 * eps * tnorm * n - 1.0e-300;
-    s.misc[3] = gu + 4.0 * eps * tnorm * n + 1.0e-300;
+    if (tid == 0) {
+      s.misc[0] = 2.2250738585072014e-308 * fmax(1.0, emax);  // pivmin
+      s.misc[1] = tnorm;
+      s.misc[2] = gl - 4.0 * eps * tnorm * n - 1.0e-300;
+      s.misc[3] = gu + 4.0 * eps * tnorm * n + 1.0e-300;
+    }
   }
   __syncthreads();
   const double pivmin = s.misc[0], tnorm = s.misc[1], glo = s.misc[2], ghi = s.misc[3];
@@ -373,25 +765,51 @@ __device__ void tridiag_eigenvalues(int n, int kval, const EigenScratch& s_, con
 }
 
 // ------------------------------------------------------------- 3. tridiagonal eigenvectors
-// Eigenvector j (< kvec) of T into Y[j*n .. j*n+n) (zero outside its block). `tf` is per-CTA
-// global scratch of kvec * 6n doubles.
-__device__ void tridiag_vectors(int n, int kvec, double* Y, double* tf, const EigenScratch& s_) {
+// Power of two that brings the larger of two magnitudes into [1, 2), as its exponent (0 for zeros).
+__device__ __forceinline__ int pair_exponent(double a, double b) {
+  const double m = fmax(fabs(a), fabs(b));
+  const int ex = (__double2hiint(m) >> 20) & 0x7ff;
+  return ex == 0 ? 0 : ex - 1023;
+}
+__device__ __forceinline__ double pow2(int ex) {  // 2^ex for normal results, 0 below, the largest power above
+  return ex < -1022 ? 0.0 : __hiloint2double((min(ex, 1023) + 1023) << 20, 0);
+}
+
+// Eigenvectors j < kvec of T, unnormalised, into Yt[i kvec + j] (zero outside the block of each). `tf` is
+// per-CTA global scratch of 6 n^2 doubles. Every array has the vector index fastest, so that the
+// threads of a warp (one vector each) touch consecutive addresses.
+//
+// The twisted factorisation N_r D_r N_r^T of T - lam gives y from the top down to row r and from the bottom up to it.
+// Both parts obey T's own three-term recurrence: f_{i+1} = ((lam - d_i) f_i - e_{i-1} f_{i-1}) / e_i
+// from f = 1 in the first row, and g likewise upward from the last row. One half of the CTA runs f, the other
+// g; with the reciprocals of e shared by all vectors, one FMA a row is in the dependent chain (the
+// pivots L+ D+ L+^T, U- D- U-^T of the same factorisation have a division in it: 150 cycles a row).
+// The twist gamma_r is 1 / [(T - lam)^-1]_rr up to a factor common to all rows, and that element is
+// proportional to f_r g_r, so r is the row of the largest |f g|; y = f / f_r above it, g / g_r below.
+// Pairs are rescaled by powers of two every 8 rows (a row grows them by at most (lam - d) / e, and e
+// is above 1000 eps ||T|| within a block); the exponents are kept per group of 8 rows.
+__device__ double* tridiag_vectors(int n, int kvec, double* tf, const EigenScratch& s_) {
   struct {
     const double *d, *e, *e2, *lam, *misc;
     const int *blk, *nblk;
     int* vinfo;
-  } s = {s_.d, s_.e, s_.e2, s_.lam, s_.misc, s_.blk, s_.nblk, s_.vinfo};
+    double *inve, *aux;
+  } s = {in_shared(s_.d),   in_shared(s_.e),    in_shared(s_.e2),    in_shared(s_.lam), in_shared(s_.misc),
+         in_shared(s_.blk), in_shared(s_.nblk), in_shared(s_.vinfo), in_shared(s_.p),   in_shared(s_.v)};
   const int tid = threadIdx.x;
   const double pivmin = s.misc[0], tnorm = s.misc[1];
   const int nb = *s.nblk;
   const double win = 1.0e-11 * fmax(tnorm, 1.0);
-  // Two halves of the CTA work on the same vectors: warps 0-3 (half 0) form the top-down
-  // factorisation L+ D+ L+^T of T - lam, warps 4-7 (half 1) the bottom-up U- D- U-^T; both are
-  // chains of divisions, so running them side by side halves the latency per vector. Then half 0
-  // picks the twist index, and the halves fill the vector above and below it. Per-vector scratch
-  // in tf (6 n): D+, L+, U-, D- (the pivots after clamping), then [twist, block], [norm parts].
+  const size_t nk = (size_t)n * kvec;
+  double* __restrict__ F = tf;
+  double* __restrict__ G = tf + nk;
+  double* __restrict__ Yt = tf + 2 * nk;
+  int* __restrict__ EF = reinterpret_cast<int*>(tf + 3 * nk);  // [group of 8 block rows][kvec]
+  int* __restrict__ EG = EF + (size_t)((n + 7) / 8) * kvec;
   constexpr int kHalf = kThreads / 2;
   const int half = tid / kHalf, hj = tid % kHalf;
+  if (tid < n) s.inve[tid] = s.e[tid] != 0.0 ? 1.0 / s.e[tid] : 0.0;
+  __syncthreads();
   for (int j = hj; j < kvec; j += kHalf) {
     const double lam = s.lam[j];
     // which unreduced block holds this eigenvalue (degenerate copies go to successive blocks);
@@ -406,110 +824,129 @@ __device__ void tridiag_vectors(int n, int kvec, double* Y, double* tf, const Ei
     }
     if (b < 0) b = 0;  // inconsistent counts (not expected): block 0
     if (half == 0) s.vinfo[j] = b;
-    const int lo = s.blk[b], hi = s.blk[b + 1] - 1, m = hi - lo + 1;
-    double* y = Y + (size_t)j * n;
-    for (int i = half; i < n; i += 2) y[i] = 0.0;
-    if (m == 1) continue;
-    double* Dp = tf + (size_t)j * 6 * n;
-    double* Lp = Dp + n;
-    double* Um = Lp + n;
-    double* Dm = Um + n;
-    if (half == 0) {  // T - lam = L+ D+ L+^T (top-down)
-      double dp = s.d[lo] - lam;
-      for (int i = 0; i < m - 1; ++i) {
-        if (fabs(dp) < pivmin) dp = dp < 0.0 ? -pivmin : pivmin;
-        Dp[i] = dp;
-        const double ei = s.e[lo + i];
-        Lp[i] = ei / dp;
-        dp = (s.d[lo + i + 1] - lam) - Lp[i] * ei;
+    const int lo = s.blk[b], m = s.blk[b + 1] - lo;
+    // step t of half 0 goes from row lo + t to the next; of half 1 from row hi - t to the one before
+    const int step = half == 0 ? 1 : -1;
+    const double* dd = s.d + (half == 0 ? lo : lo + m - 1);
+    const double* ee = s.e + (half == 0 ? lo : lo + m - 2);       // coupling crossed by step t
+    const double* iv = s.inve + (half == 0 ? lo : lo + m - 2);
+    double* __restrict__ out = (half == 0 ? F : G) + (size_t)(half == 0 ? lo : lo + m - 1) * kvec + j;
+    int* __restrict__ ex = (half == 0 ? EF : EG) + j;
+    const ptrdiff_t os = (ptrdiff_t)step * kvec;
+    double f = 1.0, fm = 0.0;  // this row's value and the one before
+    int e = 0;
+    *out = f;
+    *ex = 0;
+    for (int t0 = 0; t0 < m - 1; t0 += 8) {
+      double A[8], B[8], y[8];  // the eight rows' coefficients first: only FMAs stay in the chain
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int t = min(t0 + u, m - 2);
+        const double inv = iv[step * t];
+        A[u] = (lam - dd[step * t]) * inv;
+        B[u] = t > 0 ? ee[step * (t - 1)] * inv : 0.0;
       }
-      if (fabs(dp) < pivmin) dp = dp < 0.0 ? -pivmin : pivmin;
-      Dp[m - 1] = dp;
-    } else {  // T - lam = U- D- U-^T (bottom-up)
-      double dm = s.d[hi] - lam;
-      if (fabs(dm) < pivmin) dm = dm < 0.0 ? -pivmin : pivmin;
-      Dm[m - 1] = dm;
-      for (int i = m - 2; i >= 0; --i) {
-        const double ei = s.e[lo + i];
-        Um[i] = ei / dm;
-        dm = (s.d[lo + i] - lam) - Um[i] * ei;
-        if (fabs(dm) < pivmin) dm = dm < 0.0 ? -pivmin : pivmin;
-        Dm[i] = dm;
+      if (t0 > 0) {
+        const int q = pair_exponent(f, fm);
+        const double sc = pow2(-q);
+        f *= sc;
+        fm *= sc;
+        e += q;
       }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double fn = fma(A[u], f, -(B[u] * fm));
+        fm = f;
+        f = y[u] = fn;
+      }
+      ex[(size_t)(t0 >> 3) * kvec] = e;  // of rows t0 + 1 .. t0 + 8 of the block
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (t0 + u < m - 1) out[os * (t0 + u + 1)] = y[u];
     }
   }
   __syncthreads();
-  // twist index r minimising |gamma_i| = |D+_i + D-_i - (d_i - lam)| (the largest index among ties,
-  // as a downward scan with a strict comparison finds it)
-  if (half == 0)
-    for (int j = hj; j < kvec; j += kHalf) {
-      const double lam = s.lam[j];
-      const int b = s.vinfo[j], lo = s.blk[b], hi = s.blk[b + 1] - 1, m = hi - lo + 1;
-      if (m == 1) continue;
-      double* Dp = tf + (size_t)j * 6 * n;
-      const double* Dm = Dp + 3 * n;
-      double best = fabs(Dp[m - 1] + Dm[m - 1] - (s.d[hi] - lam));
-      int r = m - 1;
-      for (int i = m - 2; i >= 0; --i) {
-        const double g = fabs(Dp[i] + Dm[i] - (s.d[lo + i] - lam));
-        if (g < best) {
-          best = g;
-          r = i;
+  // From here every thread has one vector and a share of its groups of 8 rows (vectors fastest; more than 16
+  // shares would only lengthen the combination).
+  // Row lo + t of f is in group (t - 1) / 8 (row lo in group 0, whose exponent is 0), of g row hi - t.
+  const int shares = min(kThreads / kvec, 16), share = tid / kvec, jv = tid - share * kvec;
+  const bool in_share = share < shares;
+  // The row of the largest |f g|: as an integer, a double's bits plus its scale exponent order the scaled magnitudes.
+  long long* __restrict__ K = reinterpret_cast<long long*>(in_shared(s_.sh));      // [shares][kvec], at most kThreads
+  int* __restrict__ R = reinterpret_cast<int*>(in_shared(s_.sh) + kThreads);       // the same
+  constexpr long long kLow = -0x7fffffffffffffffLL;
+  if (in_share) {
+    const int j = jv, b = s.vinfo[j], lo = s.blk[b], hi = s.blk[b + 1] - 1;
+    long long best = kLow;
+    int br = hi;
+    for (int g = share; lo + 8 * g <= hi; g += shares) {
+      const int t0 = 8 * g + (g > 0 ? 1 : 0), t1 = min(8 * g + 8, hi - lo);  // rows t0 .. t1 of the block
+      const int ef = EF[g * kvec + j];
+      // g's rows hi - i: at most three of its groups meet nine rows
+      const int gb = max(hi - lo - t1 - 1, 0) >> 3;
+      const int e0 = EG[gb * kvec + j], e1 = EG[min(gb + 1, (n + 7) / 8 - 1) * kvec + j];
+      double p[9];
+#pragma unroll
+      for (int u = 0; u < 9; ++u) {
+        const int i = lo + min(t0 + u, t1);
+        p[u] = fabs(F[i * kvec + j] * G[i * kvec + j]);
+      }
+#pragma unroll
+      for (int u = 0; u < 9; ++u) {
+        const int t = t0 + u;
+        if (t <= t1 && p[u] > 0.0) {
+          const int q = ef + ((max(hi - lo - t - 1, 0) >> 3) == gb ? e0 : e1);
+          const long long key = __double_as_longlong(p[u]) + ((long long)q << 52);
+          if (key > best) {
+            best = key;
+            br = lo + t;
+          }
         }
       }
-      reinterpret_cast<int*>(Dp + 4 * n)[0] = r;
     }
-  __syncthreads();
-  // solve N_r D_r N_r^T y = gamma_r e_r: half 0 the rows above r, half 1 from r down; partial norms
-  for (int j = hj; j < kvec; j += kHalf) {
-    const int b = s.vinfo[j], lo = s.blk[b], hi = s.blk[b + 1] - 1, m = hi - lo + 1;
-    double* y = Y + (size_t)j * n;
-    double* Dp = tf + (size_t)j * 6 * n;
-    if (m == 1) {
-      if (half == 0) y[lo] = 1.0;
-      continue;
-    }
-    const double* Lp = Dp + n;
-    const double* Um = Lp + n;
-    const int r = reinterpret_cast<const int*>(Dp + 4 * n)[0];
-    double nrm = 0.0;
-    if (half == 0) {
-      double yn = 1.0, ynn = 0.0;  // y[lo + i + 1], y[lo + i + 2]
-      for (int i = r - 1; i >= 0; --i) {
-        double z = -Lp[i] * yn;
-        if (yn == 0.0 && i + 2 < m) z = -(s.e[lo + i + 1] / s.e[lo + i]) * ynn;
-        y[lo + i] = z;
-        nrm = fma(z, z, nrm);
-        ynn = yn;
-        yn = z;
-      }
-    } else {
-      y[lo + r] = 1.0;
-      nrm = 1.0;
-      double yc = 1.0, yp = 0.0;  // y[lo + i], y[lo + i - 1] (the latter read only after a zero)
-      for (int i = r; i < m - 1; ++i) {
-        double z = -Um[i] * yc;
-        if (yc == 0.0 && i >= 1) z = -(s.e[lo + i - 1] / s.e[lo + i]) * yp;
-        y[lo + i + 1] = z;
-        nrm = fma(z, z, nrm);
-        yp = yc;
-        yc = z;
-      }
-    }
-    Dp[5 * n + half] = nrm;
+    K[share * kvec + j] = best;
+    R[share * kvec + j] = br;
   }
   __syncthreads();
-  for (int j = hj; j < kvec; j += kHalf) {
-    const int b = s.vinfo[j], lo = s.blk[b], hi = s.blk[b + 1] - 1, m = hi - lo + 1;
-    if (m == 1) continue;
-    const double* Dp = tf + (size_t)j * 6 * n;
-    const int r = reinterpret_cast<const int*>(Dp + 4 * n)[0];
-    const double scale = 1.0 / sqrt(Dp[5 * n] + Dp[5 * n + 1]);
-    double* y = Y + (size_t)j * n;
-    if (half == 0)
-      for (int i = lo; i < lo + r; ++i) y[i] *= scale;
-    else
-      for (int i = lo + r; i <= hi; ++i) y[i] *= scale;
+  if (tid < kvec) {
+    const int j = tid;
+    long long best = K[j];
+    int r = R[j];
+    for (int q = 1; q < shares; ++q)
+      if (K[q * kvec + j] > best) {
+        best = K[q * kvec + j];
+        r = R[q * kvec + j];
+      }
+    const int b = s.vinfo[j], lo = s.blk[b];
+    s.vinfo[j] = b | ((r - lo) << 16);
+    s.inve[j] = 1.0 / F[r * kvec + j];  // the reciprocals of e are spent by now
+    s.aux[j] = 1.0 / G[r * kvec + j];
+  }
+  __syncthreads();
+  if (in_share) {
+    const int j = jv, vi = s.vinfo[j], b = vi & 0xffff, lo = s.blk[b], hi = s.blk[b + 1] - 1, r = lo + (vi >> 16);
+    const double rf = s.inve[j], rg = s.aux[j];
+    const int ef = EF[(max(r - lo - 1, 0) >> 3) * kvec + j], eg = EG[(max(hi - r - 1, 0) >> 3) * kvec + j];
+    for (int i0 = 8 * share; i0 < n; i0 += 8 * shares) {
+      double y[8];
+      int q[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int i = min(i0 + u, n - 1);
+        const bool up = i < r;
+        const bool in = i >= lo && i <= hi;
+        const double* src = up ? F : G;
+        const int* es = up ? EF : EG;
+        const int t = up ? i - lo : hi - i;
+        y[u] = in ? src[i * kvec + j] : 0.0;
+        q[u] = in ? es[(max(t - 1, 0) >> 3) * kvec + j] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const bool up = i0 + u < r;
+        if (i0 + u < n) Yt[(i0 + u) * kvec + j] = y[u] * (up ? rf : rg) * pow2(q[u] - (up ? ef : eg));
+      }
+    }
   }
   __syncthreads();
   // Eigenvalues of one block closer than 1e-7 ||T||: the twisted vectors are not reliable
@@ -517,153 +954,275 @@ __device__ void tridiag_vectors(int n, int kvec, double* Y, double* tf, const Ei
   // row-pivoted LU of T_b - lam, re-orthogonalised against the earlier members of its
   // cluster (the dstein scheme). One thread per block; clusters are rare.
   const double ctol = 1.0e-7 * fmax(tnorm, 1.0), tiny = 2.220446049250313e-16 * fmax(tnorm, 1.0);
+  const bool close = tid > 0 && tid < kvec && s.lam[tid] - s.lam[tid - 1] < ctol;  // kvec <= kThreads
+  if (!__syncthreads_or(close || nb > 1)) return Yt;
   for (int b = tid; b < nb; b += kThreads) {
     const int lo = s.blk[b], hi = s.blk[b + 1] - 1, m = hi - lo + 1;
     int head = -1, prev = -1;
     for (int j = 0; j < kvec; ++j) {
-      if (s.vinfo[j] != b) continue;
+      if ((s.vinfo[j] & 0xffff) != b) continue;
       if (prev < 0 || s.lam[j] - s.lam[prev] >= ctol) {
         head = j;
         prev = j;
         continue;
       }
+      if (prev == head) {  // the cluster's first vector is orthogonalised against: normalise it
+        double nrm = 0.0;
+        for (int i = lo; i <= hi; ++i) nrm += Yt[(size_t)i * kvec + head] * Yt[(size_t)i * kvec + head];
+        nrm = 1.0 / sqrt(nrm);
+        for (int i = lo; i <= hi; ++i) Yt[(size_t)i * kvec + head] *= nrm;
+      }
       prev = j;
-      double* dd = tf + (size_t)j * 6 * n;
-      double* dl = dd + n;
-      double* du = dl + n;
-      double* du2 = du + n;
-      double* pv = du2 + n;
+      // the LU factors take this vector's columns of scratch that is spent by now
+      auto dd = [&](int i) -> double& { return F[(size_t)(lo + i) * kvec + j]; };
+      auto dl = [&](int i) -> double& { return G[(size_t)(lo + i) * kvec + j]; };
+      auto du = [&](int i) -> double& { return tf[3 * nk + (size_t)(lo + i) * kvec + j]; };
+      auto du2 = [&](int i) -> double& { return tf[4 * nk + (size_t)(lo + i) * kvec + j]; };
+      unsigned pv[kMaxN / 32];
+#pragma unroll
+      for (int q = 0; q < kMaxN / 32; ++q) pv[q] = 0u;
       const double sg = s.lam[j];
       for (int i = 0; i < m; ++i) {
-        dd[i] = s.d[lo + i] - sg;
-        if (i + 1 < m) dl[i] = du[i] = s.e[lo + i];
+        dd(i) = s.d[lo + i] - sg;
+        if (i + 1 < m) dl(i) = du(i) = s.e[lo + i];
       }
       for (int i = 0; i + 1 < m; ++i) {
-        if (fabs(dd[i]) >= fabs(dl[i])) {
-          if (dd[i] == 0.0) dd[i] = tiny;
-          const double f = dl[i] / dd[i];
-          dl[i] = f;
-          dd[i + 1] -= f * du[i];
-          if (i + 2 < m) du2[i] = 0.0;
-          pv[i] = 0.0;
+        if (fabs(dd(i)) >= fabs(dl(i))) {
+          if (dd(i) == 0.0) dd(i) = tiny;
+          const double f = dl(i) / dd(i);
+          dl(i) = f;
+          dd(i + 1) -= f * du(i);
+          if (i + 2 < m) du2(i) = 0.0;
         } else {
-          const double f = dd[i] / dl[i];
-          dd[i] = dl[i];
-          dl[i] = f;
-          const double t = du[i];
-          du[i] = dd[i + 1];
-          dd[i + 1] = t - f * dd[i + 1];
+          const double f = dd(i) / dl(i);
+          dd(i) = dl(i);
+          dl(i) = f;
+          const double t = du(i);
+          du(i) = dd(i + 1);
+          dd(i + 1) = t - f * dd(i + 1);
           if (i + 2 < m) {
-            du2[i] = du[i + 1];
-            du[i + 1] = -f * du[i + 1];
+            du2(i) = du(i + 1);
+            du(i + 1) = -f * du(i + 1);
           }
-          pv[i] = 1.0;
+          pv[i >> 5] |= 1u << (i & 31);
         }
       }
       for (int i = 0; i < m; ++i)
-        if (fabs(dd[i]) < tiny) dd[i] = dd[i] < 0.0 ? -tiny : tiny;
-      double* x = Y + (size_t)j * n + lo;
-      for (int i = 0; i < m; ++i) x[i] = sin(1.0 + 0.7 * i + 1.3 * j);
+        if (fabs(dd(i)) < tiny) dd(i) = dd(i) < 0.0 ? -tiny : tiny;
+      auto x = [&](int i) -> double& { return Yt[(size_t)(lo + i) * kvec + j]; };
+      for (int i = 0; i < m; ++i) x(i) = sin(1.0 + 0.7 * i + 1.3 * j);
       for (int it = 0; it < 3; ++it) {
         for (int i = 0; i + 1 < m; ++i) {
-          if (pv[i] == 0.0) {
-            x[i + 1] -= dl[i] * x[i];
+          if (!((pv[i >> 5] >> (i & 31)) & 1u)) {
+            x(i + 1) -= dl(i) * x(i);
           } else {
-            const double t = x[i];
-            x[i] = x[i + 1];
-            x[i + 1] = t - dl[i] * x[i];
+            const double t = x(i);
+            x(i) = x(i + 1);
+            x(i + 1) = t - dl(i) * x(i);
           }
         }
-        x[m - 1] /= dd[m - 1];
-        if (m > 1) x[m - 2] = (x[m - 2] - du[m - 2] * x[m - 1]) / dd[m - 2];
-        for (int i = m - 3; i >= 0; --i) x[i] = (x[i] - du[i] * x[i + 1] - du2[i] * x[i + 2]) / dd[i];
+        x(m - 1) /= dd(m - 1);
+        if (m > 1) x(m - 2) = (x(m - 2) - du(m - 2) * x(m - 1)) / dd(m - 2);
+        for (int i = m - 3; i >= 0; --i) x(i) = (x(i) - du(i) * x(i + 1) - du2(i) * x(i + 2)) / dd(i);
         for (int pass = 0; pass < 2; ++pass)
           for (int q = head; q < j; ++q) {
-            if (s.vinfo[q] != b) continue;
-            const double* yq = Y + (size_t)q * n + lo;
+            if ((s.vinfo[q] & 0xffff) != b) continue;
             double dot = 0.0;
-            for (int i = 0; i < m; ++i) dot += yq[i] * x[i];
-            for (int i = 0; i < m; ++i) x[i] -= dot * yq[i];
+            for (int i = 0; i < m; ++i) dot += Yt[(size_t)(lo + i) * kvec + q] * x(i);
+            for (int i = 0; i < m; ++i) x(i) -= dot * Yt[(size_t)(lo + i) * kvec + q];
           }
         double nrm = 0.0;
-        for (int i = 0; i < m; ++i) nrm += x[i] * x[i];
+        for (int i = 0; i < m; ++i) nrm += x(i) * x(i);
         nrm = 1.0 / sqrt(nrm);
-        for (int i = 0; i < m; ++i) x[i] *= nrm;
+        for (int i = 0; i < m; ++i) x(i) *= nrm;
       }
     }
   }
   __syncthreads();
+  return Yt;
 }
 
 // ------------------------------------------------------------------- 4. back-transform
-// Y[j] <- H(0) H(1) ... H(n-3) Y[j] for j < kvec, two vectors per warp held in registers.
-// One warp applies the reflectors to NV vectors at a time, RT rows per lane held in registers
-// (n <= 32 RT). Per reflector the NV partial dot products are reduced together (their shuffle
-// chains overlap), so the latency of a reflector is paid once for NV vectors.
-template <int RT, int NV>
-__device__ __forceinline__ void back_transform_t(int n, int kvec, const double* __restrict__ A, double* Y,
-                                                 const double* __restrict__ tau_) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int j0 = NV * warp; j0 < kvec; j0 += NV * kWarps) {
+// Y[j] <- H(0) H(1) ... H(n-3) y_j for j < kvec. A group of G lanes holds NV vectors, RT rows of each
+// per lane (n <= G RT). The reflectors pass through shared memory eight at a time (one warp
+// copies one), double buffered with the next eight in registers; the NV dot products
+// are summed over the group together. With at most 16 values of z a lane two reflectors are applied at a time, v0^T
+// H1 z = v0^T z - tau1 (v1^T z) (v0^T v1), so one round of shuffles serves both (n = 48: 20.3k cycles one at a
+// time, 17.6k in pairs; with more, two reflectors and z do not fit the registers: n = 128 95k against 129k). Half of the rows are skipped once they lie above the reflectors.
+template <int G, int RT, int NV>
+__device__ __forceinline__ void back_transform_t(int n, int kvec, const double* __restrict__ V,
+                                                 const double* __restrict__ Yt, double* Y,
+                                                 const double* __restrict__ tau_, double* sh) {
+  constexpr int NG = kThreads / G, LD = G * RT, NP = (LD + 31) / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gl = tid % G, g = tid / G;
+  const int c0 = n >= 3 ? (n - 3) / 8 : -1;
+  for (int j0 = 0; j0 < kvec; j0 += NG * NV) {
     double z[NV][RT];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      const double* y = Y + (size_t)(j0 + v < kvec ? j0 + v : j0) * n;
+      const int j = j0 + v * NG + g;
 #pragma unroll
       for (int t = 0; t < RT; ++t) {
-        const int r = lane + 32 * t;
-        z[v][t] = r < n ? y[r] : 0.0;
+        const int r = gl + G * t;
+        z[v][t] = r < n && j < kvec ? Yt[(size_t)r * kvec + j] : 0.0;
       }
     }
-    for (int i = n - 3; i >= 0; --i) {
-      const double tau = tau_[i];
-      if (tau == 0.0) continue;
-      double vr[RT];
-#pragma unroll
-      for (int t = 0; t < RT; ++t) {
-        const int r = lane + 32 * t;
-        vr[t] = (r > i && r < n) ? (r == i + 1 ? 1.0 : A[tri(r) + i]) : 0.0;
-      }
-      double a[NV];
+    {  // unit norm
+      double nv[NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        double acc = 0.0;
+        double q0 = 0.0, q1 = 0.0;
 #pragma unroll
-        for (int t = 0; t < RT; ++t) acc = fma(vr[t], z[v][t], acc);
-        a[v] = acc;
+        for (int t = 0; t < RT; t += 2) {
+          q0 = fma(z[v][t], z[v][t], q0);
+          if (t + 1 < RT) q1 = fma(z[v][t + 1], z[v][t + 1], q1);
+        }
+        nv[v] = q0 + q1;
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+      for (int o = G / 2; o > 0; o >>= 1)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) a[v] += __shfl_xor_sync(0xffffffffu, a[v], o);
+        for (int v = 0; v < NV; ++v) nv[v] += __shfl_xor_sync(0xffffffffu, nv[v], o);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        const double s = a[v] * tau;
+        nv[v] = nv[v] > 0.0 ? 1.0 / sqrt(nv[v]) : 0.0;
 #pragma unroll
-        for (int t = 0; t < RT; ++t) z[v][t] = fma(-s, vr[t], z[v][t]);
+        for (int t = 0; t < RT; ++t) z[v][t] *= nv[v];
       }
     }
+    double nx[NP];
+    auto fetch = [&](int c) {
+      const int i = 8 * c + warp;
+#pragma unroll
+      for (int u = 0; u < NP; ++u) {
+        const int r = lane + 32 * u;
+        nx[u] = i <= n - 3 && r > i && r < n ? V[(size_t)i * n + r] : 0.0;
+      }
+    };
+    // stages c0 .. c1 (descending); rows of lane index below T0 are above all their reflectors
+    auto stages = [&](auto first, int cs, int ce) {
+      constexpr int T0 = decltype(first)::value;
+      for (int c = cs; c >= ce; --c) {
+        double* buf = sh + (c & 1) * 8 * LD;
+#pragma unroll
+        for (int u = 0; u < NP; ++u)
+          if (lane + 32 * u < LD) buf[warp * LD + lane + 32 * u] = nx[u];
+        __syncthreads();
+        if (c > 0) fetch(c - 1);
+        if constexpr (RT * NV <= 16) {
+#pragma unroll 1
+          for (int u = 7; u > 0; u -= 2) {  // H(i + 1), then H(i)
+            const int i = 8 * c + u - 1;
+            if (i > n - 3) continue;
+            const double t1 = i + 1 <= n - 3 ? tau_[i + 1] : 0.0, t0 = tau_[i];
+            const double* __restrict__ w1 = buf + u * LD + gl;
+            const double* __restrict__ w0 = w1 - LD;
+            double a1[NV], a0[NV], gm = 0.0;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a1[v] = a0[v] = 0.0;
+#pragma unroll
+            for (int t = T0; t < RT; ++t) {
+              const double p1 = w1[G * t], p0 = w0[G * t];
+#pragma unroll
+              for (int v = 0; v < NV; ++v) {
+                a1[v] = fma(p1, z[v][t], a1[v]);
+                a0[v] = fma(p0, z[v][t], a0[v]);
+              }
+              gm = fma(p1, p0, gm);
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+#pragma unroll
+              for (int v = 0; v < NV; ++v) {
+                a1[v] += __shfl_xor_sync(0xffffffffu, a1[v], o);
+                a0[v] += __shfl_xor_sync(0xffffffffu, a0[v], o);
+              }
+              gm += __shfl_xor_sync(0xffffffffu, gm, o);
+            }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              a1[v] *= -t1;
+              a0[v] = -t0 * fma(a1[v], gm, a0[v]);
+            }
+#pragma unroll
+            for (int t = T0; t < RT; ++t) {
+              const double p1 = w1[G * t], p0 = w0[G * t];
+#pragma unroll
+              for (int v = 0; v < NV; ++v) z[v][t] = fma(a0[v], p0, fma(a1[v], p1, z[v][t]));
+            }
+          }
+        } else {
+#pragma unroll 1
+          for (int u = 7; u >= 0; --u) {
+            const int i = 8 * c + u;
+            if (i > n - 3) continue;
+            const double tau = tau_[i];
+            const double* __restrict__ w = buf + u * LD + gl;
+            double vr[RT], a0[NV], a1[NV];
+#pragma unroll
+            for (int t = T0; t < RT; ++t) vr[t] = w[G * t];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a0[v] = a1[v] = 0.0;
+#pragma unroll
+            for (int t = T0; t < RT; t += 2)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) {
+                a0[v] = fma(vr[t], z[v][t], a0[v]);
+                if (t + 1 < RT) a1[v] = fma(vr[t + 1], z[v][t + 1], a1[v]);
+              }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a0[v] += a1[v];
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) a0[v] += __shfl_xor_sync(0xffffffffu, a0[v], o);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a0[v] *= -tau;
+#pragma unroll
+            for (int t = T0; t < RT; ++t)
+#pragma unroll
+              for (int v = 0; v < NV; ++v) z[v][t] = fma(a0[v], vr[t], z[v][t]);
+          }
+        }
+      }
+    };
+    constexpr int TH = RT / 2;         // lane rows before TH: matrix rows before G TH
+    const int ch = min(c0 + 1, G * TH / 8);  // stages from ch on touch none of them
+    if (c0 >= 0) fetch(c0);
+    stages(std::integral_constant<int, TH>{}, c0, ch);
+    stages(std::integral_constant<int, 0>{}, ch - 1, 0);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      if (j0 + v >= kvec) break;
-      double* y = Y + (size_t)(j0 + v) * n;
+      const int j = j0 + v * NG + g;
+      if (j < kvec) {
 #pragma unroll
-      for (int t = 0; t < RT; ++t) {
-        const int r = lane + 32 * t;
-        if (r < n) y[r] = z[v][t];
+        for (int t = 0; t < RT; ++t) {
+          const int r = gl + G * t;
+          if (r < n) Y[(size_t)j * n + r] = z[v][t];
+        }
       }
     }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
-// The reflectors of column i (v_{i+1} = 1, v_r = A(r, i) below) applied from the last to the
-// first. Up to n = 64 each lane holds 2 rows and a warp 4 vectors (the n/2 or so occupied vectors
-// then keep all eight warps busy, which measured faster than 8 vectors on four warps).
-__device__ void back_transform(int n, int kvec, const double* __restrict__ A, double* Y, const EigenScratch& s_) {
-  if (n <= 64) back_transform_t<2, 4>(n, kvec, A, Y, s_.tau);
-  else if (n <= 128) back_transform_t<4, 4>(n, kvec, A, Y, s_.tau);
-  else back_transform_t<kRowT, 2>(n, kvec, A, Y, s_.tau);
+// Split by size: the n x kvec block of vectors is spread over the CTA's registers, in as few passes as
+// they allow. Shared scratch: 16 rows of G RT doubles.
+constexpr int back_scratch(int n) {
+  return 16 * (n <= 32 ? 32 : n <= 64 ? 64 : n <= 96 ? 96 : n <= 128 ? 128 : n <= 160 ? 160 : 256);
+}
+__device__ __noinline__ void back_transform(int n, int kvec, const double* __restrict__ V, const double* __restrict__ Yt,
+                                            double* Y, const EigenScratch& s_) {
+  double* sh = in_shared(s_.sh);
+  const double* tau = in_shared(s_.tau);
+  if (n <= 32) back_transform_t<8, 4, 1>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 64 && kvec <= 32) back_transform_t<8, 8, 1>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 64) back_transform_t<8, 8, 2>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 96) back_transform_t<8, 12, 2>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 128 && kvec > 64) back_transform_t<16, 8, 4>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 128) back_transform_t<8, 16, 2>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 160) back_transform_t<16, 10, 3>(n, kvec, V, Yt, Y, tau, sh);
+  else back_transform_t<16, 16, 2>(n, kvec, V, Yt, Y, tau, sh);
 }
 
 // All eigenvalues of the saved tridiagonal (d, e) -- used once at the end for the MO energies.

@@ -506,7 +506,8 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
   L.off_eig = off;
   off += align(7 * nmax * 8 + (2 * nmax + 2) * 4);
   L.off_union = off;
-  const int fixed_union = std::max(20 * amax, 2 * 16 * 65);
+  const int fixed_union =
+      std::max(std::max(20 * amax, 2 * 16 * 65), std::max(tri_scratch(nmax), back_scratch(nmax)));
   auto fit = [&](int budget) {
     int nsm = nmax;
     for (; nsm > 0; --nsm)
@@ -528,7 +529,8 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
     }
   }
   L.nsm = nsm;
-  L.bytes = off + std::max(fixed_union, nsm * (nsm + 1) / 2) * 8;
+  L.uni = std::max(fixed_union, nsm * (nsm + 1) / 2);
+  L.bytes = off + L.uni * 8;
   return L;
 }
 

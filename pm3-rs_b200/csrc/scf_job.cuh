@@ -62,9 +62,8 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
   double* Pa = c.P[0];
   double* Pb = c.Q[0];
   if (J.guess == 2) {  // core-Hamiltonian orbitals, aufbau (scf.rs:929-932, 969-975)
-    double* Ap = pack_input(c, c.H, nullptr, 0.0);
     const int kv = uhf ? na : na;  // na >= nb
-    eigensolve(c, Ap, n < kv + 1 ? n : kv + 1, kv, c.Vt, c.tri_a + 2 * n, nullptr);
+    eigensolve(c, sym_input(c.H, nullptr, 0.0), n < kv + 1 ? n : kv + 1, kv, c.Vt, c.tri_a + 2 * n, nullptr);
     density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
     if (uhf) density(c, c.Vt, nb, 1.0, Pb, Pb, 0.0);
   } else if (J.guess == 4) {  // given (learned) density, scaled to the electron count
@@ -92,12 +91,10 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
       __syncthreads();
       build_fock(c, Pt, Pa, Pb, c.F, c.G);
     }
-    double* Ap = pack_input(c, c.F, nullptr, 0.0);
-    eigensolve(c, Ap, n < na + 1 ? n : na + 1, na, c.Vt, c.tri_a + 2 * n, nullptr);
+    eigensolve(c, sym_input(c.F, nullptr, 0.0), n < na + 1 ? n : na + 1, na, c.Vt, c.tri_a + 2 * n, nullptr);
     density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
     if (uhf) {
-      Ap = pack_input(c, c.G, nullptr, 0.0);
-      eigensolve(c, Ap, n < nb + 1 ? n : nb + 1, nb, c.Vb, c.tri_b + 2 * n, nullptr);
+      eigensolve(c, sym_input(c.G, nullptr, 0.0), n < nb + 1 ? n : nb + 1, nb, c.Vb, c.tri_b + 2 * n, nullptr);
       density(c, c.Vb, nb, 1.0, Pb, Pb, 0.0);
     }
   } else {
@@ -294,37 +291,23 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
     // ---- diagonalise (level shift for UHF only, scf.rs:1416-1418) and rebuild densities
     double sq_a, sq_b = 0.0;
     {
-      double* Ap = n <= A.sm.nsm ? c.Asm : c.Ag;
-      const double* __restrict__ coef = c.coef;
-      const double* __restrict__ hist = c.hist;
-      const double shift = J.shift;
       for (int spin = 0; spin < (uhf && !paired ? 2 : 1); ++spin) {
         const double* Pproj = spin == 0 ? Pc : Qc;
-        const double* Fnew = spin == 0 ? Fa : Fb;
-        // rows to warps, columns to lanes (coalesced reads of the history matrices)
-        for (int r = tid >> 5; r < n; r += kWarps)
-          for (int col = tid & 31; col <= r; col += 32) {
-            const size_t ix = (size_t)r * n + col;
-            double v;
-            if (use_hist) {
-              v = 0.0;
-              for (int l = 0; l < len; ++l) {
-                const double* bl = hist + (size_t)((head + l) % depth) * slot_mats * nn;
-                v = fma(coef[l], bl[(spin == 0 ? 0 : 2 * nn) + ix], v);
-              }
-            } else {
-              v = Fnew[ix];
-            }
-            if (uhf && shift != 0.0) v += shift * ((r == col ? 1.0 : 0.0) - Pproj[ix]);
-            Ap[tri(r) + col] = v;
-          }
-        __syncthreads();
+        SymInput in = sym_input(spin == 0 ? Fa : Fb, Pproj, uhf ? J.shift : 0.0);
+        if (use_hist) {
+          in.hist = c.hist + (spin == 0 ? 0 : 2 * nn);
+          in.coef = c.coef;
+          in.head = head;
+          in.len = len;
+          in.depth = depth;
+          in.stride = slot_mats * nn;
+        }
         if (spin == 0) {
-          eigensolve(c, Ap, kva, na, c.Vt, eps_a, c.tri_a, iter > 0, c.tri_a + 3 * n);
+          eigensolve(c, in, kva, na, c.Vt, eps_a, c.tri_a, iter > 0, c.tri_a + 3 * n);
           sq_a = density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pc, Pn, uhf ? J.damping : 0.0);
           mark(c, kPhDensity);
         } else {
-          eigensolve(c, Ap, kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
+          eigensolve(c, in, kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
           sq_b = density(c, c.Vb, nb, 1.0, Qc, Qn, J.damping);
           mark(c, kPhDensity);
         }
@@ -550,8 +533,7 @@ __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
     for (size_t k = tid; k < nn; k += kThreads) part += Qc[k] * c.G[k];
     part = block_sum(part, c.red);
     mark(c, kPhFock);
-    double* Ap = pack_input(c, c.G, Qc, J.shift);
-    eigensolve(c, Ap, kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
+    eigensolve(c, sym_input(c.G, Qc, J.shift), kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
     const double sq = density(c, c.Vb, nb, 1.0, Qc, Qn, J.damping);
     mark(c, kPhDensity);
     if (tid == 0) {
@@ -612,7 +594,8 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
   c.dpk = up;
   c.jacc = up + 10 * amax;
   c.tile = up;
-  c.Asm = up;
+  c.es.sh = up;
+  c.es.sh_doubles = L.uni;
 
   slot_ptrs(c, args.work + (size_t)blockIdx.x * args.slot, args.nmax);
 

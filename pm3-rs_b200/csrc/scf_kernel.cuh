@@ -68,7 +68,8 @@ struct JobOut {
 // Byte offsets of the dynamic shared-memory carve-up (computed on the host).
 struct SmemLayout {
   int amax;      // atoms per molecule this launch supports
-  int nsm;       // largest n whose packed matrix lives in shared memory
+  int nsm;       // largest n whose packed matrix would fit the union
+  int uni;       // doubles in the union of the phases' scratch
   int off_int, off_dbl, off_eig, off_union;
   int bytes;
 };
@@ -153,7 +154,6 @@ struct Ctx {
   double* dpk;          // [amax*10] packed densities (Fock phase)
   double* jacc;         // [amax*10] Coulomb accumulators (Fock phase)
   double* tile;         // GEMM tiles
-  double* Asm;          // packed matrix (eigen phase)
   EigenScratch es;
   unsigned long long* ph;  // [kPhases] shared accumulators
   long long tmark;
@@ -614,35 +614,26 @@ __device__ void adiis_coeffs_warp(int m, const double* mg, double* out, double* 
 }
 
 // ------------------------------------------------------------------- eigensolve + density
-// Pack sym(X) [+ shift (I - Pproj)] into the eigen input (shared or global).
-__device__ double* pack_input(Ctx& c, const double* X, const double* Pproj, double shift) {
-  const int n = c.n;
-  double* Ap = n <= c.A->sm.nsm ? c.Asm : c.Ag;
-  // rows to warps, columns to lanes (coalesced reads)
-  for (int r = threadIdx.x >> 5; r < n; r += kWarps)
-    for (int col = threadIdx.x & 31; col <= r; col += 32) {
-      double v = X[(size_t)r * n + col];
-      if (shift != 0.0) v += shift * ((r == col ? 1.0 : 0.0) - Pproj[(size_t)r * n + col]);
-      Ap[tri(r) + col] = v;
-    }
-  __syncthreads();
-  return Ap;
+// The eigen input X [+ shift (I - Pproj)].
+__device__ __forceinline__ SymInput sym_input(const double* X, const double* Pproj, double shift) {
+  return SymInput{X, nullptr, nullptr, 0, 0, 1, 0, Pproj, shift};
 }
 
-// Diagonalise the packed matrix: kval lowest eigenvalues into lam_out, kvec eigenvectors
+// Diagonalise the matrix: kval lowest eigenvalues into lam_out, kvec eigenvectors
 // into Y (rows). The tridiagonal (d, e) is saved to `tri_save` (2n) for the final MO energies.
 // With `warm`, lam_out holds the same eigenvalues from the previous SCF iteration and `dlam`
 // their last change; both seed the eigenvalue search and are updated. Without it dlam is reset.
-__device__ void eigensolve(Ctx& c, double* Ap, int kval, int kvec, double* Y, double* lam_out, double* tri_save,
+__device__ void eigensolve(Ctx& c, const SymInput& in, int kval, int kvec, double* Y, double* lam_out, double* tri_save,
                            bool warm = false, double* dlam = nullptr) {
   const int n = c.n;
   mark(c, kPhPack);
-  tridiagonalize(n, Ap, c.es);
-  if (tri_save && threadIdx.x == 0)
-    for (int i = 0; i < n; ++i) {
+  tridiagonalize(n, in, c.Ag, c.tf, c.es);
+  if (tri_save)
+    for (int i = threadIdx.x; i < n; i += kThreads) {
       tri_save[i] = c.es.d[i];
       tri_save[n + i] = c.es.e[i];
     }
+  __syncthreads();  // the splitting of T writes e
   mark(c, kPhTridiag);
   const bool seeded = warm && dlam != nullptr;
   tridiag_eigenvalues(n, kval, c.es, seeded ? lam_out : nullptr, seeded ? dlam : nullptr);
@@ -652,9 +643,9 @@ __device__ void eigensolve(Ctx& c, double* Ap, int kval, int kvec, double* Y, do
   }
   mark(c, kPhEigval);
   if (kvec > 0) {
-    tridiag_vectors(n, kvec, Y, c.tf, c.es);
+    const double* Yt = tridiag_vectors(n, kvec, c.tf, c.es);
     mark(c, kPhEigvec);
-    back_transform(n, kvec, Ap, Y, c.es);
+    back_transform(n, kvec, c.Ag, Yt, Y, c.es);
   }
   __syncthreads();
   mark(c, kPhBack);
