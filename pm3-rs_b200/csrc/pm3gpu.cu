@@ -593,12 +593,16 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
   c->last_ctas = per_sm;
   c->last_nsm = L.nsm;
   const long long slot = slot_doubles(nmax, wcap);
-  size_t free_b = 0, total_b = 0;
-  CUDA_TRY(c, cudaMemGetInfo(&free_b, &total_b));
   long long grid = std::min<long long>(nj + nr, (long long)c->sms * per_sm);
-  const size_t budget = (size_t)(0.6 * (double)(free_b + c->work.bytes));
-  while (grid > 1 && (size_t)grid * slot * 8 > budget) --grid;
-  if ((size_t)grid * slot * 8 > budget) return fail(c, PM3GPU_RESOURCE_LIMIT, "SCF workspace exceeds device memory");
+  // The free-memory query takes a driver-wide lock (75 us alone, milliseconds to tens of them while other processes use the
+  // machine's GPUs): asked only when the workspace has to grow.
+  if ((size_t)grid * slot * 8 > c->work.bytes) {
+    size_t free_b = 0, total_b = 0;
+    CUDA_TRY(c, cudaMemGetInfo(&free_b, &total_b));
+    const size_t budget = (size_t)(0.6 * (double)(free_b + c->work.bytes));
+    while (grid > 1 && (size_t)grid * slot * 8 > budget) --grid;
+    if ((size_t)grid * slot * 8 > budget) return fail(c, PM3GPU_RESOURCE_LIMIT, "SCF workspace exceeds device memory");
+  }
   CUDA_TRY(c, c->work.ensure((size_t)grid * slot * 8));
   CUDA_TRY(c, c->jobs.ensure(sizeof(JobDesc) * (nj + nr)));
   CUDA_TRY(c, c->out.ensure(sizeof(JobOut) * (nj + nr)));
