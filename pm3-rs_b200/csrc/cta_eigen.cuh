@@ -1208,7 +1208,7 @@ __device__ __forceinline__ void back_transform_t(int n, int kvec, const double* 
 
 // Split by size: the n x kvec block of vectors is spread over the CTA's registers, in as few passes as
 // they allow. Shared scratch: 16 rows of G RT doubles.
-constexpr int back_scratch(int n) {
+__host__ __device__ constexpr int back_scratch(int n) {
   return 16 * (n <= 32 ? 32 : n <= 64 ? 64 : n <= 96 ? 96 : n <= 128 ? 128 : n <= 160 ? 160 : 256);
 }
 __device__ __noinline__ void back_transform(int n, int kvec, const double* __restrict__ V, const double* __restrict__ Yt,

@@ -626,10 +626,10 @@ class LargeSolver {
     ++c_->launches;
     if (Pb)
       large::fock_pairs_kernel<true><<<gp, large::kBlock, 0, c_->stream>>>(
-          m_, B_.W.as<double>(), B_.H.as<double>(), B_.dpk.as<double>(), B_.jacc.as<double>(), Pt, Pa, Pb, F, G);
+          m_, B_.W.as<double>(), B_.H.as<double>(), Pt, Pa, Pb, F, G);
     else
       large::fock_pairs_kernel<false><<<gp, large::kBlock, 0, c_->stream>>>(
-          m_, B_.W.as<double>(), B_.H.as<double>(), B_.dpk.as<double>(), B_.jacc.as<double>(), Pt, Pa, Pb, F, G);
+          m_, B_.W.as<double>(), B_.H.as<double>(), Pt, Pa, Pb, F, G);
     large::fock_diag_kernel<<<gN, large::kBlock, 0, c_->stream>>>(m_, B_.H.as<double>(), B_.jacc.as<double>(), Pt, Pa,
                                                                   Pb, F, G);
     c_->launches += 3;

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kBlock) core_pairs_kernel(Mol m, double* H, do
     const int a = (hu || !hv) ? u : v, b = a == u ? v : u;
     double* w = const_cast<double*>(pair_block(m, W, u, v));
     ecc += core_pair(m.elem[m.z[a]], m.elem[m.z[b]], eu, ev, *m.pairs, m.xyz + 3 * (size_t)a, m.xyz + 3 * (size_t)b,
-                     m.ao[a], m.ao[b], (size_t)m.n, nullptr, nullptr, w, H);
+                     m.ao[a], m.ao[b], (size_t)m.n, nullptr, nullptr, w, 1, H);
   }
   block_partial(ecc, partial);
 }
@@ -229,9 +229,8 @@ __global__ void __launch_bounds__(kBlock) coulomb_atoms_kernel(Mol m, const doub
   }
 }
 template <bool UHF>
-__global__ void __launch_bounds__(kBlock) fock_pairs_kernel(Mol m, const double* W, const double* H, const double* dpk,
-                                                            double* jacc, const double* Pt, const double* Pa,
-                                                            const double* Pb, double* F, double* G) {
+__global__ void __launch_bounds__(kBlock) fock_pairs_kernel(Mol m, const double* W, const double* H, const double* Pt,
+                                                            const double* Pa, const double* Pb, double* F, double* G) {
   const long long np = pair_count(m.N);
   for (long long t = blockIdx.x * (long long)kBlock + threadIdx.x; t < np; t += (long long)gridDim.x * kBlock) {
     int u, v;
@@ -241,9 +240,9 @@ __global__ void __launch_bounds__(kBlock) fock_pairs_kernel(Mol m, const double*
     const int a = (hu || !hv) ? u : v, b = a == u ? v : u;
     const double* w = pair_block(m, W, u, v);
     const int oa = m.ao[a], ob = m.ao[b];
-    if (hu && hv) fock_pair<4, 4, UHF, false>(m.n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-    else if (hu || hv) fock_pair<4, 1, UHF, false>(m.n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-    else fock_pair<1, 1, UHF, false>(m.n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
+    if (hu && hv) fock_pair<4, 4, UHF>(m.n, oa, ob, H, w, Pt, Pa, Pb, F, G);
+    else if (hu || hv) fock_pair<4, 1, UHF>(m.n, oa, ob, H, w, Pt, Pa, Pb, F, G);
+    else fock_pair<1, 1, UHF>(m.n, oa, ob, H, w, Pt, Pa, Pb, F, G);
   }
 }
 // atom-diagonal blocks: H + one-centre J - K + two-centre J

@@ -493,8 +493,9 @@ int g_scf_static_smem = 1024;
 // two CTAs share an SM as long as at least 90% of the launch's jobs still fit in shared memory.
 // ctas: 0 = choose (two CTAs per SM when at least 90% of the batch keeps its packed eigen input
 // in the smaller layout), 1 or 2 = the autotuner's measured choice.
+// wcap: doubles of the launch's largest pair table; the union is widened to hold it when two CTAs per SM allow.
 SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const std::vector<int>* naos = nullptr,
-                       int ctas = 0) {
+                       int ctas = 0, long long wcap = 0) {
   SmemLayout L{};
   L.amax = amax;
   auto align = [](int b) { return (b + 15) & ~15; };
@@ -502,12 +503,11 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
   L.off_int = off;
   off += align((3 * amax + 1 + 16) * 4);
   L.off_dbl = off;
-  off += align(amax * 8 + (3 * amax + 4 * kMaxDepth * kWarps + 4 * kMaxDepth + 2 * kMaxDepth * kMaxDepth + kMaxDepth + 8) * 8);
+  off += align(((3 * amax + 1) / 2 * 2 + 4 * kMaxDepth * kWarps + 4 * kMaxDepth + 2 * kMaxDepth * kMaxDepth + kMaxDepth + 8) * 8);
   L.off_eig = off;
   off += align(7 * nmax * 8 + (2 * nmax + 2) * 4);
   L.off_union = off;
-  const int fixed_union =
-      std::max(std::max(20 * amax, 2 * 16 * 65), std::max(tri_scratch(nmax), back_scratch(nmax)));
+  const int fixed_union = union_keep(nmax);
   auto fit = [&](int budget) {
     int nsm = nmax;
     for (; nsm > 0; --nsm)
@@ -530,6 +530,10 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
   }
   L.nsm = nsm;
   L.uni = std::max(fixed_union, nsm * (nsm + 1) / 2);
+  if (smem_per_sm > 0 && wcap > 0) {
+    const long long want = fixed_union + wcap;
+    if (off + want * 8 <= smem_per_sm / 2 - 1024 - g_scf_static_smem) L.uni = std::max(L.uni, (int)want);
+  }
   L.bytes = off + L.uni * 8;
   return L;
 }
@@ -586,7 +590,7 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
     }
   for (const JobDesc& j : jobs) naos.push_back(j.nao);
   const int ctas = c->force_ctas ? c->force_ctas : tune_lookup(c->tune_batch, nmax, 0);
-  const SmemLayout L = make_layout(amax, nmax, c->smem_optin, c->smem_per_sm, &naos, ctas);
+  const SmemLayout L = make_layout(amax, nmax, c->smem_optin, c->smem_per_sm, &naos, ctas, wcap);
   int per_sm = 0;
   CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scf_batch_kernel, kThreads, L.bytes));
   if (per_sm < 1) return fail(c, PM3GPU_RESOURCE_LIMIT, "SCF kernel does not fit on an SM");

@@ -86,10 +86,7 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
     if (!uhf) {
       build_fock(c, Pa, nullptr, nullptr, c.F, nullptr);
     } else {
-      double* Pt = c.Vb + nn;
-      for (size_t k = tid; k < nn; k += kThreads) Pt[k] = Pa[k] + Pb[k];
-      __syncthreads();
-      build_fock(c, Pt, Pa, Pb, c.F, c.G);
+      build_fock(c, nullptr, Pa, Pb, c.F, c.G);
     }
     eigensolve(c, sym_input(c.F, nullptr, 0.0), n < na + 1 ? n : na + 1, na, c.Vt, c.tri_a + 2 * n, nullptr);
     density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
@@ -187,32 +184,11 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
         Dh = base + 2 * nn;
       }
     }
-    double e_elec;
-    if (!uhf) {
-      build_fock(c, Pc, nullptr, nullptr, Fa, nullptr);
-      double part = 0.0;
-      for (size_t k = tid; k < nn; k += kThreads) part = fma(Pc[k], c.H[k] + Fa[k], part);
-      e_elec = 0.5 * block_sum(part, c.red);
-      mark(c, kPhFock);
-    } else if (paired) {  // alpha here; the helper builds F_beta and returns its energy part
-      double* Pt = c.Vb + nn;
-      for (size_t k = tid; k < nn; k += kThreads) Pt[k] = Pc[k] + Qc[k];
-      __syncthreads();
-      build_fock(c, Pt, Pc, nullptr, Fa, nullptr);
-      double part = 0.0;
-      for (size_t k = tid; k < nn; k += kThreads) part += Pt[k] * c.H[k] + Pc[k] * Fa[k];
-      e_elec = block_sum(part, c.red);  // completed with the helper's part below
-      mark(c, kPhFock);
-    } else {
-      double* Pt = c.Vb + nn;  // scratch right after Vb (slot reserves it)
-      for (size_t k = tid; k < nn; k += kThreads) Pt[k] = Pc[k] + Qc[k];
-      __syncthreads();
-      build_fock(c, Pt, Pc, Qc, Fa, Fb);
-      double part = 0.0;
-      for (size_t k = tid; k < nn; k += kThreads) part += Pt[k] * c.H[k] + Pc[k] * Fa[k] + Qc[k] * Fb[k];
-      e_elec = 0.5 * block_sum(part, c.red);
-      mark(c, kPhFock);
-    }
+    // twice the electronic energy; paired: the helper builds F_beta and returns its part
+    double e_elec = uhf ? build_fock(c, nullptr, Pc, Qc, Fa, paired ? nullptr : Fb)
+                        : build_fock(c, Pc, nullptr, nullptr, Fa, nullptr);
+    if (!paired) e_elec *= 0.5;
+    mark(c, kPhFock);
 
     // ---- accelerator (scf.rs:1240-1259 RHF; 1398-1413 UHF)
     bool use_hist = false;
@@ -352,10 +328,7 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
   double* Qf = c.Q[c.cur];
   double* Pt = Pf;
   if (!uhf) {
-    build_fock(c, Pf, nullptr, nullptr, c.F, nullptr);
-    double part = 0.0;
-    for (size_t k = tid; k < nn; k += kThreads) part = fma(Pf[k], c.H[k] + c.F[k], part);
-    o.electronic = 0.5 * block_sum(part, c.red);
+    o.electronic = 0.5 * build_fock(c, Pf, nullptr, nullptr, c.F, nullptr);
     o.spin_max = 0.0;
   } else {
     Pt = c.Vb + nn;
@@ -365,10 +338,7 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
       mx = fmax(mx, fabs(Pf[k] - Qf[k]));
     }
     o.spin_max = block_max(mx, c.red);
-    build_fock(c, Pt, Pf, Qf, c.F, c.G);
-    double part = 0.0;
-    for (size_t k = tid; k < nn; k += kThreads) part += Pt[k] * c.H[k] + Pf[k] * c.F[k] + Qf[k] * c.G[k];
-    o.electronic = 0.5 * block_sum(part, c.red);
+    o.electronic = 0.5 * build_fock(c, Pt, Pf, Qf, c.F, c.G);
   }
   o.converged = converged ? 1 : 0;
   o.iterations = iterations;
@@ -447,7 +417,8 @@ __device__ __forceinline__ void slot_ptrs(Ctx& c, double* slot, int nmax) {
   c.hist = slot + 17 * nn;   // 32 nn: accelerator history
   c.tri_a = slot + 49 * nn;
   c.tri_b = c.tri_a + 4 * nmax;  // per spin: saved tridiagonal (2n), eigenvalues (n), their change (n)
-  c.W = c.tri_b + 4 * nmax;
+  c.Wg = c.tri_b + 4 * nmax;
+  c.W = c.Wg;
 }
 
 // The beta spin of CTA L's unrestricted job (offer generation `mygen`, already taken by this
@@ -497,7 +468,6 @@ __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
   c.Vt = own_vt;
   c.Ag = own_ag;
   c.tf = own_tf;
-  double* Pt = own_vb + nn;
   double* eps_b = c.tri_b + 2 * n;
   const int kvb = n < nb + 1 ? n : nb + 1;
   for (;; ++iter) {
@@ -526,12 +496,7 @@ __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
     const double* Pc = c.P[cur];
     double* Qc = c.Q[cur];
     double* Qn = c.Q[1 - cur];
-    for (size_t k = tid; k < nn; k += kThreads) Pt[k] = Pc[k] + Qc[k];
-    __syncthreads();
-    build_fock(c, Pt, Qc, nullptr, c.G, nullptr);
-    double part = 0.0;
-    for (size_t k = tid; k < nn; k += kThreads) part += Qc[k] * c.G[k];
-    part = block_sum(part, c.red);
+    const double part = build_fock(c, nullptr, Qc, Pc, c.G, nullptr);
     mark(c, kPhFock);
     eigensolve(c, sym_input(c.G, Qc, J.shift), kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
     const double sq = density(c, c.Vb, nb, 1.0, Qc, Qn, J.damping);
@@ -559,13 +524,11 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
   int* ip = reinterpret_cast<int*>(smem + L.off_int);
   c.sz = ip;
   c.soff = ip + amax;
-  c.sprow = ip + 2 * amax;
+  c.order = ip + 2 * amax;
   c.iv = ip + 3 * amax + 1;
-  long long* lp = reinterpret_cast<long long*>(smem + L.off_dbl);
-  c.sroff = lp;
-  double* dp = reinterpret_cast<double*>(lp + amax);
+  double* dp = reinterpret_cast<double*>(smem + L.off_dbl);
   c.sxyz = dp;
-  dp += 3 * amax;
+  dp += (3 * amax + 1) & ~1;  // the reduction scratch is read 16 bytes at a time
   c.red = dp;
   dp += 4 * kMaxDepth * kWarps;
   c.misc = dp;
@@ -591,11 +554,8 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
   c.es.nblk = eip + nm + 1;
   c.es.vinfo = eip + nm + 2;
   double* up = reinterpret_cast<double*>(smem + L.off_union);
-  c.dpk = up;
-  c.jacc = up + 10 * amax;
   c.tile = up;
   c.es.sh = up;
-  c.es.sh_doubles = L.uni;
 
   slot_ptrs(c, args.work + (size_t)blockIdx.x * args.slot, args.nmax);
 

@@ -142,8 +142,8 @@ struct Ctx {
   // shared
   int* sz;              // [amax] Z of each atom
   int* soff;            // [amax] first AO
-  int* sprow;           // [amax+1] prefix of packed sizes
-  long long* sroff;     // [amax] pair-table row offsets
+  int* order;           // [amax] atoms with p orbitals first, then the others, each in the molecule's order
+  int nh;               // atoms with p orbitals
   double* sxyz;         // [3 amax]
   double* red;          // reduction scratch
   double* misc;         // broadcast scalars
@@ -151,14 +151,12 @@ struct Ctx {
   double* mg;           // [8*8] <D_i,F_j>
   double* coef;         // [kMaxDepth+1]
   int* iv;              // small ints
-  double* dpk;          // [amax*10] packed densities (Fock phase)
-  double* jacc;         // [amax*10] Coulomb accumulators (Fock phase)
-  double* tile;         // GEMM tiles
+  double* tile;         // the union: GEMM tiles, the Fock build's packed rows, the eigensolver's scratch
   EigenScratch es;
   unsigned long long* ph;  // [kPhases] shared accumulators
   long long tmark;
   // global (slot)
-  double *H, *P[2], *Q[2], *F, *G, *Vt, *Vb, *Ag, *tf, *hist, *W, *tri_a, *tri_b;
+  double *H, *P[2], *Q[2], *F, *G, *Vt, *Vb, *Ag, *tf, *hist, *W, *Wg, *tri_a, *tri_b;  // W: the pair table, in Wg or in shared memory
   int cur;              // which P/Q buffer is current
 };
 
@@ -171,10 +169,6 @@ __device__ __forceinline__ void mark(Ctx& c, int phase) {
 }
 
 __device__ __forceinline__ bool heavy(const Ctx& c, int a) { return c.A->elem[c.sz[a]].norb == 4; }
-__device__ __forceinline__ int psize(const Ctx& c, int a) { return heavy(c, a) ? 10 : 1; }
-__device__ __forceinline__ long long woff(const Ctx& c, int u, int v) {
-  return c.sroff[u] + (long long)psize(c, u) * (c.sprow[v] - c.sprow[u + 1]);
-}
 // pair index t -> (u < v)
 __device__ __forceinline__ void pair_uv(int N, int t, int& u, int& v) {
   const double b = 2.0 * N - 1.0;
@@ -186,6 +180,35 @@ __device__ __forceinline__ void pair_uv(int N, int t, int& u, int& v) {
   v = t - uu * (2 * N - uu - 1) / 2 + uu + 1;
 }
 
+// The same for one molecule's short lists, in single precision with the integer correction.
+__device__ __forceinline__ void pair_uv_short(int N, int t, int& u, int& v) {
+  const float b = 2.0f * N - 1.0f;
+  int uu = max(0, min(N - 2, (int)((b - sqrtf(fmaxf(b * b - 8.0f * t, 0.0f))) * 0.5f)));
+  while (uu > 0 && uu * (2 * N - uu - 1) / 2 > t) --uu;
+  while ((uu + 1) * (2 * N - uu - 2) / 2 <= t) ++uu;
+  u = uu;
+  v = t - uu * (2 * N - uu - 1) / 2 + uu + 1;
+}
+
+// A molecule's atom pairs by kind, so that the threads of a warp do the same work: both atoms with p orbitals
+// (heavy, nhh pairs), one of them (nhl), none (nll). The pair table W holds the integrals of a kind
+// with the pair index fastest (100, 10 and 1 rows of nhh, nhl and nll values), so that a warp reads
+// consecutive addresses. Rows of packed densities and Coulomb sums: 10 per heavy atom, then 1 per light one.
+struct PairKinds {
+  int nh, nl, nhh, nhl, nll, rows;
+  __device__ __forceinline__ PairKinds(int nh_, int N)
+      : nh(nh_), nl(N - nh_), nhh(nh_ * (nh_ - 1) / 2), nhl(nh_ * (N - nh_)), nll((N - nh_) * (N - nh_ - 1) / 2),
+        rows(10 * nh_ + (N - nh_)) {}
+  __device__ __forceinline__ int row(int i) const { return i < nh ? 10 * i : 10 * nh + (i - nh); }
+};
+
+// Doubles of the union that the phases of an n-function molecule use beside a pair table kept there.
+__host__ __device__ constexpr int union_keep(int n) {
+  const int a = 2 * 16 * 65, b = tri_scratch(n), c = back_scratch(n), d = 25 * n;
+  const int m = a > b ? a : b, k = c > d ? c : d;
+  return m > k ? m : k;
+}
+
 // ------------------------------------------------------------------ job setup + H_core
 __device__ void setup_job(Ctx& c) {
   const KernelArgs& A = *c.A;
@@ -195,32 +218,39 @@ __device__ void setup_job(Ctx& c) {
     for (int k = 0; k < 3; ++k) c.sxyz[3 * a + k] = A.xyz[3 * (size_t)(c.job.atom0 + a) + k];
   }
   __syncthreads();
-  if (tid == 0) {
-    int off = 0, pr = 0;
-    for (int a = 0; a < c.N; ++a) {
-      c.soff[a] = off;
-      off += A.elem[c.sz[a]].norb;
-      c.sprow[a] = pr;
-      pr += psize(c, a);
-    }
-    c.sprow[c.N] = pr;
-    long long ro = 0;
-    for (int a = 0; a < c.N; ++a) {
-      c.sroff[a] = ro;
-      ro += (long long)psize(c, a) * (pr - c.sprow[a + 1]);
-    }
+  // first AO of every atom and the heavy-first order, by counting the heavy atoms before each
+  for (int a = tid; a < c.N; a += kThreads) {
+    int hv = 0;
+    for (int k = 0; k < a; ++k) hv += heavy(c, k) ? 1 : 0;
+    c.soff[a] = a + 3 * hv;
+    c.iv[0] = 0;
+    if (a == c.N - 1) c.iv[1] = hv + (heavy(c, a) ? 1 : 0);
   }
+  __syncthreads();
+  c.nh = c.iv[1];
+  for (int a = tid; a < c.N; a += kThreads) {
+    const int hv = (c.soff[a] - a) / 3;  // heavy atoms before a
+    c.order[heavy(c, a) ? hv : c.nh + (a - hv)] = a;
+  }
+  // A small molecule keeps its pair table at the end of the union (n = 60 and 12 + 12 atoms: 63 KB); with
+  // helpers another CTA may have to read it, from global memory.
+  const PairKinds K(c.nh, c.N);
+  const int wsize = 100 * K.nhh + 10 * K.nhl + K.nll;
+  const bool near = A.help == nullptr && union_keep(c.n) + wsize <= A.sm.uni;
+  c.W = near ? c.tile + (A.sm.uni - wsize) : c.Wg;
+  c.es.sh_doubles = near ? A.sm.uni - wsize : A.sm.uni;
   __syncthreads();
 }
 
 // One atom pair of H_core (hamiltonian.rs:191-344): both atoms' electron-core attraction blocks
-// (added to their packed diagonal accumulators), the pair table block W in (a, b) orientation (a
-// the atom with more orbitals), and the resonance block H_ab = (beta_i + beta_j)/2 S_ij written to
+// (stored to hacc_a, hacc_b), the pair table block W in (a, b) orientation (a
+// the atom with more orbitals; consecutive integrals ws apart), and the resonance block H_ab = (beta_i + beta_j)/2 S_ij written to
 // both triangles of H (row stride n). Returns the pair's core-core energy (repulsion.rs:57-120),
 // evaluated with the atoms in the caller's (u, v) order.
 __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb, const ElemDev& eu, const ElemDev& ev,
                                             const PairDev& pp, const double* xa, const double* xb, int oa, int ob,
-                                            size_t n, double* hacc_a, double* hacc_b, double* w, double* H) {
+                                            size_t n, double* hacc_a, double* hacc_b, double* w, int ws,
+                                            double* H) {
   const double d[3] = {xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]};
   const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
   const double dv[3] = {d[0] / r * r, d[1] / r * r, d[2] / r * r};
@@ -228,9 +258,9 @@ __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb
   if (hacc_a) {  // null: the caller adds the electron-core blocks per atom itself
     double blk[10];
     core_attraction(ea, eb, dv, blk);
-    for (int k = 0; k < (ea.norb == 4 ? 10 : 1); ++k) atomicAdd(&hacc_a[k], blk[k]);
+    for (int k = 0; k < (ea.norb == 4 ? 10 : 1); ++k) hacc_a[k] = blk[k];
     core_attraction(eb, ea, mdv, blk);
-    for (int k = 0; k < (eb.norb == 4 ? 10 : 1); ++k) atomicAdd(&hacc_b[k], blk[k]);
+    for (int k = 0; k < (eb.norb == 4 ? 10 : 1); ++k) hacc_b[k] = blk[k];
   }
   const double ir = 1.0 / r;
   double R[9];
@@ -243,14 +273,14 @@ __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb
     double ri[4];
     local4(ee_pole(ea), eb.rho0, rv, ri);
     for (int kk = 0; kk < 4; ++kk)
-      for (int ll = 0; ll <= kk; ++ll) w[pk(kk, ll)] = w4(ri, R, kk, ll);
+      for (int ll = 0; ll <= kk; ++ll) w[(size_t)pk(kk, ll) * ws] = w4(ri, R, kk, ll);
   } else {
     double ri[22];
     local22(ee_pole(ea), ee_pole(eb), rv, ri);
     for (int kk = 0; kk < 4; ++kk)
       for (int ll = 0; ll <= kk; ++ll)
         for (int mm = 0; mm < 4; ++mm)
-          for (int nn = 0; nn <= mm; ++nn) w[pk(kk, ll) * 10 + pk(mm, nn)] = w22(ri, R, kk, ll, mm, nn);
+          for (int nn = 0; nn <= mm; ++nn) w[(size_t)(pk(kk, ll) * 10 + pk(mm, nn)) * ws] = w22(ri, R, kk, ll, mm, nn);
   }
   double s[16];
   overlap_block(ea, eb, d, s);
@@ -267,33 +297,78 @@ __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb
   return core_core(eu, ev, pp, dd);
 }
 
+// Item t of the pair kinds in turn: atoms (positions in the heavy-first order), table entry and its stride.
+__device__ __forceinline__ void pair_item(const PairKinds& K, int t, int& ia, int& ib, size_t& w0, int& ws) {
+  if (t < K.nhh) {
+    pair_uv_short(K.nh, t, ia, ib);
+    w0 = t;
+    ws = K.nhh;
+  } else if (t < K.nhh + K.nhl) {
+    const int q = t - K.nhh;
+    ia = q / K.nl;
+    ib = K.nh + q - ia * K.nl;
+    w0 = (size_t)100 * K.nhh + q;
+    ws = K.nhl;
+  } else {
+    const int q = t - K.nhh - K.nhl;
+    pair_uv_short(K.nl, q, ia, ib);
+    ia += K.nh;
+    ib += K.nh;
+    w0 = (size_t)100 * K.nhh + (size_t)10 * K.nhl + q;
+    ws = K.nll;
+  }
+}
+
+// Sums every packed row r over the partner atoms, in their order: S[y rows + r] holds partner y's part. With few rows
+// the partners are split over 2 or 4 groups of threads; out[g rows + r] gets group g's sum, and the number of groups is returned.
+__device__ __forceinline__ int gather_rows(const PairKinds& K, int N, const double* __restrict__ S, double* out) {
+  const int groups = K.rows <= 64 ? 4 : (K.rows <= 128 ? 2 : 1), per = kThreads / groups;
+  const int g = threadIdx.x / per, y0 = N * g / groups, y1 = N * (g + 1) / groups;
+  for (int r = threadIdx.x % per; r < K.rows; r += per) {
+    const int self = r < 10 * K.nh ? r / 10 : K.nh + (r - 10 * K.nh);
+    double acc = 0.0;
+    for (int y = y0; y < y1; y += 8) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = y + u < y1 && y + u != self ? S[(size_t)(y + u) * K.rows + r] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += x[u];
+    }
+    out[g * K.rows + r] = acc;
+  }
+  return groups;
+}
+
 // H_core (hamiltonian.rs:191-344) and the pair table W; returns the core-core energy
-// (repulsion.rs:13-27) to every thread.
-__device__ double build_core(Ctx& c) {
+// (repulsion.rs:13-27) to every thread. Each pair writes its two electron-core blocks to its own place
+// in scratch and every element of an atom's block is summed over the partners in order: sums of the shared accumulators
+// with atomics took most of the time (5.8M of 6M cycles at n = 148, 61 atoms).
+__device__ __noinline__ double build_core(Ctx& c) {
   const KernelArgs& A = *c.A;
   const int n = c.n, N = c.N, tid = threadIdx.x;
-  double* hacc = c.jacc;  // [N*10] diagonal-block accumulators
-  for (int k = tid; k < N * 10; k += kThreads) hacc[k] = 0.0;
-  __syncthreads();
+  const PairKinds K(c.nh, N);
+  double* S = c.hist;  // [N][rows]
   double ecc = 0.0;
-  const int npairs = N * (N - 1) / 2;
-  for (int t = tid; t < npairs; t += kThreads) {
-    int u, v;
-    pair_uv(N, t, u, v);
-    const bool hu = heavy(c, u), hv = heavy(c, v);
-    const int a = (hu || !hv) ? u : v, b = a == u ? v : u;
+  for (int t = tid; t < K.nhh + K.nhl + K.nll; t += kThreads) {
+    int ia, ib, ws;
+    size_t w0;
+    pair_item(K, t, ia, ib, w0, ws);
+    const int a = c.order[ia], b = c.order[ib], u = min(a, b), v = max(a, b);
     ecc += core_pair(A.elem[c.sz[a]], A.elem[c.sz[b]], A.elem[c.sz[u]], A.elem[c.sz[v]], *A.pairs, c.sxyz + 3 * a,
-                     c.sxyz + 3 * b, c.soff[a], c.soff[b], (size_t)n, hacc + a * 10, hacc + b * 10, c.W + woff(c, u, v),
-                     c.H);
+                     c.sxyz + 3 * b, c.soff[a], c.soff[b], (size_t)n, S + (size_t)ib * K.rows + K.row(ia),
+                     S + (size_t)ia * K.rows + K.row(ib), c.W + w0, ws, c.H);
   }
+  __syncthreads();
+  double* sums = in_shared(c.tile);
+  const int groups = gather_rows(K, N, S, sums);
   __syncthreads();
   // diagonal blocks: U + sum of electron-core attractions
   for (int k = tid; k < N * 16; k += kThreads) {
-    const int a = k >> 4, mu = (k >> 2) & 3, nu = k & 3;
+    const int i = k >> 4, mu = (k >> 2) & 3, nu = k & 3, a = c.order[i];
     const ElemDev& e = A.elem[c.sz[a]];
     if (mu >= e.norb || nu >= e.norb) continue;
-    double h = hacc[a * 10 + pk(mu, nu)];
-    if (mu == nu) h += mu == 0 ? e.uss : e.upp;
+    double h = mu == nu ? (mu == 0 ? e.uss : e.upp) : 0.0;
+    for (int g = 0; g < groups; ++g) h += sums[g * K.rows + K.row(i) + pk(mu, nu)];
     c.H[(size_t)(c.soff[a] + mu) * n + c.soff[a] + nu] = h;
   }
   __syncthreads();
@@ -301,46 +376,19 @@ __device__ double build_core(Ctx& c) {
 }
 
 // ------------------------------------------------------------------------ Fock build
-// Two-centre part of one atom pair (fock.rs:106-193): Coulomb sums into the atoms' packed
-// accumulators and the exchange block F_ab = H_ab - K_ab, written to both triangles. NA / NB are
-// the orbital counts of atom a (the heavier one) and b, so every loop has a fixed trip count and
-// every array stays in registers. W is the pair's (PA x PB) row-major integral block.
-// kJ = false leaves out the two-centre Coulomb sums into jacc (the whole-GPU path adds them per
-// atom in a fixed order instead of with atomics).
-// SPIN = true builds one spin's Fock matrix of an unrestricted job, F = H + J(Pt) - K(Pa) (the
-// first spin of the UHF form alone), for a job whose two spins run on two CTAs.
-template <int NA, int NB, bool UHF, bool kJ = true, bool SPIN = false>
-__device__ __forceinline__ void fock_pair(int n, int a, int b, int oa, int ob, const double* __restrict__ dpk,
-                                          double* jacc, const double* __restrict__ H, const double* __restrict__ w,
-                                          const double* Pt, const double* Pa, const double* Pb, double* F, double* G) {
-  constexpr int PA = NA == 4 ? 10 : 1, PB = NB == 4 ? 10 : 1;
-  if (kJ) {  // Coulomb: J_a[p] += sum_q W[p][q] Pb_q, J_b[q] += sum_p Pa_p W[p][q]
-    double db[PB], jb[PB];
-#pragma unroll
-    for (int q = 0; q < PB; ++q) {
-      db[q] = dpk[b * 10 + q];
-      jb[q] = 0.0;
-    }
-#pragma unroll
-    for (int p = 0; p < PA; ++p) {
-      const double da = dpk[a * 10 + p];
-      double acc = 0.0;
-#pragma unroll
-      for (int q = 0; q < PB; ++q) {
-        const double wv = w[p * PB + q];
-        acc = fma(db[q], wv, acc);
-        jb[q] = fma(da, wv, jb[q]);
-      }
-      atomicAdd(&jacc[a * 10 + p], acc);
-    }
-#pragma unroll
-    for (int q = 0; q < PB; ++q) atomicAdd(&jacc[b * 10 + q], jb[q]);
-  }
+// Exchange block of one atom pair on the whole-GPU path (fock.rs:106-193): F_ab = H_ab - K_ab, written to both
+// triangles. NA / NB are the orbital counts of atom a (the heavier one) and b, so every loop has a fixed trip
+// count. W is the pair's (PA x PB) row-major integral block.
+template <int NA, int NB, bool UHF>
+__device__ __forceinline__ void fock_pair(int n, int oa, int ob, const double* __restrict__ H,
+                                          const double* __restrict__ w, const double* Pt, const double* Pa,
+                                          const double* Pb, double* F, double* G) {
+  constexpr int PB = NB == 4 ? 10 : 1;
   // exchange: K[mu][la] = sum_{nu, si} X[nu][si] (mu nu | la si), one spin at a time
 #pragma unroll
   for (int spin = 0; spin < (UHF ? 2 : 1); ++spin) {
-    const double* X = (UHF || SPIN) ? (spin == 0 ? Pa : Pb) : Pt;
-    const double xs = (UHF || SPIN) ? 1.0 : 0.5;
+    const double* X = UHF ? (spin == 0 ? Pa : Pb) : Pt;
+    const double xs = UHF ? 1.0 : 0.5;
     double* out = spin == 0 ? F : G;
     double x[NA * NB];
 #pragma unroll
@@ -363,99 +411,178 @@ __device__ __forceinline__ void fock_pair(int n, int a, int b, int oa, int ob, c
   }
 }
 
-// F = H + J(Pt) - K(Ps) (fock.rs:285-332). Pt = total density; for RHF Ps = Pt/2 (pb == null),
-// for UHF two spin Focks F (from Pa) and G (from Pb) are built in one pass.
-// With Pa given and Pb null, one spin of an unrestricted job: F = H + J(Pt) - K(Pa) (G unused).
-__device__ void build_fock(Ctx& c, const double* Pt, const double* Pa, const double* Pb, double* F, double* G) {
-  const KernelArgs& A = *c.A;
-  const int n = c.n, N = c.N, tid = threadIdx.x;
-  const bool uhf = Pb != nullptr;
-  const bool spin1 = !uhf && Pa != nullptr;
-  // stage packed atomic densities (fock.rs:93-100) and zero the Coulomb accumulators
-  for (int k = tid; k < N * 10; k += kThreads) {
-    const int a = k / 10, p = k % 10;
-    const int no = A.elem[c.sz[a]].norb;
-    c.jacc[k] = 0.0;
-    double v = 0.0;
-    if (no == 4 || p == 0) {
-      int hi, lo;
-      unpk(p, hi, lo);
-      const int oa = c.soff[a];
-      v = Pt[(size_t)(oa + hi) * n + oa + lo];
-      if (hi != lo) v *= 2.0;
+// One pair of the per-CTA Fock build for one spin density X (times xs): the exchange block F_ab = H_ab - K_ab to both
+// triangles and, with kJ, the pair's Coulomb parts J_a[p] = sum_q W[p][q] d_b[q] and
+// J_b[q] = sum_p d_a[p] W[p][q] to sa and sb. The integrals stream through once, row by row with the next row's loads in
+// flight: element (mu nu | la si) adds to the up to four exchange elements that share it. Returns the
+// pair's part of sum P (H + F), both triangles.
+template <int NA, int NB, bool kJ>
+__device__ __forceinline__ double fock_item(int n, int oa, int ob, const double* __restrict__ w, size_t ws,
+                                            const double* da, const double* db, double* sa, double* sb,
+                                            const double* __restrict__ H, const double* __restrict__ X, double xs,
+                                            double* __restrict__ F) {
+  constexpr int PA = NA == 4 ? 10 : 1, PB = NB == 4 ? 10 : 1;
+  double x[NA][NB], k[NA][NB], jb[PB], wv[PB], wn[PB];
+#pragma unroll
+  for (int q = 0; q < PB; ++q) wn[q] = w[q * ws];
+#pragma unroll
+  for (int i = 0; i < NA; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      x[i][j] = xs * X[(size_t)(oa + i) * n + ob + j];
+      k[i][j] = 0.0;
     }
-    c.dpk[k] = v;
-  }
-  __syncthreads();
-  const int npairs = N * (N - 1) / 2;
-  {
-    const int* __restrict__ sprow = c.sprow;
-    const int* __restrict__ soff = c.soff;
-    const long long* __restrict__ sroff = c.sroff;
-    const double* __restrict__ W = c.W;
-    const double* __restrict__ H = c.H;
-    const double* __restrict__ dpk = c.dpk;
-    double* jacc = c.jacc;
-    for (int t = tid; t < npairs; t += kThreads) {
-      int u, v;
-      pair_uv(N, t, u, v);
-      const int su = sprow[u + 1] - sprow[u], sv = sprow[v + 1] - sprow[v];  // packed sizes: 10 sp, 1 s
-      const bool hu = su == 10, hv = sv == 10;
-      const int a = (hu || !hv) ? u : v, b = a == u ? v : u;
-      const double* w = W + sroff[u] + (long long)su * (sprow[v] - sprow[u + 1]);
-      const int oa = soff[a], ob = soff[b];
-      if (hu && hv) {
-        if (uhf) fock_pair<4, 4, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else if (spin1) fock_pair<4, 4, false, true, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else fock_pair<4, 4, false>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-      } else if (hu || hv) {
-        if (uhf) fock_pair<4, 1, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else if (spin1) fock_pair<4, 1, false, true, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else fock_pair<4, 1, false>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-      } else {
-        if (uhf) fock_pair<1, 1, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else if (spin1) fock_pair<1, 1, false, true, true>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
-        else fock_pair<1, 1, false>(n, a, b, oa, ob, dpk, jacc, H, w, Pt, Pa, Pb, F, G);
+#pragma unroll
+  for (int q = 0; q < PB; ++q) jb[q] = 0.0;
+#pragma unroll
+  for (int mu = 0; mu < NA; ++mu)
+#pragma unroll
+    for (int nu = 0; nu <= mu; ++nu) {
+      const int p = pk(mu, nu);
+#pragma unroll
+      for (int q = 0; q < PB; ++q) wv[q] = wn[q];
+      if (p + 1 < PA) {
+#pragma unroll
+        for (int q = 0; q < PB; ++q) wn[q] = w[((p + 1) * PB + q) * ws];
       }
-    }
-  }
-  __syncthreads();
-  // atom-diagonal blocks: H + one-centre J - K + two-centre J
-  for (int k = tid; k < N * 16; k += kThreads) {
-    const int a = k >> 4, mu = (k >> 2) & 3, nu = k & 3;
-    const ElemDev& e = A.elem[c.sz[a]];
-    const int no = e.norb;
-    if (mu >= no || nu >= no) continue;
-    const int oa = c.soff[a];
-    double ja = 0.0, ka = 0.0, kb = 0.0;
-    for (int la = 0; la < no; ++la)
-      for (int si = 0; si < no; ++si) {
-        const double coul = oc_integral(e, mu, nu, la, si), exch = oc_integral(e, mu, la, nu, si);
-        const size_t ix = (size_t)(oa + la) * n + oa + si;
-        ja = fma(Pt[ix], coul, ja);
-        if (uhf) {
-          ka = fma(Pa[ix], exch, ka);
-          kb = fma(Pb[ix], exch, kb);
-        } else if (spin1) {
-          ka = fma(Pa[ix], exch, ka);
-        } else {
-          ka = fma(0.5 * Pt[ix], exch, ka);
+      if (kJ) {
+        const double dp = da[p];
+        double acc = 0.0;
+#pragma unroll
+        for (int q = 0; q < PB; ++q) {
+          acc = fma(db[q], wv[q], acc);
+          jb[q] = fma(dp, wv[q], jb[q]);
         }
+        sa[p] = acc;
       }
-    const size_t ix = (size_t)(oa + mu) * n + oa + nu;
-    const double base = c.H[ix] + c.jacc[a * 10 + pk(mu, nu)] + ja;
-    F[ix] = base - ka;
-    if (uhf) G[ix] = base - kb;
+#pragma unroll
+      for (int la = 0; la < NB; ++la)
+#pragma unroll
+        for (int si = 0; si <= la; ++si) {
+          const double e = wv[pk(la, si)];
+          k[mu][la] = fma(x[nu][si], e, k[mu][la]);
+          if (mu != nu) k[nu][la] = fma(x[mu][si], e, k[nu][la]);
+          if (la != si) k[mu][si] = fma(x[nu][la], e, k[mu][si]);
+          if (mu != nu && la != si) k[nu][si] = fma(x[mu][la], e, k[nu][si]);
+        }
+    }
+  if (kJ) {
+#pragma unroll
+    for (int q = 0; q < PB; ++q) sb[q] = jb[q];
   }
-  __syncthreads();
+  double en = 0.0;
+#pragma unroll
+  for (int mu = 0; mu < NA; ++mu)
+#pragma unroll
+    for (int la = 0; la < NB; ++la) {
+      const double h = H[(size_t)(oa + mu) * n + ob + la], f = h - k[mu][la];
+      F[(size_t)(oa + mu) * n + ob + la] = f;
+      F[(size_t)(ob + la) * n + oa + mu] = f;
+      en = fma(x[mu][la], h + f, en);
+    }
+  return 2.0 * en / xs;
 }
 
-// sum_ij X_ij Y_ij over n x n
-__device__ __forceinline__ double fdot(const Ctx& c, const double* X, const double* Y) {
-  double s = 0.0;
-  const size_t nn = (size_t)c.n * c.n;
-  for (size_t k = threadIdx.x; k < nn; k += kThreads) s = fma(X[k], Y[k], s);
-  return block_sum(s, c.red);
+// The off-diagonal blocks of one spin's Fock matrix over all pairs of the molecule; with kJ also every pair's Coulomb
+// parts to S (gather_rows' layout). Returns this thread's part of sum P (H + F).
+template <bool kJ>
+__device__ __noinline__ double fock_pairs(const Ctx& c, const double* dpk_, double* S, const double* X, double xs, double* F) {
+  const PairKinds K(c.nh, c.N);
+  const int n = c.n, tid = threadIdx.x;
+  const int* soff = in_shared(c.soff);
+  const int* order = in_shared(c.order);
+  const double* dpk = in_shared(dpk_);
+  const double* __restrict__ W = c.W;
+  const double* __restrict__ H = c.H;
+  double en = 0.0;
+  auto run = [&](auto na, auto nb, int t) {
+    int ia, ib, ws;
+    size_t w0;
+    pair_item(K, t, ia, ib, w0, ws);
+    const int ra = K.row(ia), rb = K.row(ib);
+    en += fock_item<decltype(na)::value, decltype(nb)::value, kJ>(n, soff[order[ia]], soff[order[ib]], W + w0, ws, dpk + ra, dpk + rb,
+                                                                 S + (size_t)ib * K.rows + ra, S + (size_t)ia * K.rows + rb, H, X, xs, F);
+  };
+  using I4 = std::integral_constant<int, 4>;
+  using I1 = std::integral_constant<int, 1>;
+  for (int t = tid; t < K.nhh; t += kThreads) run(I4{}, I4{}, t);
+  // the other kinds from the last thread on: the warps that had one heavy pair less begin first
+  for (int t = kThreads - 1 - tid; t < K.nhl; t += kThreads) run(I4{}, I1{}, K.nhh + t);
+  for (int t = kThreads - 1 - tid; t < K.nll; t += kThreads) run(I1{}, I1{}, K.nhh + K.nhl + t);
+  return en;
+}
+
+// F = H + J(Pt) - K(Ps) (fock.rs:285-332), and the sum over the built spins of Ps (H + F) to all threads. Pt = total
+// density (null: Pa + Pb). RHF: Pa null, Ps = Pt / 2. UHF: two spin Focks F (from Pa) and G (from Pb).
+// With Pa and Pb given and G null, the spin of Pa alone.
+// Every Coulomb part goes to its own place in scratch and is summed per packed row in a fixed order, so
+// repeated solves agree bit for bit (atomics on the atoms' accumulators, 32 lanes at one address, took
+// most of the build: 680k cycles at n = 148, 61 atoms).
+__device__ __noinline__ double build_fock(Ctx& c, const double* Pt, const double* Pa, const double* Pb, double* F, double* G) {
+  const KernelArgs& A = *c.A;
+  const int n = c.n, N = c.N, tid = threadIdx.x;
+  const PairKinds K(c.nh, N);
+  double* dpk = in_shared(c.tile);  // [rows] packed densities (fock.rs:93-100)
+  double* sums = dpk + K.rows;      // [groups][rows] Coulomb sums
+  const int* soff = in_shared(c.soff);
+  const int* order = in_shared(c.order);
+  for (int r = tid; r < K.rows; r += kThreads) {
+    const int i = r < 10 * K.nh ? r / 10 : K.nh + (r - 10 * K.nh);
+    int hi, lo;
+    unpk(r - K.row(i), hi, lo);
+    const int o = soff[order[i]];
+    const size_t ix = (size_t)(o + hi) * n + o + lo;
+    const double v = Pt ? Pt[ix] : Pa[ix] + Pb[ix];
+    dpk[r] = hi != lo ? 2.0 * v : v;
+  }
+  __syncthreads();
+  double* S = c.tf;  // [N][rows]
+  double en = fock_pairs<true>(c, dpk, S, Pa ? Pa : Pt, Pa ? 1.0 : 0.5, F);
+  if (G) en += fock_pairs<false>(c, dpk, S, Pb, 1.0, G);
+  __syncthreads();
+  const int groups = gather_rows(K, N, S, sums);
+  __syncthreads();
+  // atom-diagonal blocks: H + one-centre J - K (fock.rs:244-282) + two-centre J
+  for (int k = tid; k < 16 * K.nh + K.nl; k += kThreads) {
+    const bool hv = k < 16 * K.nh;
+    const int i = hv ? k >> 4 : K.nh + (k - 16 * K.nh), mu = hv ? (k >> 2) & 3 : 0, nu = hv ? k & 3 : 0;
+    const int a = order[i], o = soff[a];
+    const ElemDev& e = A.elem[c.sz[a]];
+    const double hpp = 0.5 * (e.gpp - e.gp2);
+    auto tot = [&](int x, int y) {
+      const size_t ix = (size_t)(o + x) * n + o + y;
+      return Pt ? Pt[ix] : Pa[ix] + Pb[ix];
+    };
+    double j = 0.0;
+    for (int g = 0; g < groups; ++g) j += sums[g * K.rows + K.row(i) + pk(mu, nu)];
+    // integrals (mu mu | x x) and (mu x | mu x) of the atom
+    auto gm = [&](int x, int y) { return x == y ? (x == 0 ? e.gss : e.gpp) : (x == 0 || y == 0 ? e.gsp : e.gp2); };
+    auto hm = [&](int x, int y) { return x == y ? (x == 0 ? e.gss : e.gpp) : (x == 0 || y == 0 ? e.hsp : hpp); };
+    if (mu == nu) {
+      for (int x = 0; x < (hv ? 4 : 1); ++x) j = fma(tot(x, x), gm(mu, x), j);
+    } else {
+      j = fma(hm(mu, nu), tot(mu, nu) + tot(nu, mu), j);
+    }
+    const size_t ix = (size_t)(o + mu) * n + o + nu;
+    const double h = c.H[ix];
+#pragma unroll
+    for (int spin = 0; spin < 2; ++spin) {
+      if (spin == 1 && !G) break;
+      const double* P = spin == 1 ? Pb : (Pa ? Pa : Pt);
+      const double xs = Pa ? 1.0 : 0.5;
+      auto den = [&](int x, int y) { return P[(size_t)(o + x) * n + o + y]; };
+      double ex = 0.0;
+      if (mu == nu) {
+        for (int x = 0; x < (hv ? 4 : 1); ++x) ex = fma(den(x, x), hm(mu, x), ex);
+      } else {
+        ex = fma(gm(mu, nu), den(mu, nu), hm(mu, nu) * den(nu, mu));
+      }
+      const double f = h + j - xs * ex;
+      (spin == 1 ? G : F)[ix] = f;
+      en = fma(P[ix], h + f, en);
+    }
+  }
+  return block_sum(en, c.red);  // its barriers also publish F
 }
 
 // E = F P - P F into E (scf.rs:1039-1054): one GEMM, then antisymmetrise in place.
