@@ -1,5 +1,5 @@
-// CTA-level building blocks: reductions and a shared-memory tiled FP64 GEMM used by the
-// per-molecule SCF (commutator F.P and the density C_occ C_occ^T).
+// CTA-level building blocks: reductions and the symmetric-form FP64 products of the
+// per-molecule SCF (commutator F P - P F and the density C_occ C_occ^T).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -61,89 +61,124 @@ __device__ __forceinline__ void block_sums(double (&v)[K], double* red, double* 
   __syncthreads();
 }
 
-// This thread's 4 + 4 elements of the 64 x 16 chunks of op(A) and op(B) at k0 (the layout of
-// cta_gemm's shared tiles), zero outside the matrices.
-template <bool TA, bool TB>
-__device__ __forceinline__ void cta_gemm_fetch(double (&pa)[4], double (&pb)[4], int k0, int i0, int j0, int m, int n,
-                                               int k, const double* __restrict__ A, int lda,
-                                               const double* __restrict__ B, int ldb) {
-  constexpr int BM = 64, BN = 64, BK = 16;
+// Sums 32 values over the warp, lane l ending with the total of value l: 31 shuffles (5 per value when summed one by one).
+__device__ __forceinline__ double warp_sum32(double (&v)[32]) {
+  const int l = threadIdx.x & 31;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = threadIdx.x + q * kThreads;
-    int ii, kk;
-    if (TA) { ii = e % BM; kk = e / BM; } else { kk = e % BK; ii = e / BK; }
-    const int gi = i0 + ii, gk = k0 + kk;
-    pa[q] = (gi < m && gk < k) ? (TA ? A[(size_t)gk * lda + gi] : A[(size_t)gi * lda + gk]) : 0.0;
-    int jj;
-    if (TB) { kk = e % BK; jj = e / BK; } else { jj = e % BN; kk = e / BN; }
-    const int gj = j0 + jj, gk2 = k0 + kk;
-    pb[q] = (gj < n && gk2 < k) ? (TB ? B[(size_t)gj * ldb + gk2] : B[(size_t)gk2 * ldb + gj]) : 0.0;
-  }
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const double send = (l & o) ? v[k] : v[k + o], keep = (l & o) ? v[k + o] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  return v[0];
 }
 
-// C (m x n) = alpha * op(A) * op(B) with op(A) m x k, op(B) k x n; A, B row-major in global
-// memory. TA: A stored as k x m (use its transpose). Each output element goes through
-// `epi(i, j, value)`. Tiles of 64 x 64, k-chunks of 16 (the next chunk's loads in flight while the
-// current one is multiplied), 4 x 4 outputs per thread; `tile` needs 2 * 64 * 17 doubles of shared
-// memory. If `lower_only`, only tiles touching the lower
-// triangle (i >= j) are computed (for symmetric results).
-template <bool TA, bool TB, class Epi>
-__device__ void cta_gemm(int m, int n, int k, double alpha, const double* __restrict__ A, int lda,
-                         const double* __restrict__ B, int ldb, double* tile, bool lower_only, Epi epi) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  double* As = tile;              // [BK][BM+1]
-  double* Bs = tile + BK * (BM + 1);  // [BK][BN+1]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads
-  const int tiles_m = (m + BM - 1) / BM, tiles_n = (n + BN - 1) / BN;
-  for (int t = 0; t < tiles_m * tiles_n; ++t) {
-    const int bi = t / tiles_n, bj = t % tiles_n;
-    if (lower_only && bj > bi) continue;  // uniform across the CTA
-    const int i0 = bi * BM, j0 = bj * BN;
-    double acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    // the next k-chunk's elements are loaded into registers while the current one is multiplied
-    // (each thread holds 4 of op(A) and 4 of op(B): 64 x 16 / 256 threads)
-    double pa[4], pb[4];
-    cta_gemm_fetch<TA, TB>(pa, pb, 0, i0, j0, m, n, k, A, lda, B, ldb);
-    for (int k0 = 0; k0 < k; k0 += BK) {
-      __syncthreads();  // the previous chunk's products have read As, Bs
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + q * kThreads;
-        int ii, kk;
-        if (TA) { ii = e % BM; kk = e / BM; } else { kk = e % BK; ii = e / BK; }
-        As[kk * (BM + 1) + ii] = pa[q];
-        int jj;
-        if (TB) { kk = e % BK; jj = e / BK; } else { jj = e % BN; kk = e / BN; }
-        Bs[kk * (BN + 1) + jj] = pb[q];
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool in) {  // zero when !in
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int bytes = in ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+// Lower triangle of an n x n product of symmetric form on the FP64 tensor instructions, k summed over K:
+//   kComm:  C_ij = sum_k A_ik B_jk - B_ik A_jk   (A, B symmetric, row-major n x n, K = n)
+//   else:   C_ij = sum_k A_ki A_kj               (A row-major K x n)
+// A stage of 8 k-values of every row passes through shared memory once for all blocks (8-byte asynchronous copies, two
+// stages in flight), and the warps keep 16 x 16 blocks of the lower triangle in registers, five each: one pass up to
+// n = 128, two up to 176. Shared layout [k / 4][row][4]: the half-warps' fragment loads are 16 consecutive doubles. `sh`: lower_scratch(n) doubles.
+// Each element goes through epi(i, j, value), i >= j. What bounds it: FP64 issue (n^3 / 64 cycles for the commutator).
+__host__ __device__ constexpr int lower_scratch(int n, bool comm) { return 2 * 8 * ((n + 15) / 16 * 16) * (comm ? 2 : 1); }
+template <bool kComm, class Epi>
+__device__ __forceinline__ void lower_product(int n, int K, const double* __restrict__ A, const double* __restrict__ B,
+                                              double* sh, Epi epi) {
+  constexpr int kOwn = 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tg = lane & 3;
+  const int nb = (n + 15) / 16, M = 16 * nb, blocks = nb * (nb + 1) / 2;
+  const int stage = 8 * M * (kComm ? 2 : 1);  // doubles of one stage: A, then B
+  const int steps = (K + 7) / 8;
+  auto fill = [&](int st) {
+    double* dst = sh + (st & 1) * stage;
+    const int k0 = 8 * st;
+    if (kComm) {  // rows of 8 consecutive values
+      for (int e = tid; e < 8 * M; e += kThreads) {
+        const int r = e >> 3, k = e & 7;
+        const bool in = r < n && k0 + k < K;
+        const int at = ((k >> 2) * M + r) * 4 + (k & 3), ix = in ? r * n + k0 + k : 0;
+        cp_async8(dst + at, A + ix, in);
+        cp_async8(dst + 8 * M + at, B + ix, in);
       }
-      __syncthreads();
-      if (k0 + BK < k) cta_gemm_fetch<TA, TB>(pa, pb, k0 + BK, i0, j0, m, n, k, A, lda, B, ldb);
-#pragma unroll
-      for (int kk = 0; kk < BK; ++kk) {
-        double a[4], b[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          a[q] = As[kk * (BM + 1) + ty + 16 * q];
-          b[q] = Bs[kk * (BN + 1) + tx + 16 * q];
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+    } else {  // one warp a k-value
+      const int k = warp;
+      for (int r = lane; r < M; r += 32) {
+        const bool in = r < n && k0 + k < K;
+        cp_async8(dst + ((k >> 2) * M + r) * 4 + (k & 3), A + (in ? (k0 + k) * n + r : 0), in);
       }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int first = 0; first < blocks; first += kWarps * kOwn) {
+    double acc[kOwn][2][4];
+    int bi[kOwn], bj[kOwn];
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int q = 0; q < kOwn; ++q) {
+      const int t = first + warp + kWarps * q;
+      int I = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+      while (I * (I + 1) / 2 > t) --I;
+      while ((I + 1) * (I + 2) / 2 <= t) ++I;
+      bi[q] = t < blocks ? I : -1;
+      bj[q] = t - I * (I + 1) / 2;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int gi = i0 + ty + 16 * p, gj = j0 + tx + 16 * q;
-        if (gi < m && gj < n) epi(gi, gj, alpha * acc[p][q]);
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[q][h][e] = 0.0;
+    }
+    fill(0);
+    for (int st = 0; st < steps; ++st) {
+      if (st + 1 < steps) {
+        fill(st + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
+      __syncthreads();
+      const double* __restrict__ sa = sh + (st & 1) * stage;
+      const double* __restrict__ sb = sa + 8 * M;
+#pragma unroll
+      for (int q = 0; q < kOwn; ++q) {
+        if (bi[q] < 0) continue;  // uniform in the warp
+        const int ri = (16 * bi[q] + g) * 4 + tg, rj = (16 * bj[q] + g) * 4 + tg;
+        const double af[4] = {sa[ri], sa[ri + 32], sa[4 * M + ri], sa[4 * M + ri + 32]};
+        if (kComm) {
+          const double pf[4] = {sb[ri], sb[ri + 32], sb[4 * M + ri], sb[4 * M + ri + 32]};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            mma_f64(acc[q][h], af, sb[rj + 32 * h], sb[4 * M + rj + 32 * h]);
+            mma_f64(acc[q][h], pf, -sa[rj + 32 * h], -sa[4 * M + rj + 32 * h]);
+          }
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) mma_f64(acc[q][h], af, sa[rj + 32 * h], sa[4 * M + rj + 32 * h]);
+        }
+      }
+      __syncthreads();  // this stage is filled again next
+    }
+#pragma unroll
+    for (int q = 0; q < kOwn; ++q) {
+      if (bi[q] < 0) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 16 * bi[q] + g + 8 * (e >> 1), j = 16 * bj[q] + 8 * h + 2 * tg + (e & 1);
+          if (i < n && j <= i) epi(i, j, acc[q][h][e]);
+        }
+    }
   }
   __syncthreads();
 }

@@ -22,6 +22,99 @@ __device__ __forceinline__ bool wait_at_least(const volatile int* p, int want) {
   return false;
 }
 
+// The accelerator of one iteration (scf.rs:1065-1173, 1240-1259, 1398-1413): the density joins the history, the new Gram row
+// against the surviving entries and the new diagonal, then the CDIIS or A-DIIS weights of len + 1
+// entries to c.coef. Returns whether they are usable.
+__device__ __noinline__ bool diis_step(Ctx& c, const JobDesc& J, bool uhf, bool keep, int len, int head, int depth,
+                                       int slot_mats, const double* __restrict__ Fa, const double* __restrict__ Fb,
+                                       const double* __restrict__ Ea, const double* __restrict__ Eb, double* __restrict__ Dh,
+                                       const double* __restrict__ Pc) {
+  const int n = c.n, tid = threadIdx.x;
+  const size_t nn = (size_t)n * n;
+  double* bg = in_shared(c.bg);
+  double* mg = in_shared(c.mg);
+  double* coef = in_shared(c.coef);
+  double* red = in_shared(c.red);
+  int* iv = in_shared(c.iv);
+  // acc[l], acc[8 + l], acc[16 + l]: <E_l, E>, <D, F_l>, <D_l, F>; acc[24], acc[25]: <E, E>, <D, F>
+  static_assert(kMaxDepth == 8, "the sums of one warp are reduced 32 at a time");
+  double acc[32];
+#pragma unroll
+  for (int q = 0; q < 32; ++q) acc[q] = 0.0;
+  int off[kMaxDepth];
+#pragma unroll
+  for (int l = 0; l < kMaxDepth; ++l) off[l] = ((head + l) % depth) * slot_mats * (int)nn;
+  const double* __restrict__ hist = c.hist;
+  const int in = (int)nn;
+  // Every product pairs two symmetric (F, D) or two antisymmetric (E) matrices, so the sum
+  // over all n^2 elements is the diagonal plus twice the strict lower triangle: half the
+  // history reads. All loads of an element are issued before the first is used (with a branch around each
+  // history entry they were waited for one entry at a time: 470k cycles at n = 148).
+  int r = 0;
+  for (int t = tid; t < n * (n + 1) / 2; t += kThreads) {
+    while ((r + 1) * (r + 2) / 2 <= t) ++r;
+    const int col = t - r * (r + 1) / 2, k = r * n + col;
+    const double wgt = col == r ? 1.0 : 2.0;
+    double vE[kMaxDepth], vF[kMaxDepth], vD[kMaxDepth];
+#pragma unroll
+    for (int l = 0; l < kMaxDepth; ++l) {
+      vE[l] = l < len ? hist[off[l] + in + k] : 0.0;
+      vF[l] = l < len && keep ? hist[off[l] + k] : 0.0;
+      vD[l] = l < len && keep ? hist[off[l] + 2 * in + k] : 0.0;
+    }
+    const double e = Ea[k], f = Fa[k], dn = keep ? Pc[k] : 0.0;
+    if (keep) Dh[k] = dn;
+    const double we = wgt * e, wf = wgt * f, wd = wgt * dn;
+    acc[24] = fma(we, e, acc[24]);
+    acc[25] = fma(wd, f, acc[25]);
+#pragma unroll
+    for (int l = 0; l < kMaxDepth; ++l) {
+      acc[l] = fma(vE[l], we, acc[l]);
+      acc[8 + l] = fma(wd, vF[l], acc[8 + l]);
+      acc[16 + l] = fma(vD[l], wf, acc[16 + l]);
+    }
+    if (uhf) {
+      const double eb = Eb[k], web = wgt * eb;
+      acc[24] = fma(web, eb, acc[24]);
+#pragma unroll
+      for (int l = 0; l < kMaxDepth; ++l)
+        if (l < len) acc[l] = fma(hist[off[l] + 3 * in + k], web, acc[l]);
+    }
+  }
+  const double sum = warp_sum32(acc);
+  __syncthreads();
+  red[(tid & 31) * kWarps + (tid >> 5)] = sum;
+  __syncthreads();
+  if (tid < 32) {  // the rest on the first warp
+    const double t = sum8(red + tid * kWarps);
+    const double ee = __shfl_sync(0xffffffffu, t, 24);
+    if (tid < len) {
+      bg[tid * kMaxDepth + len] = t;
+      bg[len * kMaxDepth + tid] = t;
+    } else if (tid >= 8 && tid < 8 + len) {
+      mg[len * kMaxDepth + tid - 8] = t;
+    } else if (tid >= 16 && tid < 16 + len) {
+      mg[(tid - 16) * kMaxDepth + len] = t;
+    } else if (tid == 24) {
+      bg[len * kMaxDepth + len] = t;
+    } else if (tid == 25) {
+      mg[len * kMaxDepth + len] = t;
+    }
+    __syncwarp();
+    const int m = len + 1;
+    bool ok;
+    if (!uhf && J.accel == 2 && sqrt(ee) > J.adiis_switch) {
+      ok = keep && m >= 2;
+      if (ok) adiis_coeffs_warp(m, mg, coef);
+    } else {
+      ok = cdiis_coeffs_warp(m, bg, coef);
+    }
+    if (tid == 0) iv[0] = ok ? 1 : 0;
+  }
+  __syncthreads();
+  return iv[0] != 0;
+}
+
 __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, int jidx = -1) {
   const KernelArgs& A = *c.A;
   c.job = job;
@@ -195,72 +288,9 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
     if (J.accel != 0) {
       commutator(c, Fa, Pc, Ea);
       if (uhf) commutator(c, Fb, Qc, Eb);
-      if (keep)
-        for (size_t k = tid; k < nn; k += kThreads) Dh[k] = Pc[k];
-      __syncthreads();
       mark(c, kPhCommutator);
-      // new Gram row against the surviving entries l < len, then the new diagonal
-      double acc[3 * kMaxDepth + 2];
-#pragma unroll
-      for (int q = 0; q < 3 * kMaxDepth + 2; ++q) acc[q] = 0.0;
-      // Every product pairs two symmetric (F, D) or two antisymmetric (E) matrices, so the sum
-      // over all n^2 elements is the diagonal plus twice the strict lower triangle: half the
-      // history reads. Rows go to warps, columns to lanes (coalesced).
-      for (int r = tid >> 5; r < n; r += kWarps)
-        for (int col = tid & 31; col <= r; col += 32) {
-          const size_t k = (size_t)r * n + col;
-          const double wgt = col == r ? 1.0 : 2.0;
-          const double ea = Ea[k], fa = Fa[k];
-          const double eb = uhf ? Eb[k] : 0.0;
-          const double dn = keep ? Dh[k] : 0.0;
-          double ee = ea * ea;
-          if (uhf) ee = fma(eb, eb, ee);
-          acc[3 * kMaxDepth] = fma(wgt, ee, acc[3 * kMaxDepth]);
-          if (keep) acc[3 * kMaxDepth + 1] = fma(wgt, dn * fa, acc[3 * kMaxDepth + 1]);
-#pragma unroll
-          for (int l = 0; l < kMaxDepth; ++l) {
-            if (l < len) {
-              const double* bl = c.hist + (size_t)((head + l) % depth) * slot_mats * nn;
-              double v = bl[nn + k] * ea;
-              if (uhf) v = fma(bl[3 * nn + k], eb, v);
-              acc[l] = fma(wgt, v, acc[l]);
-              if (keep) {
-                acc[kMaxDepth + l] = fma(wgt, dn * bl[k], acc[kMaxDepth + l]);             // <D_new, F_l>
-                acc[2 * kMaxDepth + l] = fma(wgt, bl[2 * nn + k] * fa, acc[2 * kMaxDepth + l]);  // <D_l, F_new>
-              }
-            }
-          }
-        }
-      block_sums<3 * kMaxDepth + 2>(acc, c.red, c.misc);
-      if (tid == 0) {
-        for (int l = 0; l < len; ++l) {
-          c.bg[l * kMaxDepth + len] = c.misc[l];
-          c.bg[len * kMaxDepth + l] = c.misc[l];
-          c.mg[len * kMaxDepth + l] = c.misc[kMaxDepth + l];
-          c.mg[l * kMaxDepth + len] = c.misc[2 * kMaxDepth + l];
-        }
-        c.bg[len * kMaxDepth + len] = c.misc[3 * kMaxDepth];
-        c.mg[len * kMaxDepth + len] = c.misc[3 * kMaxDepth + 1];
-        const int m = len + 1;
-        const double err = sqrt(c.misc[3 * kMaxDepth]);
-        bool ok;
-        int mode = 0;
-        if (!uhf && J.accel == 2 && err > J.adiis_switch) {
-          ok = keep && m >= 2;
-          mode = ok ? 1 : 0;  // A-DIIS weights: solved by warp 0 below
-        } else {
-          ok = cdiis_coeffs(m, c.bg, c.coef);
-        }
-        c.iv[0] = ok ? 1 : 0;
-        c.iv[1] = mode;
-      }
+      use_hist = diis_step(c, J, uhf, keep, len, head, depth, slot_mats, Fa, Fb, Ea, Eb, Dh, Pc);
       ++len;
-      __syncthreads();
-      if (c.iv[1] == 1) {  // uniform across the CTA
-        if (tid < 32) adiis_coeffs_warp(len, c.mg, c.coef, c.red);
-        __syncthreads();
-      }
-      use_hist = c.iv[0] != 0;
       mark(c, kPhDiisSolve);
     }
 

@@ -204,7 +204,7 @@ struct PairKinds {
 
 // Doubles of the union that the phases of an n-function molecule use beside a pair table kept there.
 __host__ __device__ constexpr int union_keep(int n) {
-  const int a = 2 * 16 * 65, b = tri_scratch(n), c = back_scratch(n), d = 25 * n;
+  const int a = lower_scratch(n, true) > 2080 ? lower_scratch(n, true) : 2080, b = tri_scratch(n), c = back_scratch(n), d = 25 * n;
   const int m = a > b ? a : b, k = c > d ? c : d;
   return m > k ? m : k;
 }
@@ -585,27 +585,17 @@ __device__ __noinline__ double build_fock(Ctx& c, const double* Pt, const double
   return block_sum(en, c.red);  // its barriers also publish F
 }
 
-// E = F P - P F into E (scf.rs:1039-1054): one GEMM, then antisymmetrise in place.
-__device__ void commutator(Ctx& c, const double* Fm, const double* Pm, double* E) {
+// The lower triangle of E = F P - P F (scf.rs:1039-1054), which is antisymmetric: nothing reads the other half. The
+// transposed subtraction of a full product F P cost as much as the product (n = 148: 550k cycles before, 150k now).
+__device__ __noinline__ void commutator(Ctx& c, const double* Fm, const double* Pm, double* E) {
   const int n = c.n;
-  cta_gemm<false, false>(n, n, n, 1.0, Fm, n, Pm, n, c.tile, false,
-                         [&](int i, int j, double v) { E[(size_t)i * n + j] = v; });
-  for (int k = threadIdx.x; k < n * n; k += kThreads) {
-    const int i = k / n, j = k % n;
-    if (j < i) {
-      const double lo = E[(size_t)i * n + j], up = E[(size_t)j * n + i];
-      E[(size_t)i * n + j] = lo - up;
-      E[(size_t)j * n + i] = up - lo;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += kThreads) E[(size_t)i * n + i] = 0.0;
-  __syncthreads();
+  lower_product<true>(n, n, Fm, Pm, in_shared(c.tile),
+                      [&](int i, int j, double v) { E[(size_t)i * n + j] = i == j ? 0.0 : v; });
 }
 
-// ------------------------------------------------------------ small dense solves (thread 0)
-// Pulay coefficients from the Gram matrix (scf.rs:1544-1630); false = singular / unusable.
-__host__ __device__ bool cdiis_coeffs(int m, const double* gram, double* x) {
+// ------------------------------------------------------------ small dense solves
+// Pulay coefficients from the Gram matrix (scf.rs:1544-1630), on the host; false = singular / unusable.
+inline bool cdiis_coeffs(int m, const double* gram, double* x) {
   if (m < 2) return false;
   double scale = 0.0;
   for (int i = 0; i < m * m; ++i) scale = fmax(scale, fabs(gram[(i / m) * kMaxDepth + i % m]));
@@ -656,87 +646,130 @@ __host__ __device__ bool cdiis_coeffs(int m, const double* gram, double* x) {
   return true;
 }
 
-// A-DIIS weights on the simplex by projected gradient (scf.rs:1152-1172, 1637-1693), one warp:
-// lane k owns weight c_k and its gradient component; the Euclidean projection onto the simplex
-// sorts the trial point (descending, ties by index, as a stable insertion sort does) and every
-// lane runs the reference's serial cumulative-sum scan over the sorted values, so the weights are
-// the ones the serial loop produces. `sm` is shared scratch of kMaxDepth * (2 kMaxDepth + 1) doubles.
-__device__ void adiis_coeffs_warp(int m, const double* mg, double* out, double* sm) {
-  constexpr int K = kMaxDepth;
-  const int k = threadIdx.x & 31;
-  const int last = m - 1;
-  const double mnn = mg[last * K + last];
-  double* S = sm;           // [K][K]
-  double* T = sm + K * K;   // [K][K] S + S^T, the gradient's matrix (same sums as the reference's)
-  double* d = T + K * K;    // [K]
-  if (k < m) {
-    d[k] = mg[k * K + last] - mnn;
-    for (int j = 0; j < m; ++j) S[k * K + j] = mg[k * K + j] - mg[k * K + last] - mg[last * K + j] + mnn;
-  }
-  __syncwarp();
-  if (k < m)
-    for (int j = 0; j < m; ++j) T[k * K + j] = S[k * K + j] + S[j * K + k];
-  __syncwarp();
-  double L = 1.0e-12;
-  for (int i = 0; i < m; ++i) {
-    double row = 0.0;
-    for (int j = 0; j < m; ++j) row += fabs(T[i * K + j]);
-    L = fmax(L, row);
-  }
-  const double lr = 1.0 / L;
-  // Every lane runs the whole iteration on the full state in registers (the lanes agree), so the
-  // loop needs no shuffles: gradient, trial point, its stable descending order, the reference's
-  // cumulative-sum scan for the simplex projection, and the change.
-  double c[K];
+// The same on one warp: lane r holds row r of the scaled bordered matrix (and its right-hand side), the pivot rows
+// come round by shuffles. Coefficients to x; false = singular / unusable. `gram` and x in shared memory.
+__device__ __forceinline__ bool cdiis_coeffs_warp(int m, const double* gram, double* x) {
+  constexpr int D = kMaxDepth + 1;
+  constexpr unsigned full = 0xffffffffu;
+  if (m < 2) return false;
+  const int lane = threadIdx.x & 31, dim = m + 1;
+  double scale = 0.0;
+  for (int i = lane; i < m * m; i += 32) scale = fmax(scale, fabs(gram[(i / m) * kMaxDepth + i % m]));
+  scale = warp_max(scale);
+  if (!(scale > 0.0) || !isfinite(scale)) return false;
+  double B[D], rhs = lane == m ? -1.0 : 0.0;
 #pragma unroll
-  for (int j = 0; j < K; ++j) c[j] = j == last ? 1.0 : 0.0;
+  for (int j = 0; j < D; ++j) {
+    double v = 0.0;
+    if (lane < m && j < m) v = gram[lane * kMaxDepth + j] / scale;
+    else if ((lane < m && j == m) || (lane == m && j < m)) v = -1.0;
+    B[j] = v;
+  }
+  bool done = lane >= dim;  // rows that have been pivots (or are not there)
+  int mine = -1;            // the column this row was the pivot of
+#pragma unroll
+  for (int col = 0; col < D; ++col) {
+    if (col >= dim) break;
+    // largest element of the column among the rows left
+    double best = done ? -1.0 : fabs(B[col]);
+    int piv = lane;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(full, best, o);
+      const int op = __shfl_xor_sync(full, piv, o);
+      if (ob > best || (ob == best && op < piv)) {
+        best = ob;
+        piv = op;
+      }
+    }
+    best = __shfl_sync(full, best, 0);  // the first 16 lanes hold all rows
+    piv = __shfl_sync(full, piv, 0);
+    if (best < 1.0e-12) return false;
+    const double pv = __shfl_sync(full, B[col], piv);
+    const double f = done || lane == piv ? 0.0 : B[col] / pv;
+    if (lane == piv) {
+      done = true;
+      mine = col;
+    }
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+      if (j >= col) B[j] -= f * __shfl_sync(full, B[j], piv);
+    rhs -= f * __shfl_sync(full, rhs, piv);
+  }
+#pragma unroll
+  for (int col = D - 1; col >= 0; --col) {
+    if (col >= dim) continue;
+    const int src = __ffs(__ballot_sync(full, mine == col)) - 1;
+    const double xc = __shfl_sync(full, rhs / B[col], src);
+    if (lane == 0) x[col] = xc;
+    rhs -= B[col] * xc;
+  }
+  __syncwarp();
+  return true;
+}
+
+// A-DIIS weights on the simplex by projected gradient (scf.rs:1152-1172, 1637-1693), one warp:
+// lane k owns row k of the gradient's matrix; all lanes hold the whole trial point and weights. The Euclidean projection onto
+// the simplex subtracts the theta for which the positive parts sum to 1; the set of positive entries rarely
+// changes between steps, so theta is first formed from the previous set and accepted when the set reproduces itself
+// (which makes it the projection), else the set is rebuilt from all entries, dropping those below theta until none
+// is. A step is one chain of about 300 cycles, up to 400 steps (1300 when every lane sorted the trial point and
+// scanned it as the reference does).
+__device__ __forceinline__ void adiis_coeffs_warp(int m, const double* mg, double* out) {
+  constexpr int K = kMaxDepth;
+  constexpr unsigned full = 0xffffffffu;
+  const int k = threadIdx.x & 31, last = m - 1, row = k < m ? k : 0;
+  const double mnn = mg[last * K + last];
+  // S = mg - (last row and column), T = S + S^T: the gradient is 2 d + T c
+  auto S = [&](int i, int j) { return mg[i * K + j] - mg[i * K + last] - mg[last * K + j] + mnn; };
+  const double d2 = 2.0 * (mg[row * K + last] - mnn);
+  double T[K], c[K], own = row == last && k < m ? 1.0 : 0.0, rs = 0.0;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    T[j] = j < m ? S(row, j) + S(j, row) : 0.0;
+    rs += fabs(T[j]);
+    c[j] = j == last ? 1.0 : 0.0;
+  }
+  const double lr = 1.0 / fmax(1.0e-12, warp_max(rs));
+  unsigned set = (1u << m) - 1u;
   for (int it = 0; it < 400; ++it) {
+    const double g = d2 + (((T[0] * c[0] + T[1] * c[1]) + (T[2] * c[2] + T[3] * c[3])) +
+                           ((T[4] * c[4] + T[5] * c[5]) + (T[6] * c[6] + T[7] * c[7])));
+    const double mine = own - lr * g;
     double t[K];
 #pragma unroll
-    for (int q = 0; q < K; ++q) {
-      double g = 2.0 * d[q < m ? q : 0];
+    for (int j = 0; j < K; ++j) t[j] = __shfl_sync(full, mine, j);
+    double theta = 0.0;
+    unsigned cur = set;
+    for (int tries = 0; tries < 2 * K + 2; ++tries) {
+      double v[K];
 #pragma unroll
-      for (int j = 0; j < K; ++j)
-        if (j < m) g += T[q * K + j] * c[j];
-      t[q] = q < m ? c[q] - lr * g : 0.0;
+      for (int j = 0; j < K; ++j) v[j] = (cur >> j) & 1u ? t[j] : 0.0;
+      const double sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+      // 1 / count for 1 .. 8
+      const int q = __popc(cur);
+      const double inv = q <= 2 ? (q == 1 ? 1.0 : 0.5) : q <= 4 ? (q == 3 ? 1.0 / 3.0 : 0.25)
+                         : q <= 6 ? (q == 5 ? 0.2 : 1.0 / 6.0) : (q == 7 ? 1.0 / 7.0 : 0.125);
+      theta = (sum - 1.0) * inv;
+      unsigned nx = 0;
+#pragma unroll
+      for (int j = 0; j < K; ++j) nx |= j < m && t[j] > theta ? 1u << j : 0u;
+      if (nx == cur) break;
+      // first the whole set, then only shrinking ones
+      cur = tries == 0 ? (1u << m) - 1u : (cur & nx ? cur & nx : cur);
     }
-    // the trial point sorted descending by a 19-comparator network on a copy (unused entries
-    // -inf, so they sort last); ties give equal values in either order, so the cumulative sums,
-    // and with them the projection, are those of the reference's stable sort
-    double u[K];
+    set = cur;
+    double dl[K];
 #pragma unroll
-    for (int q = 0; q < K; ++q) u[q] = q < m ? t[q] : -INFINITY;
-    constexpr int kNet[19][2] = {{0, 2}, {1, 3}, {4, 6}, {5, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}, {0, 1}, {2, 3},
-                                 {4, 5}, {6, 7}, {2, 4}, {3, 5}, {1, 4}, {3, 6}, {1, 2}, {3, 4}, {5, 6}};
-#pragma unroll
-    for (int e = 0; e < 19; ++e) {
-      const double a = u[kNet[e][0]], b = u[kNet[e][1]];
-      u[kNet[e][0]] = fmax(a, b);
-      u[kNet[e][1]] = fmin(a, b);
+    for (int j = 0; j < K; ++j) {
+      const double pj = j < m ? fmax(t[j] - theta, 0.0) : 0.0;
+      dl[j] = fabs(pj - c[j]);
+      c[j] = pj;
     }
-    double css = 0.0, theta = 0.0;
-#pragma unroll
-    for (int p = 0; p < K; ++p) {
-      if (p >= m) break;
-      css += u[p];
-      const double tt = (css - 1.0) / (double)(p + 1);
-      if (u[p] - tt > 0.0) theta = tt;
-    }
-    double delta = 0.0;
-#pragma unroll
-    for (int q = 0; q < K; ++q) {
-      if (q >= m) break;
-      const double pq = fmax(t[q] - theta, 0.0);
-      delta += fabs(pq - c[q]);
-      c[q] = pq;
-    }
-    if (delta < 1.0e-12) break;
+    own = fmax(mine - theta, 0.0);
+    if (((dl[0] + dl[1]) + (dl[2] + dl[3])) + ((dl[4] + dl[5]) + (dl[6] + dl[7])) < 1.0e-12) break;
   }
-  if (k < m) {
-#pragma unroll
-    for (int q = 0; q < K; ++q)
-      if (q == k) out[k] = c[q];
-  }
+  if (k < m) out[k] = own;
   __syncwarp();
 }
 
@@ -781,7 +814,7 @@ __device__ void eigensolve(Ctx& c, const SymInput& in, int kval, int kvec, doubl
 // Pnew = w Y^T Y (first k rows of Y); returns sum (Pnew - Pold)^2 to all threads. With
 // damping lam > 0 the stored value is (1-lam) Pnew + lam Pold (scf.rs:1440-1448); the RMS
 // uses the undamped Pnew, as the reference does.
-__device__ double density(Ctx& c, const double* Y, int k, double w, const double* Pold, double* Pnew, double damp) {
+__device__ __noinline__ double density(Ctx& c, const double* Y, int k, double w, const double* Pold, double* Pnew, double damp) {
   const int n = c.n;
   double sq = 0.0;
   if (k == 0) {
@@ -793,8 +826,8 @@ __device__ double density(Ctx& c, const double* Y, int k, double w, const double
     __syncthreads();
     return block_sum(sq, c.red);
   }
-  cta_gemm<true, false>(n, n, k, w, Y, n, Y, n, c.tile, true, [&](int i, int j, double v) {
-    if (i < j) return;
+  lower_product<false>(n, k, Y, nullptr, in_shared(c.tile), [&](int i, int j, double y) {
+    const double v = w * y;
     const size_t ij = (size_t)i * n + j, ji = (size_t)j * n + i;
     const double o = Pold[ij];
     const double dlt = v - o;
