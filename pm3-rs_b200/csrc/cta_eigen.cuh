@@ -579,20 +579,31 @@ __device__ __forceinline__ int sturm(const double* d, const double* e2, int lo, 
   return cnt;
 }
 
+// Power of two that brings the larger of two magnitudes into [1, 2), as its exponent (0 for zeros).
+__device__ __forceinline__ int pair_exponent(double a, double b) {
+  const double m = fmax(fabs(a), fabs(b));
+  const int ex = (__double2hiint(m) >> 20) & 0x7ff;
+  return ex == 0 ? 0 : ex - 1023;
+}
+__device__ __forceinline__ double pow2(int ex) {  // 2^ex for normal results, 0 below, the largest power above
+  return ex < -1022 ? 0.0 : __hiloint2double((min(ex, 1023) + 1023) << 20, 0);
+}
+
 // Sturm counts at M shifts at once, without divisions (see the ratio form above for the
 // reference recurrence): p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}; sign changes between
 // consecutive values count the eigenvalues below x. Pairs are rescaled by powers of two every
 // 8 steps (each step grows |p| by far less than 2^32 for the matrices here), exact for ratios.
+// val[t] 2^(256 ex[t]) is the characteristic polynomial at x[t].
 template <int M>
 __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const double* __restrict__ e2, int n,
-                                            const double (&x)[M], double pivmin, int (&cnt)[M]) {
-  (void)pivmin;
+                                            const double (&x)[M], int (&cnt)[M], double (&val)[M], int (&ex)[M]) {
   constexpr double kBig = 0x1p256, kSmall = 0x1p-256;
   double p[M], pm[M];
   unsigned sg[M];
 #pragma unroll
   for (int t = 0; t < M; ++t) {
     pm[t] = 1.0;
+    ex[t] = 0;
     p[t] = d[0] - x[t];
     sg[t] = __double_as_longlong(p[t]) < 0 ? 1u : 0u;
     cnt[t] = (int)sg[t];
@@ -616,6 +627,7 @@ __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const 
     for (int t = 0; t < M; ++t) {
       const double m = fmax(fabs(p[t]), fabs(pm[t]));
       const double sc = m > kBig ? kSmall : (m < kSmall ? kBig : 1.0);
+      ex[t] += m > kBig ? 1 : (m < kSmall ? -1 : 0);
       p[t] *= sc;
       pm[t] *= sc;
     }
@@ -632,6 +644,135 @@ __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const 
       p[t] = pn;
     }
   }
+#pragma unroll
+  for (int t = 0; t < M; ++t) val[t] = p[t];
+}
+
+// Eigenvalue j of T by multisection: a group of g lanes (a power of two, at most 32) brackets it; each step the group takes Sturm counts at P = g * kPts points (kPts
+// per lane, evaluated together) and keeps the interval between the neighbouring two that holds it.
+// Invariant: count(lo) <= j < count(hi). The points are evenly spaced (the bracket shrinks by P + 1) until
+// the interval holds this eigenvalue alone. From then on they close in geometrically on the
+// secant estimate of the characteristic polynomial's root, whose values the counts yield on the way; the counts
+// still decide, and a step that gained less than a factor of 4 is followed by an even one.
+// What bounds it: the recurrence, about 40 cycles a row and step; steps from a cold start at n = 64, k = 33:
+// 17 when all were even.
+// With `prev` (eigenvalue j of the previous SCF iteration) and `dprev` (its last change) the search starts from a
+// bracket around prev[j] once two counts confirm it. Whole warps call; lanes without an eigenvalue pass
+// active = false.
+__device__ __forceinline__ double multisect(const double* __restrict__ d, const double* __restrict__ e2, int n, int j,
+                                            bool active, int g, double glo, double ghi, double pivmin, double tnorm,
+                                            const double* prev, const double* dprev) {
+  constexpr double eps = 2.220446049250313e-16;
+  constexpr int kPts = 2;
+  const int P = g * kPts;
+  const int lane = threadIdx.x & 31;
+  const int gbase = lane & ~(g - 1), gl = lane & (g - 1);
+  const unsigned gbits = g == 32 ? 0xffffffffu : ((1u << g) - 1u);
+  double lo = glo, hi = ghi;
+  double flo = 0.0, fhi = 0.0;  // polynomial at lo and hi, 0 while unknown
+  int elo = 0, ehi = 0, clo = 0, chi = n;
+  if (prev) {
+    // warm bracket around the previous SCF iteration's value, widened until two Sturm
+    // counts confirm that it holds eigenvalue j (else the Gershgorin interval stays)
+    const double c0 = active ? prev[j] : 0.0;
+    const double w0 = active ? fmax(4.0 * fabs(dprev[j]), 1.0e-9 * fmax(tnorm, 1.0)) : 0.0;
+    double x[4], fv[4];
+    int cn[4], fe[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {  // brackets w0 and 64 w0: lower ends on even t, upper on odd
+      const double w = w0 * (t >= 2 ? 64.0 : 1.0);
+      x[t] = (t & 1) ? fmin(c0 + w, ghi) : fmax(c0 - w, glo);
+    }
+    if (active) sturm_multi<4>(d, e2, n, x, cn, fv, fe);
+    if (active) {
+#pragma unroll
+      for (int t = 2; t >= 0; t -= 2)  // the narrow one last
+        if (x[t] < x[t + 1] && cn[t] <= j && cn[t + 1] >= j + 1) {
+          lo = x[t];
+          hi = x[t + 1];
+          flo = fv[t];
+          fhi = fv[t + 1];
+          elo = fe[t];
+          ehi = fe[t + 1];
+          clo = cn[t];
+          chi = cn[t + 1];
+        }
+    }
+  }
+  bool act = active, even = false;
+  for (int it = 0; it < 160; ++it) {
+    if (act) {
+      const double mid = 0.5 * (lo + hi);
+      if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
+    }
+    if (!__any_sync(0xffffffffu, act)) break;
+    const double w = hi - lo;
+    const bool close = !even && clo == j && chi == j + 1 && flo != 0.0 && fhi != 0.0;
+    double x[kPts], fv[kPts];
+    int cn[kPts], fe[kPts];
+    if (close) {
+      const double a = fabs(flo), b = fabs(fhi);  // the one of the smaller scale counts as 0
+      const double r = elo == ehi ? a / (a + b) : (elo > ehi ? 1.0 : 0.0);
+      const double xs = lo + w * r, tiny = eps * fmax(fabs(lo), fabs(hi));
+#pragma unroll
+      for (int t = 0; t < kPts; ++t) {  // distances w/4 .. w/2^26 (w/16 for P = 2), below and above
+        const int q = gl * kPts + t, k = q < g ? q : P - 1 - q;
+        const int ex = g == 1 ? 4 : 2 + 24 * k / (g - 1);
+        const double dl = fmax(w * pow2(-ex), tiny);
+        x[t] = fmin(fmax(q < g ? xs - dl : xs + dl, lo), hi);
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < kPts; ++t) x[t] = lo + w * (double)(gl * kPts + t + 1) / (double)(P + 1);
+    }
+    if (act) sturm_multi<kPts>(d, e2, n, x, cn, fv, fe);
+    int tf = kPts;  // this lane's first point above eigenvalue j
+#pragma unroll
+    for (int t = kPts - 1; t >= 0; --t)
+      if (act && cn[t] > j) tf = t;
+    const unsigned bal = __ballot_sync(0xffffffffu, act && tf < kPts);
+    const unsigned mine = (bal >> gbase) & gbits;
+    // upper end: point f (the first above), lower end: point f - 1; either may be the bracket's own end
+    const int hl = mine ? gbase + __ffs(mine) - 1 : gbase + g - 1;
+    const int th = __shfl_sync(0xffffffffu, tf, hl);
+    const int f = mine ? (hl - gbase) * kPts + th : P;
+    auto take = [&](int q, double& px, double& pf, int& pe, int& pc) {  // point q of the group (any lane asks)
+      const int src = gbase + min(max(q, 0), P - 1) / kPts, tt = min(max(q, 0), P - 1) % kPts;
+      double vx = 0.0, vf = 0.0;
+      int ve = 0, vc = 0;
+#pragma unroll
+      for (int t = 0; t < kPts; ++t) {
+        const double sx = __shfl_sync(0xffffffffu, x[t], src), sf = __shfl_sync(0xffffffffu, fv[t], src);
+        const int se = __shfl_sync(0xffffffffu, fe[t], src), sc = __shfl_sync(0xffffffffu, cn[t], src);
+        if (t == tt) {
+          vx = sx;
+          vf = sf;
+          ve = se;
+          vc = sc;
+        }
+      }
+      if (q >= 0 && q < P && act) {
+        px = vx;
+        pf = vf;
+        pe = ve;
+        pc = vc;
+      }
+    };
+    double nlo = lo, nhi = hi;
+    take(f - 1, nlo, flo, elo, clo);
+    take(f, nhi, fhi, ehi, chi);
+    if (act) {
+      if (!(nhi - nlo < w)) {
+        if (close) even = true;  // no gain around the estimate: split evenly
+        else act = false;
+      } else {
+        even = close && (nhi - nlo) * 4.0 > w;
+        lo = nlo;
+        hi = nhi;
+      }
+    }
+  }
+  return 0.5 * (lo + hi);
 }
 
 // Splits T where the coupling is negligible and computes the lowest `kval` eigenvalues.
@@ -684,97 +825,18 @@ __device__ void tridiag_eigenvalues(int n, int kval, const EigenScratch& s_, con
   }
   __syncthreads();
   const double pivmin = s.misc[0], tnorm = s.misc[1], glo = s.misc[2], ghi = s.misc[3];
-  // Multisection: a group of g lanes (a power of two, g <= 32, kval * g <= kThreads) brackets
-  // one eigenvalue; each step the group takes Sturm counts at P = g * kPts interior points (kPts
-  // per lane, evaluated together), which cuts the bracket by P + 1 instead of 2.
-  // Invariant: count(lo) <= j < count(hi).
-  constexpr int kPts = 2;
+  // a group of g lanes per eigenvalue (a power of two, g <= 32, kval * g <= kThreads)
   int g = 1;
   while (g < 32 && kval * (2 * g) <= kThreads) g *= 2;
-  const int P = g * kPts;
-  const int lane = tid & 31;
-  const int gbase = lane & ~(g - 1), gl = lane & (g - 1);
-  const unsigned gbits = g == 32 ? 0xffffffffu : ((1u << g) - 1u);
   for (int j0 = 0; j0 < kval; j0 += kThreads / g) {
     const int j = j0 + tid / g;
-    const bool active = j < kval;
-    double lo = glo, hi = ghi;
-    if (prev) {
-      // warm bracket around the previous SCF iteration's value, widened until two Sturm
-      // counts confirm that it holds eigenvalue j (else the Gershgorin interval stays)
-      const double c0 = active ? prev[j] : 0.0;
-      const double w0 = active ? fmax(4.0 * fabs(dprev[j]), 1.0e-9 * fmax(tnorm, 1.0)) : 0.0;
-      double x[4];
-      int cn[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {  // brackets w0 and 64 w0: lower ends on even t, upper on odd
-        const double w = w0 * (t >= 2 ? 64.0 : 1.0);
-        x[t] = (t & 1) ? fmin(c0 + w, ghi) : fmax(c0 - w, glo);
-      }
-      if (active) sturm_multi<4>(s.d, s.e2, n, x, pivmin, cn);
-      if (active) {
-        if (x[0] < x[1] && cn[0] <= j && cn[1] >= j + 1) {
-          lo = x[0];
-          hi = x[1];
-        } else if (x[2] < x[3] && cn[2] <= j && cn[3] >= j + 1) {
-          lo = x[2];
-          hi = x[3];
-        }
-      }
-    }
-    bool act = active;
-    for (int it = 0; it < 128; ++it) {
-      if (act) {
-        const double mid = 0.5 * (lo + hi);
-        if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
-      }
-      if (!__any_sync(0xffffffffu, act)) break;
-      double x[kPts];
-      int cn[kPts];
-#pragma unroll
-      for (int t = 0; t < kPts; ++t) x[t] = lo + (hi - lo) * (double)(gl * kPts + t + 1) / (double)(P + 1);
-      if (act) sturm_multi<kPts>(s.d, s.e2, n, x, pivmin, cn);
-      int tf = kPts;  // this lane's first point above eigenvalue j
-#pragma unroll
-      for (int t = kPts - 1; t >= 0; --t)
-        if (act && cn[t] > j) tf = t;
-      const unsigned bal = __ballot_sync(0xffffffffu, act && tf < kPts);
-      const unsigned mine = (bal >> gbase) & gbits;
-      const int src = mine ? gbase + __ffs(mine) - 1 : gbase;
-      const int tsrc = __shfl_sync(0xffffffffu, tf, src);
-      if (act) {
-        double nlo, nhi;
-        if (mine == 0u) {  // every point is at or below eigenvalue j
-          nlo = lo + (hi - lo) * (double)P / (double)(P + 1);
-          nhi = hi;
-        } else {
-          const int f = (src - gbase) * kPts + tsrc;  // first point above it
-          nlo = f > 0 ? lo + (hi - lo) * (double)f / (double)(P + 1) : lo;
-          nhi = lo + (hi - lo) * (double)(f + 1) / (double)(P + 1);
-        }
-        if (!(nhi - nlo < hi - lo)) act = false;
-        else {
-          lo = nlo;
-          hi = nhi;
-        }
-      }
-    }
-    if (active && gl == 0) s.lam[j] = 0.5 * (lo + hi);
+    const double v = multisect(s.d, s.e2, n, j, j < kval, g, glo, ghi, pivmin, tnorm, prev, dprev);
+    if (j < kval && (tid & (g - 1)) == 0) s.lam[j] = v;
   }
   __syncthreads();
 }
 
 // ------------------------------------------------------------- 3. tridiagonal eigenvectors
-// Power of two that brings the larger of two magnitudes into [1, 2), as its exponent (0 for zeros).
-__device__ __forceinline__ int pair_exponent(double a, double b) {
-  const double m = fmax(fabs(a), fabs(b));
-  const int ex = (__double2hiint(m) >> 20) & 0x7ff;
-  return ex == 0 ? 0 : ex - 1023;
-}
-__device__ __forceinline__ double pow2(int ex) {  // 2^ex for normal results, 0 below, the largest power above
-  return ex < -1022 ? 0.0 : __hiloint2double((min(ex, 1023) + 1023) << 20, 0);
-}
-
 // Eigenvectors j < kvec of T, unnormalised, into Yt[i kvec + j] (zero outside the block of each). `tf` is
 // per-CTA global scratch of 6 n^2 doubles. Every array has the vector index fastest, so that the
 // threads of a warp (one vector each) touch consecutive addresses.

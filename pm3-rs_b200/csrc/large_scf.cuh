@@ -713,75 +713,9 @@ __global__ void __launch_bounds__(kWy) wy_t_block_kernel(const double* __restric
 __global__ void __launch_bounds__(kBlock) multisect_kernel(const double* d, const double* e2, int n, int kval,
                                                            int g, double glo, double ghi, double pivmin, double tnorm,
                                                            const double* prev, const double* dprev, double* lam) {
-  constexpr double eps = 2.220446049250313e-16;
-  constexpr int kPts = 2;
-  const int gt = blockIdx.x * kBlock + threadIdx.x;
-  const int j = gt / g, gl = gt % g;
-  const int lane = threadIdx.x & 31;
-  const int gbase = lane & ~(g - 1);
-  const unsigned gbits = g == 32 ? 0xffffffffu : ((1u << g) - 1u);
-  const int P = g * kPts;
-  const bool active = j < kval;
-  double lo = glo, hi = ghi;
-  if (prev) {
-    const double c0 = active ? prev[j] : 0.0;
-    const double w0 = active ? fmax(4.0 * fabs(dprev[j]), 1.0e-9 * fmax(tnorm, 1.0)) : 0.0;
-    double x[4];
-    int cn[4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const double w = w0 * (t >= 2 ? 64.0 : 1.0);
-      x[t] = (t & 1) ? fmin(c0 + w, ghi) : fmax(c0 - w, glo);
-    }
-    if (active) {
-      sturm_multi<4>(d, e2, n, x, pivmin, cn);
-      if (x[0] < x[1] && cn[0] <= j && cn[1] >= j + 1) {
-        lo = x[0];
-        hi = x[1];
-      } else if (x[2] < x[3] && cn[2] <= j && cn[3] >= j + 1) {
-        lo = x[2];
-        hi = x[3];
-      }
-    }
-  }
-  bool act = active;
-  for (int it = 0; it < 160; ++it) {
-    if (act) {
-      const double mid = 0.5 * (lo + hi);
-      if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
-    }
-    if (!__any_sync(0xffffffffu, act)) break;
-    double x[kPts];
-    int cn[kPts];
-#pragma unroll
-    for (int t = 0; t < kPts; ++t) x[t] = lo + (hi - lo) * (double)(gl * kPts + t + 1) / (double)(P + 1);
-    if (act) sturm_multi<kPts>(d, e2, n, x, pivmin, cn);
-    int tf = kPts;
-#pragma unroll
-    for (int t = kPts - 1; t >= 0; --t)
-      if (act && cn[t] > j) tf = t;
-    const unsigned bal = __ballot_sync(0xffffffffu, act && tf < kPts);
-    const unsigned mine = (bal >> gbase) & gbits;
-    const int src = mine ? gbase + __ffs(mine) - 1 : gbase;
-    const int tsrc = __shfl_sync(0xffffffffu, tf, src);
-    if (act) {
-      double nlo, nhi;
-      if (mine == 0u) {
-        nlo = lo + (hi - lo) * (double)P / (double)(P + 1);
-        nhi = hi;
-      } else {
-        const int f = (src - gbase) * kPts + tsrc;
-        nlo = f > 0 ? lo + (hi - lo) * (double)f / (double)(P + 1) : lo;
-        nhi = lo + (hi - lo) * (double)(f + 1) / (double)(P + 1);
-      }
-      if (!(nhi - nlo < hi - lo)) act = false;
-      else {
-        lo = nlo;
-        hi = nhi;
-      }
-    }
-  }
-  if (active && gl == 0) lam[j] = 0.5 * (lo + hi);
+  const int gt = blockIdx.x * kBlock + threadIdx.x, j = gt / g;
+  const double v = multisect(d, e2, n, j, j < kval, g, glo, ghi, pivmin, tnorm, prev, dprev);
+  if (j < kval && gt % g == 0) lam[j] = v;
 }
 // Eigenvector j < kvec of T by twisted factorisation (thread per vector), written as column j of
 // Y (n x kvec, row-major); zero outside the unreduced block that holds eigenvalue j. Scratch
