@@ -195,10 +195,9 @@ int pm3gpu_single_point(pm3gpu_ctx* ctx, int n_atoms, const int32_t* z, const do
  * code), so make it before any stream capture begins. A device reset invalidates that address
  * with everything else on the device: create a new context after a reset (creating a context
  * makes the next call look the address up again).
- * The call always runs the one-CTA-per-molecule kernel: a molecule that pm3gpu_single_point sends
- * to the whole-GPU path (pm3gpu_set_large_threshold, or 192+ basis functions when no threshold is
- * set) returns PM3GPU_RESOURCE_LIMIT here, so
- * that the two entry points never run different algorithms on the same input. The caller clears nothing: each call resets
+ * The call always runs the one-CTA-per-molecule kernel: a molecule at or above the whole-GPU
+ * threshold (pm3gpu_set_large_threshold, or 192 basis functions when no threshold is
+ * set) returns PM3GPU_RESOURCE_LIMIT here. The caller clears nothing: each call resets
  * the queue counters and flags it needs at zero itself. All contexts of a process on one device
  * share the one array, so calls that overlap in time on that device (two contexts, or two
  * threads on different contexts) race and give wrong results; calls through one context are
@@ -329,7 +328,7 @@ int pm3gpu_last_launch_layout(pm3gpu_ctx* ctx, int* ctas_per_sm, int* smem_matri
  * (grid-wide integral and Fock kernels, blocked eigensolver, the library's FP64 tensor-core GEMM for
  * the dense products) instead of one CTA each. Default and maximum 257: every molecule beyond one CTA's
  * 256 basis functions; by default a call with a single molecule also sends it there from 192 basis
- * functions, where all SMs beat one CTA (setting a threshold replaces that rule). Lower values send
+ * functions when mixed precision or the eigensolver checks are on (setting a threshold replaces that rule). Lower values send
  * smaller molecules to that path too (one molecule at a time, all SMs on it). Same run_pm3
  * semantics either way (no reference counterpart: the reference has one CPU path). */
 int pm3gpu_set_large_threshold(pm3gpu_ctx* ctx, int nao);

@@ -48,7 +48,8 @@ struct DevBuf {
 };
 
 constexpr int kMaxDiisDepthHost = 8;
-// Basis size from which a call's only molecule goes to the whole-GPU path by default.
+// Basis size from which a call's only molecule goes to the whole-GPU path by default when its modes or records are asked for
+// (mixed precision, eigensolver checks), and from which the allocation-free entry refuses a molecule.
 constexpr int kSingleWholeNao = 192;
 constexpr int kMaxLargeAtoms = 30000;  // pair indices of the whole-GPU kernels stay in 32 bits
 // scf.rs:309-331
@@ -1154,10 +1155,11 @@ int run_batch(pm3gpu_ctx* c, int n_mol, const int32_t* h_offs, const int32_t* h_
     if (na < 0) return fail(c, PM3GPU_INVALID_INPUT, "atom_offsets must be non-decreasing");
     const pm3gpu_options* o = per_mol ? opts + m : opts;
     plan_molecule(c, h_z + p.atom0, h_xyz ? h_xyz + 3 * (size_t)p.atom0 : nullptr, na, o, p);
-    // A lone molecule of kSingleWholeNao basis functions or more finishes sooner on all SMs than on
-    // the one CTA the batched kernel gives it (n = 204: 47 against 54 ms; n = 252: 62 against 183).
+    // A lone molecule finishes sooner on the one CTA the batched kernel gives it than on all SMs, whose grid barriers cost more than
+    // they spread, over that kernel's whole range (n = 204: 23 against 45 ms; n = 252: 44 against 60). The whole-GPU
+    // path still takes it where only that path has what was asked for.
     if (n_mol == 1 && !c->large_set && p.status == PM3GPU_OK && !p.large && p.nao >= kSingleWholeNao &&
-        o->guess != PM3GPU_GUESS_LEARNED)
+        o->guess != PM3GPU_GUESS_LEARNED && (c->precision == PM3GPU_PRECISION_MIXED || c->large_checks))
       p.large = true;
     if (p.status != PM3GPU_OK || p.large) continue;  // large molecules: whole-GPU path below
     JobDesc j = p.steered ? make_job(p, o->guess, o->accelerator, o->level_shift_ev, o->damping, false, 0)
@@ -2332,8 +2334,8 @@ int noalloc_run(pm3gpu_ctx* c, int n_atoms, const int32_t* z, const double* xyz,
     c->err = p.msg;
     return p.status;
   }
-  // pm3gpu_single_point would run the whole-GPU algorithm, which needs allocations: by the context's
-  // threshold, or (none set) by the lone-molecule rule of run_batch
+  // the whole-GPU algorithm needs allocations: by the context's threshold, or (none set) the size from which
+  // this entry has always left molecules to it
   const bool lone_whole = !c->large_set && p.nao >= kSingleWholeNao && o->guess != PM3GPU_GUESS_LEARNED;
   if (p.large || lone_whole) {
     char msg[220];
