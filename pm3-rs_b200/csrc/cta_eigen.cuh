@@ -585,6 +585,12 @@ __device__ __forceinline__ int pair_exponent(double a, double b) {
   const int ex = (__double2hiint(m) >> 20) & 0x7ff;
   return ex == 0 ? 0 : ex - 1023;
 }
+// A number that orders the magnitudes p 2^ex (p >= 0): exponent plus fraction, a piecewise linear log2.
+__device__ __forceinline__ double scaled_order(double p, int ex) {
+  const int hi = __double2hiint(p), e = hi >> 20;
+  if (e == 0) return -INFINITY;
+  return (double)(e + ex) + (__hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(p)) - 1.0);
+}
 __device__ __forceinline__ double pow2(int ex) {  // 2^ex for normal results, 0 below, the largest power above
   return ex < -1022 ? 0.0 : __hiloint2double((min(ex, 1023) + 1023) << 20, 0);
 }
@@ -933,13 +939,12 @@ __device__ double* tridiag_vectors(int n, int kvec, double* tf, const EigenScrat
   // Row lo + t of f is in group (t - 1) / 8 (row lo in group 0, whose exponent is 0), of g row hi - t.
   const int shares = min(kThreads / kvec, 16), share = tid / kvec, jv = tid - share * kvec;
   const bool in_share = share < shares;
-  // The row of the largest |f g|: as an integer, a double's bits plus its scale exponent order the scaled magnitudes.
-  long long* __restrict__ K = reinterpret_cast<long long*>(in_shared(s_.sh));      // [shares][kvec], at most kThreads
+  // The row of the largest |f g|.
+  double* __restrict__ K = in_shared(s_.sh);                                       // [shares][kvec], at most kThreads
   int* __restrict__ R = reinterpret_cast<int*>(in_shared(s_.sh) + kThreads);       // the same
-  constexpr long long kLow = -0x7fffffffffffffffLL;
   if (in_share) {
     const int j = jv, b = s.vinfo[j], lo = s.blk[b], hi = s.blk[b + 1] - 1;
-    long long best = kLow;
+    double best = -INFINITY;
     int br = hi;
     for (int g = share; lo + 8 * g <= hi; g += shares) {
       const int t0 = 8 * g + (g > 0 ? 1 : 0), t1 = min(8 * g + 8, hi - lo);  // rows t0 .. t1 of the block
@@ -956,9 +961,8 @@ __device__ double* tridiag_vectors(int n, int kvec, double* tf, const EigenScrat
 #pragma unroll
       for (int u = 0; u < 9; ++u) {
         const int t = t0 + u;
-        if (t <= t1 && p[u] > 0.0) {
-          const int q = ef + ((max(hi - lo - t - 1, 0) >> 3) == gb ? e0 : e1);
-          const long long key = __double_as_longlong(p[u]) + ((long long)q << 52);
+        if (t <= t1) {
+          const double key = scaled_order(p[u], ef + ((max(hi - lo - t - 1, 0) >> 3) == gb ? e0 : e1));
           if (key > best) {
             best = key;
             br = lo + t;
@@ -972,7 +976,7 @@ __device__ double* tridiag_vectors(int n, int kvec, double* tf, const EigenScrat
   __syncthreads();
   if (tid < kvec) {
     const int j = tid;
-    long long best = K[j];
+    double best = K[j];
     int r = R[j];
     for (int q = 1; q < shares; ++q)
       if (K[q * kvec + j] > best) {

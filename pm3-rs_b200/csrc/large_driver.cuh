@@ -44,9 +44,9 @@ struct LargeBufs {
   DevBuf ao, sprow, sroff;
   DevBuf H, W, hacc, dpk, jacc, part, part2, scal;
   DevBuf P[2], Q[2], Pt, F, G, hist, A;
-  DevBuf d, e, e2, tau, lam, dlam, blk;
+  DevBuf d, e, e2, inve, tau, lam, dlam, blk;
   DevBuf V, Wp, y, wtmp, ps, s64, vcol, tp, ctr, refl;
-  DevBuf X, Xt, Dp, Lp, Um;
+  DevBuf X, Xt, Tf, Tg, Te;  // eigenvectors; the twisted sweeps' values and exponents
   DevBuf Gm, Mm, Tm, Z1, Z2, blocks, Gk;
   DevBuf mh[2], ml[2], c32;  // mixed mode: BF16 hi / lo parts of two operands, FP32 product
   DevBuf gsync, vw, wv;      // cooperative panels: grid barrier, X = [V | W] and Y = [W | V]
@@ -55,8 +55,8 @@ struct LargeBufs {
   bool tcerr_zeroed = false;
   void release() {
     for (DevBuf* b : {&ao, &sprow, &sroff, &H, &W, &hacc, &dpk, &jacc, &part, &part2, &scal, &P[0], &P[1], &Q[0], &Q[1], &Pt,
-                      &F, &G, &hist, &A, &d, &e, &e2, &tau, &lam, &dlam, &blk, &V, &Wp, &y, &wtmp, &ps, &s64, &vcol, &tp, &ctr, &refl, &X, &Xt,
-                      &Dp, &Lp, &Um, &Gm, &Mm, &Tm, &Z1, &Z2, &blocks, &Gk, &mh[0], &mh[1], &ml[0], &ml[1], &c32, &gsync, &vw, &wv, &Fchk, &tcerr})
+                      &F, &G, &hist, &A, &d, &e, &e2, &inve, &tau, &lam, &dlam, &blk, &V, &Wp, &y, &wtmp, &ps, &s64, &vcol, &tp, &ctr, &refl, &X, &Xt,
+                      &Tf, &Tg, &Te, &Gm, &Mm, &Tm, &Z1, &Z2, &blocks, &Gk, &mh[0], &mh[1], &ml[0], &ml[1], &c32, &gsync, &vw, &wv, &Fchk, &tcerr})
       b->release();
     tcerr_zeroed = false;
     gwork.release();
@@ -187,7 +187,7 @@ class LargeSolver {
     CUDA_TRY(c_, B_.hacc.ensure(80 * (size_t)N_));
     CUDA_TRY(c_, B_.dpk.ensure(80 * (size_t)N_));
     CUDA_TRY(c_, B_.jacc.ensure(80 * (size_t)N_));
-    CUDA_TRY(c_, B_.part.ensure(8 * (size_t)large::kRedBlocks));
+    CUDA_TRY(c_, B_.part.ensure(8 * 32 * (size_t)large::kRedBlocks));
     CUDA_TRY(c_, B_.part2.ensure(8 * (size_t)large::kRedBlocks));
     CUDA_TRY(c_, B_.scal.ensure(8 * 128));
     const long long np = (long long)N_ * (N_ - 1) / 2;
@@ -331,10 +331,9 @@ class LargeSolver {
       if (!uhf) {
         int rc = fock(Pc, nullptr, nullptr, Fa, nullptr);
         if (rc) return rc;
-        double h1, h2;
-        if ((rc = dot(Pc, B_.H.as<double>(), nullptr, nullptr, &h1)) || (rc = dot(Pc, Fa, nullptr, nullptr, &h2)))
-          return rc;
-        e_elec = 0.5 * (h1 + h2);
+        double h;
+        if ((rc = dot(Pc, B_.H.as<double>(), Pc, Fa, &h))) return rc;
+        e_elec = 0.5 * h;
       } else {
         double* Pt = B_.Pt.as<double>();
         large::add_kernel<<<grid_for(nn_), large::kBlock, 0, c_->stream>>>(Pc, Qc, Pt, nn_);
@@ -353,22 +352,32 @@ class LargeSolver {
         if (rc) return rc;
         if (uhf && (rc = commutator(Fb, Qc, Eb, lowp_iter))) return rc;
         if (keep && (rc = copy(Pc, Dh))) return rc;
-        double ee;
-        if ((rc = dot(Ea, Ea, Eb, Eb, &ee))) return rc;
-        double dnf = 0.0;
-        if (keep && (rc = dot(Dh, Fa, nullptr, nullptr, &dnf))) return rc;
+        double gs[32];
+        {
+          large::GramIn in{};
+          in.len = len;
+          for (int l = 0; l < len; ++l) {
+            double* bl = slot(head, l, depth, slot_mats);
+            in.E[l] = bl + nn_;
+            in.E2[l] = uhf ? bl + 3 * nn_ : nullptr;
+            in.F[l] = bl;
+            in.D[l] = keep ? bl + 2 * nn_ : nullptr;
+          }
+          const int blocks = std::min(large::kRedBlocks, (n + large::kBlock / 32 - 1) / (large::kBlock / 32));
+          large::gram_kernel<<<blocks, large::kBlock, 0, c_->stream>>>(in, Ea, uhf ? Eb : nullptr, Fa, keep ? Dh : nullptr, n,
+                                                                       B_.part.as<double>());
+          large::gram_finish_kernel<<<1, large::kBlock, 0, c_->stream>>>(B_.part.as<double>(), blocks, B_.scal.as<double>());
+          c_->launches += 2;
+          CUDA_TRY(c_, cudaMemcpyAsync(gs, B_.scal.p, sizeof(gs), cudaMemcpyDeviceToHost, c_->stream));
+          CUDA_TRY(c_, cudaStreamSynchronize(c_->stream));
+        }
+        const double ee = gs[24], dnf = gs[25];
         for (int l = 0; l < len; ++l) {
-          double* bl = slot(head, l, depth, slot_mats);
-          double v;
-          if ((rc = dot(bl + nn_, Ea, uhf ? bl + 3 * nn_ : nullptr, Eb, &v))) return rc;
-          bg[l * kMaxDepth + len] = v;
-          bg[len * kMaxDepth + l] = v;
+          bg[l * kMaxDepth + len] = gs[l];
+          bg[len * kMaxDepth + l] = gs[l];
           if (keep) {
-            double a1, a2;
-            if ((rc = dot(Dh, bl, nullptr, nullptr, &a1)) || (rc = dot(bl + 2 * nn_, Fa, nullptr, nullptr, &a2)))
-              return rc;
-            mg[len * kMaxDepth + l] = a1;  // <D_new, F_l>
-            mg[l * kMaxDepth + len] = a2;  // <D_l, F_new>
+            mg[len * kMaxDepth + l] = gs[8 + l];   // <D_new, F_l>
+            mg[l * kMaxDepth + len] = gs[16 + l];  // <D_l, F_new>
           }
         }
         bg[len * kMaxDepth + len] = ee;
@@ -899,7 +908,7 @@ class LargeSolver {
     }
     const double tnorm = std::max(std::fabs(gl), std::fabs(gu));
     const double cut = 1000.0 * eps * tnorm;
-    std::vector<double> e2(n);
+    std::vector<double> e2(n), inve(n);
     hblk_.assign(1, 0);
     double emax = 0.0;
     for (int i = 0; i < n; ++i) {
@@ -910,6 +919,7 @@ class LargeSolver {
         hblk_.push_back(i + 1);
       }
       e2[i] = ei * ei;
+      inve[i] = ei != 0.0 ? 1.0 / ei : 0.0;
       emax = std::max(emax, ei * ei);
     }
     hblk_.push_back(n);
@@ -922,6 +932,8 @@ class LargeSolver {
     CUDA_TRY(c_, B_.dlam.ensure(16 * (size_t)n));
     CUDA_TRY(c_, cudaMemcpyAsync(B_.e.p, e.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, c_->stream));
     CUDA_TRY(c_, cudaMemcpyAsync(B_.e2.p, e2.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, c_->stream));
+    CUDA_TRY(c_, B_.inve.ensure(8 * (size_t)n));
+    CUDA_TRY(c_, cudaMemcpyAsync(B_.inve.p, inve.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, c_->stream));
     CUDA_TRY(c_, cudaMemcpyAsync(B_.blk.p, hblk_.data(), 4 * hblk_.size(), cudaMemcpyHostToDevice, c_->stream));
     const bool seeded = warm && (int)lam.size() == kval && (int)dl.size() == kval;
     double* prev = B_.dlam.as<double>();
@@ -993,12 +1005,22 @@ class LargeSolver {
     // ---- 3. eigenvectors of the tridiagonal
     CUDA_TRY(c_, B_.X.ensure(8 * (size_t)n * K));
     CUDA_TRY(c_, B_.Xt.ensure(8 * (size_t)n * K));
-    for (DevBuf* bf : {&B_.Dp, &B_.Lp, &B_.Um}) CUDA_TRY(c_, bf->ensure(8 * (size_t)n * K));
+    const size_t groups = ((size_t)n + 7) / 8;
+    for (DevBuf* bf : {&B_.Tf, &B_.Tg}) CUDA_TRY(c_, bf->ensure(8 * (size_t)n * K));
+    CUDA_TRY(c_, B_.Te.ensure(4 * (2 * groups + 1) * K));
     double* X = B_.X.as<double>();
-    large::twisted_kernel<<<(kvec + large::kBlock - 1) / large::kBlock, large::kBlock, 0, c_->stream>>>(
-        d, e, B_.e2.as<double>(), n, kvec, B_.lam.as<double>(), B_.blk.as<int>(), (int)hblk_.size() - 1, pivmin_, tnorm_,
-        X, B_.Dp.as<double>(), B_.Lp.as<double>(), B_.Um.as<double>());
-    ++c_->launches;
+    {
+      int* ef = B_.Te.as<int>();
+      int* eg = ef + groups * K;
+      int* vb = eg + groups * K;
+      const dim3 sweep((unsigned)((kvec + large::kTwist - 1) / large::kTwist), 2);
+      large::twist_sweep_kernel<<<sweep, large::kTwist, 0, c_->stream>>>(
+          d, e, B_.e2.as<double>(), B_.inve.as<double>(), n, kvec, B_.lam.as<double>(), B_.blk.as<int>(),
+          (int)hblk_.size() - 1, pivmin_, tnorm_, B_.Tf.as<double>(), B_.Tg.as<double>(), ef, eg, vb);
+      large::twist_vector_kernel<<<(kvec + 31) / 32, large::kBlock, 0, c_->stream>>>(
+          n, kvec, B_.blk.as<int>(), vb, B_.Tf.as<double>(), B_.Tg.as<double>(), ef, eg, X);
+      c_->launches += 2;
+    }
     CUDA_TRY(c_, cudaGetLastError());
     tick(kLgEigvec);
     // ---- 4. back-transformation X <- Q X, blocks of kWy reflectors from the last to the first
@@ -1018,7 +1040,7 @@ class LargeSolver {
       double* Xr = X + (size_t)r0 * K;
       // G = V^T V (b x b); column-major: Vc Vc^T
       GEMM_TRY(gemm(false, true, b, b, m, one, Vr, large::kWy, Vr, large::kWy, zero, B_.Gm.as<double>(), b));
-      large::wy_t_block_kernel<<<1, large::kWy, 0, c_->stream>>>(B_.Gm.as<double>(), tau, p, b, B_.Tm.as<double>());
+      large::wy_t_block_kernel<<<1, large::kBlock, large::kTSmem, c_->stream>>>(B_.Gm.as<double>(), tau, p, b, B_.Tm.as<double>());
       ++c_->launches;
       // Z = V^T X  -> column-major Zc = Xc Vc^T (K x b)
       GEMM_TRY(gemm(false, true, (int)K, b, m, one, Xr, (int)K, Vr, large::kWy, zero, B_.Z1.as<double>(), (int)K));

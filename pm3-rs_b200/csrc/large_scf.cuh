@@ -684,27 +684,82 @@ __global__ void __launch_bounds__(kBlock) block_v_kernel(const double* A, int n,
   }
 }
 // T (kWy x kWy, row-major, upper triangular) of H(p) ... H(p+b-1) = I - V T V^T from the Gram
-// G = V^T V (b x b) and tau: T[k][k] = tau_k, T[m][k] = -tau_k sum_{m <= l < k} T[m][l] G[l][k].
-// Row m depends only on its own earlier entries, so thread m forms row m alone (no barriers).
-__global__ void __launch_bounds__(kWy) wy_t_block_kernel(const double* __restrict__ G, const double* __restrict__ tau,
-                                                         int p, int b, double* __restrict__ T) {
-  const int m = threadIdx.x;
-  double* row = T + (size_t)m * kWy;
-  for (int k = 0; k < kWy; ++k) row[k] = 0.0;
-  if (m >= b) return;
-  row[m] = tau[p + m];
-  for (int k = m + 1; k < b; ++k) {
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int l = m;
-    for (; l + 3 < k; l += 4) {
-      a0 = fma(row[l], G[(size_t)l * b + k], a0);
-      a1 = fma(row[l + 1], G[(size_t)(l + 1) * b + k], a1);
-      a2 = fma(row[l + 2], G[(size_t)(l + 2) * b + k], a2);
-      a3 = fma(row[l + 3], G[(size_t)(l + 3) * b + k], a3);
-    }
-    for (; l < k; ++l) a0 = fma(row[l], G[(size_t)l * b + k], a0);
-    row[k] = -tau[p + k] * ((a0 + a1) + (a2 + a3));
+// G = V^T V (b x b) and tau: T[k][k] = tau_k, T[m][k] = -tau_k sum_{m <= l < k} T[m][l] G[l][k]. The 16 x 16 diagonal
+// blocks are formed row by row (a row depends only on its own earlier entries), then neighbours are
+// joined three times, [T1, -T1 G12 T2; 0, T2], by products in shared memory. One CTA; forming whole rows of 128 one
+// thread each took most of the back-transformation (3.6 of 3.7 ms at n = 966, against 0.6).
+constexpr int kTld = kWy + 1;
+constexpr int kTGs = 64 * 65;  // G12 of a level, all pairs: at most 64 (s + 1)
+constexpr int kTSmem = (kWy * kTld + 2 * kTGs) * 8;
+__global__ void __launch_bounds__(kBlock) wy_t_block_kernel(const double* __restrict__ G, const double* __restrict__ tau,
+                                                            int p, int b, double* __restrict__ T) {
+  static_assert(kWy == 128 && kBlock == 256, "the joins below are laid out for 128 rows and 256 threads");
+  extern __shared__ __align__(16) double wy_smem[];
+  double* Ts = wy_smem;
+  double* Gs = Ts + kWy * kTld;
+  double* Ms = Gs + kTGs;
+  const int tid = threadIdx.x;
+  for (int q = tid; q < kWy * kTld; q += kBlock) Ts[q] = 0.0;
+  for (int q = tid; q < kWy * 16; q += kBlock) {  // diagonal blocks of G
+    const int r = q >> 4, c = (r & ~15) + (q & 15);
+    Gs[q] = r < b && c < b ? G[(size_t)r * b + c] : 0.0;
   }
+  __syncthreads();
+  if (tid < b) {
+    const int m = tid, B = m & ~15, end = min(B + 16, b);
+    double* row = Ts + m * kTld;
+    row[m] = tau[p + m];
+    for (int k = m + 1; k < end; ++k) {
+      double a = 0.0;
+      for (int l = m; l < k; ++l) a = fma(row[l], Gs[l * 16 + (k - B)], a);
+      row[k] = -tau[p + k] * a;
+    }
+  }
+  for (int s = 16; s < kWy; s *= 2) {
+    const int ld = s + 1, pairs = kWy / (2 * s), q4 = s / 4;
+    __syncthreads();
+    for (int e = tid; e < pairs * s * s; e += kBlock) {
+      const int q = e / (s * s), i = (e / s) % s, j = e % s, r = 2 * s * q + i, c = 2 * s * q + s + j;
+      Gs[q * s * ld + i * ld + j] = r < b && c < b ? G[(size_t)r * b + c] : 0.0;
+    }
+    __syncthreads();
+    // tile of 4 x 4 elements, rows ti + q4 a, columns tj + q4 c, of one pair per thread
+    const bool on = tid < pairs * q4 * q4;
+    const int q = tid / (q4 * q4), ti = (tid / q4) % q4, tj = tid % q4, o1 = 2 * s * q, o2 = o1 + s;
+    double acc[4][4];
+    for (int pass = 0; pass < 2; ++pass) {  // M = G12 T2, then T12 = -T1 M
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[a][c] = 0.0;
+      if (on) {
+        const double* L = pass == 0 ? Gs + q * s * ld : Ts + o1 * kTld + o1;
+        const double* R = pass == 0 ? Ts + o2 * kTld + o2 : Ms + q * s * ld;
+        const int ll = pass == 0 ? ld : kTld, lr = pass == 0 ? kTld : ld;
+        for (int l = 0; l < s; ++l) {
+          double x[4], y[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            x[a] = L[(ti + q4 * a) * ll + l];
+            y[a] = R[l * lr + tj + q4 * a];
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[a][c] = fma(x[a], y[c], acc[a][c]);
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (pass == 0) Ms[q * s * ld + (ti + q4 * a) * ld + tj + q4 * c] = acc[a][c];
+            else Ts[(o1 + ti + q4 * a) * kTld + o2 + tj + q4 * c] = -acc[a][c];
+          }
+      }
+      __syncthreads();
+    }
+  }
+  for (int q = tid; q < kWy * kWy; q += kBlock) T[q] = Ts[(q / kWy) * kTld + q % kWy];
 }
 
 // ---------------------------------------------------------------- tridiagonal eigenproblem
@@ -717,22 +772,26 @@ __global__ void __launch_bounds__(kBlock) multisect_kernel(const double* d, cons
   const double v = multisect(d, e2, n, j, j < kval, g, glo, ghi, pivmin, tnorm, prev, dprev);
   if (j < kval && gt % g == 0) lam[j] = v;
 }
-// Eigenvector j < kvec of T by twisted factorisation (thread per vector), written as column j of
-// Y (n x kvec, row-major); zero outside the unreduced block that holds eigenvalue j. Scratch
-// arrays are interleaved by vector (element i of vector j at i * kvec + j) so a warp's accesses
-// coalesce. `blk` lists the nb + 1 block starts.
-__global__ void __launch_bounds__(kBlock) twisted_kernel(const double* d, const double* e, const double* e2, int n,
-                                                         int kvec, const double* lam, const int* blk, int nb,
-                                                         double pivmin, double tnorm, double* Y, double* Dp, double* Lp,
-                                                         double* Um) {
-  const int j = blockIdx.x * kBlock + threadIdx.x;
+// Eigenvectors j < kvec of T by the twisted factorisation as the per-CTA path forms them (cta_eigen.cuh): the recurrence of T
+// from the first row down (F, blockIdx.y = 0) and from the last row up (G, blockIdx.y = 1), one thread per vector and
+// direction, pairs rescaled every 8 rows with the exponents in EF / EG. All arrays have the vector index fastest
+// (element i of vector j at i * kvec + j). `inve` holds 1 / e (0 where T splits), `blk` the nb + 1 block starts;
+// the unreduced block that holds eigenvalue j goes to vb[j].
+constexpr int kTwist = 64;
+__global__ void __launch_bounds__(kTwist) twist_sweep_kernel(const double* __restrict__ d, const double* __restrict__ e,
+                                                             const double* __restrict__ e2, const double* __restrict__ inve, int n,
+                                                             int kvec, const double* __restrict__ lam, const int* __restrict__ blk,
+                                                             int nb, double pivmin, double tnorm, double* __restrict__ F,
+                                                             double* __restrict__ G, int* __restrict__ EF, int* __restrict__ EG,
+                                                             int* __restrict__ vb) {
+  const int j = blockIdx.x * kTwist + threadIdx.x;
   if (j >= kvec) return;
+  const bool down = blockIdx.y == 0;
   const double lj = lam[j];
   const double win = 1.0e-11 * fmax(tnorm, 1.0);
-  const size_t K = (size_t)kvec;
   // which unreduced block holds this eigenvalue (equal eigenvalues go to successive blocks)
-  int pos = j - sturm(d, e2, 0, n - 1, lj - win, pivmin);
-  int b = -1;
+  int b = nb == 1 ? 0 : -1;
+  int pos = nb == 1 ? 0 : j - sturm(d, e2, 0, n - 1, lj - win, pivmin);
   for (int q = 0; q < nb && b < 0; ++q) {
     const int lo = blk[q], hi = blk[q + 1] - 1;
     const int cnt = sturm(d, e2, lo, hi, lj + win, pivmin) - sturm(d, e2, lo, hi, lj - win, pivmin);
@@ -740,64 +799,189 @@ __global__ void __launch_bounds__(kBlock) twisted_kernel(const double* d, const 
     else pos -= cnt;
   }
   if (b < 0) b = 0;
-  const int lo = blk[b], hi = blk[b + 1] - 1, m = hi - lo + 1;
-  for (int i = 0; i < n; ++i) Y[i * K + j] = 0.0;
-  if (m == 1) {
-    Y[(size_t)lo * K + j] = 1.0;
-    return;
-  }
-  double dp = d[lo] - lj;
-  for (int i = 0; i < m - 1; ++i) {
-    if (fabs(dp) < pivmin) dp = dp < 0.0 ? -pivmin : pivmin;
-    Dp[(lo + i) * K + j] = dp;
-    const double ei = e[lo + i];
-    const double l = ei / dp;
-    Lp[(lo + i) * K + j] = l;
-    dp = (d[lo + i + 1] - lj) - l * ei;
-  }
-  if (fabs(dp) < pivmin) dp = dp < 0.0 ? -pivmin : pivmin;
-  Dp[(size_t)hi * K + j] = dp;
-  double dm = d[hi] - lj;
-  if (fabs(dm) < pivmin) dm = dm < 0.0 ? -pivmin : pivmin;
-  double best = fabs(Dp[(size_t)hi * K + j] + dm - (d[hi] - lj));
-  int r = m - 1;
-  for (int i = m - 2; i >= 0; --i) {
-    const double ei = e[lo + i];
-    const double u = ei / dm;
-    Um[(lo + i) * K + j] = u;
-    dm = (d[lo + i] - lj) - u * ei;
-    if (fabs(dm) < pivmin) dm = dm < 0.0 ? -pivmin : pivmin;
-    const double gm = fabs(Dp[(lo + i) * K + j] + dm - (d[lo + i] - lj));
-    if (gm < best) {
-      best = gm;
-      r = i;
+  if (down) vb[j] = b;
+  const int lo = blk[b], m = blk[b + 1] - lo;
+  // step t goes from row lo + t to the next, or from row hi - t to the one before
+  const int step = down ? 1 : -1;
+  const double* dd = d + (down ? lo : lo + m - 1);
+  const double* ee = e + (down ? lo : lo + m - 2);
+  const double* iv = inve + (down ? lo : lo + m - 2);
+  double* out = (down ? F : G) + (size_t)(down ? lo : lo + m - 1) * kvec + j;
+  int* ex = (down ? EF : EG) + j;
+  const ptrdiff_t os = (ptrdiff_t)step * kvec;
+  double f = 1.0, fm = 0.0;
+  int exq = 0;
+  *out = f;
+  *ex = 0;
+  for (int t0 = 0; t0 < m - 1; t0 += 8) {
+    double A[8], B[8], y[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int t = min(t0 + u, m - 2);
+      const double inv = iv[step * t];
+      A[u] = (lj - dd[step * t]) * inv;
+      B[u] = t > 0 ? ee[step * (t - 1)] * inv : 0.0;
     }
+    if (t0 > 0) {
+      const int q = pair_exponent(f, fm);
+      const double sc = pow2(-q);
+      f *= sc;
+      fm *= sc;
+      exq += q;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const double fn = fma(A[u], f, -(B[u] * fm));
+      fm = f;
+      f = y[u] = fn;
+    }
+    ex[(size_t)(t0 >> 3) * kvec] = exq;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (t0 + u < m - 1) out[os * (t0 + u + 1)] = y[u];
   }
-  // N_r D_r N_r^T y = gamma_r e_r
-  double ynext = 1.0, ynext2 = 0.0;  // y[i+1], y[i+2] going up
-  double yrm1 = 0.0;                 // y[r-1], seeds the downward sweep
-  Y[(size_t)(lo + r) * K + j] = 1.0;
-  double nrm = 1.0;
-  for (int i = r - 1; i >= 0; --i) {
-    double zv = -Lp[(lo + i) * K + j] * ynext;
-    if (ynext == 0.0 && i + 2 < m) zv = -(e[lo + i + 1] / e[lo + i]) * ynext2;
-    Y[(size_t)(lo + i) * K + j] = zv;
-    nrm = fma(zv, zv, nrm);
-    if (i == r - 1) yrm1 = zv;
-    ynext2 = ynext;
-    ynext = zv;
+}
+// The twist row r of the largest |f g| and the vector, y = f / f_r above it, g / g_r from it on, unit norm, into column j of
+// Y (n x kvec, row-major; zero outside its block). 32 vectors a block, the rows shared by 8 threads each.
+__global__ void __launch_bounds__(kBlock) twist_vector_kernel(int n, int kvec, const int* __restrict__ blk, const int* __restrict__ vb,
+                                                              const double* __restrict__ F, const double* __restrict__ G,
+                                                              const int* __restrict__ EF, const int* __restrict__ EG,
+                                                              double* __restrict__ Y) {
+  constexpr int S = kBlock / 32;
+  __shared__ double skey[S][32];
+  __shared__ int srow[S][32];
+  __shared__ double snrm[S][32];
+  const int lane = threadIdx.x & 31, sh = threadIdx.x >> 5;
+  const int jj = blockIdx.x * 32 + lane, j = min(jj, kvec - 1);
+  const size_t K = (size_t)kvec;
+  const int b = vb[j], lo = blk[b], hi = blk[b + 1] - 1;
+  auto ef = [&](int i) { return EF[(size_t)(max(i - lo - 1, 0) >> 3) * K + j]; };
+  auto eg = [&](int i) { return EG[(size_t)(max(hi - i - 1, 0) >> 3) * K + j]; };
+  double best = -INFINITY;
+  int br = hi;
+  for (int i0 = lo + 8 * sh; i0 <= hi; i0 += 8 * S) {
+    double key[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int i = min(i0 + u, hi);
+      key[u] = scaled_order(fabs(F[(size_t)i * K + j] * G[(size_t)i * K + j]), ef(i) + eg(i));
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (key[u] > best) {
+        best = key[u];
+        br = min(i0 + u, hi);
+      }
   }
-  double yprev = 1.0, yprev2 = yrm1;  // y[i], y[i-1] going down
-  for (int i = r; i < m - 1; ++i) {
-    double zv = -Um[(lo + i) * K + j] * yprev;
-    if (yprev == 0.0 && i >= 1) zv = -(e[lo + i - 1] / e[lo + i]) * yprev2;
-    Y[(size_t)(lo + i + 1) * K + j] = zv;
-    nrm = fma(zv, zv, nrm);
-    yprev2 = yprev;
-    yprev = zv;
+  skey[sh][lane] = best;
+  srow[sh][lane] = br;
+  __syncthreads();
+  int r = srow[0][lane];
+  best = skey[0][lane];
+#pragma unroll
+  for (int q = 1; q < S; ++q)
+    if (skey[q][lane] > best) {
+      best = skey[q][lane];
+      r = srow[q][lane];
+    }
+  const double rf = 1.0 / F[(size_t)r * K + j], rg = 1.0 / G[(size_t)r * K + j];
+  const int efr = ef(r), egr = eg(r);
+  auto value = [&](int i) {
+    if (i < lo || i > hi) return 0.0;
+    return i < r ? F[(size_t)i * K + j] * rf * pow2(ef(i) - efr) : G[(size_t)i * K + j] * rg * pow2(eg(i) - egr);
+  };
+  double nrm = 0.0;
+  for (int i0 = 8 * sh; i0 < n; i0 += 8 * S) {
+    double y[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[u] = i0 + u < n ? value(i0 + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) nrm = fma(y[u], y[u], nrm);
   }
-  const double sc = 1.0 / sqrt(nrm);
-  for (int i = lo; i <= hi; ++i) Y[(size_t)i * K + j] *= sc;
+  snrm[sh][lane] = nrm;
+  __syncthreads();
+  double t = 0.0;
+#pragma unroll
+  for (int q = 0; q < S; ++q) t += snrm[q][lane];
+  const double sc = 1.0 / sqrt(t);
+  for (int i0 = 8 * sh; i0 < n; i0 += 8 * S) {
+    double y[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[u] = i0 + u < n ? value(i0 + u) * sc : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i0 + u < n && jj < kvec) Y[(size_t)(i0 + u) * K + j] = y[u];
+  }
+}
+
+// The accelerator's new Gram row in one pass over the lower triangles (every product pairs two symmetric or two antisymmetric
+// matrices): per block 32 partial sums, [l] <E_l, E>, [8 + l] <D, F_l>, [16 + l] <D_l, F>, [24] <E, E>, [25] <D, F>.
+// Eb is null for a restricted run, D for one that keeps no densities.
+struct GramIn {
+  const double* E[kMaxDepth];
+  const double* E2[kMaxDepth];
+  const double* F[kMaxDepth];
+  const double* D[kMaxDepth];
+  int len;
+};
+__global__ void __launch_bounds__(kBlock) gram_kernel(GramIn in, const double* __restrict__ E, const double* __restrict__ Eb,
+                                                      const double* __restrict__ F, const double* __restrict__ D, int n,
+                                                      double* __restrict__ partial) {
+  const int warps = gridDim.x * (kBlock / 32), lane = threadIdx.x & 31;
+  double acc[32];
+#pragma unroll
+  for (int q = 0; q < 32; ++q) acc[q] = 0.0;
+  for (int r = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); r < n; r += warps)
+    for (int col = lane; col <= r; col += 32) {
+      const size_t k = (size_t)r * n + col;
+      const double wgt = col == r ? 1.0 : 2.0;
+      double vE[kMaxDepth], vF[kMaxDepth], vD[kMaxDepth];
+#pragma unroll
+      for (int l = 0; l < kMaxDepth; ++l) {
+        vE[l] = l < in.len ? in.E[l][k] : 0.0;
+        vF[l] = l < in.len && D ? in.F[l][k] : 0.0;
+        vD[l] = l < in.len && D ? in.D[l][k] : 0.0;
+      }
+      const double e = E[k], f = F[k], dn = D ? D[k] : 0.0;
+      const double we = wgt * e, wf = wgt * f, wd = wgt * dn;
+      acc[24] = fma(we, e, acc[24]);
+      acc[25] = fma(wd, f, acc[25]);
+#pragma unroll
+      for (int l = 0; l < kMaxDepth; ++l) {
+        acc[l] = fma(vE[l], we, acc[l]);
+        acc[8 + l] = fma(wd, vF[l], acc[8 + l]);
+        acc[16 + l] = fma(vD[l], wf, acc[16 + l]);
+      }
+      if (Eb) {
+        const double eb = Eb[k], web = wgt * eb;
+        acc[24] = fma(web, eb, acc[24]);
+#pragma unroll
+        for (int l = 0; l < kMaxDepth; ++l)
+          if (l < in.len) acc[l] = fma(in.E2[l][k], web, acc[l]);
+      }
+    }
+  __shared__ double red[kBlock / 32][32];
+  red[threadIdx.x >> 5][lane] = warp_sum32(acc);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    for (int w = 0; w < kBlock / 32; ++w) t += red[w][threadIdx.x];
+    partial[(size_t)blockIdx.x * 32 + threadIdx.x] = t;
+  }
+}
+// out[q] = sum over the blocks of partial[block][q], q < 32, in a fixed order
+__global__ void __launch_bounds__(kBlock) gram_finish_kernel(const double* __restrict__ partial, int np, double* __restrict__ out) {
+  __shared__ double red[kBlock / 32][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double t = 0.0;
+  for (int b = w; b < np; b += kBlock / 32) t += partial[(size_t)b * 32 + lane];
+  red[w][lane] = t;
+  __syncthreads();
+  if (w == 0) {
+    t = 0.0;
+    for (int q = 0; q < kBlock / 32; ++q) t += red[q][lane];
+    out[lane] = t;
+  }
 }
 
 // ---------------------------------------------------------------- properties

@@ -756,7 +756,9 @@ cudaError_t dgemm_ready(int device) {
   if (device < 0) return cudaErrorInvalidDevice;
   if ((int)done.size() <= device) done.resize(device + 1, 0);
   if (done[device]) return cudaSuccess;
-  const cudaError_t e = dg::set_attributes();
+  cudaError_t e = dg::set_attributes();
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(large::wy_t_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, large::kTSmem);
   if (e == cudaSuccess) done[device] = 1;
   return e;
 }
