@@ -50,13 +50,14 @@ struct LargeBufs {
   DevBuf Gm, Mm, Tm, Z1, Z2, blocks, Gk;
   DevBuf mh[2], ml[2], c32;  // mixed mode: BF16 hi / lo parts of two operands, FP32 product
   DevBuf gsync, vw, wv;      // cooperative panels: grid barrier, X = [V | W] and Y = [W | V]
+  DevBuf tsync, tbuf;        // register-tile reduction: grid barrier, exchange buffer
   DevBuf Fchk;               // eigen-residual check: the diagonalised matrix rebuilt
   DevBuf tcerr;              // error flag of the tcgen05 split-BF16 GEMM
   bool tcerr_zeroed = false;
   void release() {
     for (DevBuf* b : {&ao, &sprow, &sroff, &H, &W, &hacc, &dpk, &jacc, &part, &part2, &scal, &P[0], &P[1], &Q[0], &Q[1], &Pt,
                       &F, &G, &hist, &A, &d, &e, &e2, &inve, &tau, &lam, &dlam, &blk, &V, &Wp, &y, &wtmp, &ps, &s64, &vcol, &tp, &ctr, &refl, &X, &Xt,
-                      &Tf, &Tg, &Te, &Gm, &Mm, &Tm, &Z1, &Z2, &blocks, &Gk, &mh[0], &mh[1], &ml[0], &ml[1], &c32, &gsync, &vw, &wv, &Fchk, &tcerr})
+                      &Tf, &Tg, &Te, &Gm, &Mm, &Tm, &Z1, &Z2, &blocks, &Gk, &mh[0], &mh[1], &ml[0], &ml[1], &c32, &gsync, &vw, &wv, &tsync, &tbuf, &Fchk, &tcerr})
       b->release();
     tcerr_zeroed = false;
     gwork.release();
@@ -557,10 +558,10 @@ class LargeSolver {
       float t = 0.0f;
       CUDA_TRY(c_, cudaEventElapsedTime(&t, c_->kev[0], c_->kev[1]));
       *ms = t;
-      if (rc == PM3GPU_OK && coop_grid() > 0) {
+      if (rc == PM3GPU_OK && reduction_sync()) {
         large::GridSync gsh{};
-        CUDA_TRY(c_, cudaMemcpy(&gsh, B_.gsync.p, sizeof(gsh), cudaMemcpyDeviceToHost));
-        if (gsh.err) rc = fail(c_, PM3GPU_CUDA_ERROR, "Householder panel: a grid barrier wait ran out");
+        CUDA_TRY(c_, cudaMemcpy(&gsh, reduction_sync(), sizeof(gsh), cudaMemcpyDeviceToHost));
+        if (gsh.err) rc = fail(c_, PM3GPU_CUDA_ERROR, "Householder reduction: a grid barrier wait ran out");
       }
     }
     c_->force_coop = -1;
@@ -574,6 +575,7 @@ class LargeSolver {
   const int32_t* hz_ = nullptr;
   int N_ = 0, n_ = 0;
   int coop_g_ = -1;  // cooperative panel grid for this device (-1: not yet queried)
+  int tile_g_ = -1;  // resident CTAs of the register-tile reduction (-1: not yet queried)
   int passes_ = 0;  // SCF passes of this molecule (first pass, stability rungs)
   size_t nn_ = 0;
   long long wcap_ = 1;
@@ -728,6 +730,20 @@ class LargeSolver {
   // set of buffers, so it is captured once into a CUDA graph and replayed in later SCF
   // iterations (it is ~5 launches per column). Streams that cannot be captured run it directly.
   int run_tridiag(double* A) {
+    if (const int tiles = tile_grid()) {
+      CUDA_TRY(c_, B_.tsync.ensure(sizeof(large::GridSync)));
+      CUDA_TRY(c_, B_.tbuf.ensure(8 * large::tile_exchange(n_)));
+      CUDA_TRY(c_, cudaMemsetAsync(B_.tsync.p, 0, sizeof(large::GridSync), c_->stream));
+      double *d = B_.d.as<double>(), *e = B_.e.as<double>(), *tau = B_.tau.as<double>();
+      double *tp = B_.tp.as<double>(), *buf = B_.tbuf.as<double>();
+      large::GridSync* gs = B_.tsync.as<large::GridSync>();
+      int n = n_;
+      void* args[] = {&A, &n, &d, &e, &tau, &tp, &buf, &gs};
+      CUDA_TRY(c_, cudaLaunchCooperativeKernel((const void*)large::tile_reduce_kernel, dim3(tiles), dim3(large::kBlock), args,
+                                               0, c_->stream));
+      ++c_->launches;
+      return PM3GPU_OK;
+    }
     if (coop_grid() > 0) {  // one cooperative launch per panel: few enough launches to issue directly
       int launches = 0;
       const int rc = enqueue_tridiag(A, launches);
@@ -801,6 +817,26 @@ class LargeSolver {
     return coop_g_;
   }
   static constexpr int kCoopSmallN = 512;  // at most 8 stripes of 64 rows
+
+  // Grid of the register-tile reduction (tile_reduce.cuh), 0 when the matrix has more tiles than can be resident (two CTAs per
+  // SM: n > 1472 on 148 SMs) or the cooperative reductions are off. Up to there it beats the panels at every size
+  // (n = 966: 4.6 against 12.7 ms).
+  int tile_grid() {
+    if (n_ < 3 || coop_grid() <= 0) return 0;
+    if (tile_g_ < 0) {
+      int occ = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large::tile_reduce_kernel, large::kBlock, 0) != cudaSuccess) {
+        (void)cudaGetLastError();
+        occ = 0;
+      }
+      tile_g_ = std::min(occ, 2) * c_->sms;
+    }
+    const int nts = large::tile_stripes(n_);
+    const long long tiles = (long long)nts * (nts + 1) / 2;
+    return nts <= large::kTileMaxStripes && tiles <= tile_g_ ? (int)tiles : 0;
+  }
+  // The barrier record of the reduction that run_tridiag takes, null for the multi-launch one.
+  const void* reduction_sync() { return tile_grid() > 0 ? B_.tsync.p : (coop_grid() > 0 ? B_.gsync.p : nullptr); }
 
   // Enqueues the blocked reduction of A (no host synchronisation inside).
   int enqueue_tridiag(double* A, int& launches) {
@@ -988,10 +1024,10 @@ class LargeSolver {
       CUDA_TRY(c_, cudaMemcpyAsync(hd.data(), d, 8 * (size_t)n, cudaMemcpyDeviceToHost, c_->stream));
       CUDA_TRY(c_, cudaMemcpyAsync(he.data(), e, 8 * (size_t)n, cudaMemcpyDeviceToHost, c_->stream));
       large::GridSync gsh{};
-      if (coop_grid() > 0)
-        CUDA_TRY(c_, cudaMemcpyAsync(&gsh, B_.gsync.p, sizeof(gsh), cudaMemcpyDeviceToHost, c_->stream));
+      if (reduction_sync())
+        CUDA_TRY(c_, cudaMemcpyAsync(&gsh, reduction_sync(), sizeof(gsh), cudaMemcpyDeviceToHost, c_->stream));
       CUDA_TRY(c_, cudaStreamSynchronize(c_->stream));
-      if (gsh.err) return fail(c_, PM3GPU_CUDA_ERROR, "Householder panel: a grid barrier wait ran out");
+      if (gsh.err) return fail(c_, PM3GPU_CUDA_ERROR, "Householder reduction: a grid barrier wait ran out");
       if (tri) {
         tri->assign(2 * (size_t)n, 0.0);
         std::copy(hd.begin(), hd.end(), tri->begin());

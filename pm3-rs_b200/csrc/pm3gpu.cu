@@ -19,6 +19,7 @@
 #include "gradient_kernel.cuh"
 #include "large_scf.cuh"
 #include "panel_coop.cuh"
+#include "tile_reduce.cuh"
 #include "guess_mlp.cuh"
 #include "scf_job.cuh"
 #include "tc_gemm.cuh"
