@@ -303,8 +303,10 @@ inline Plan plan(int m, int n, int k, int sms) {
   p.tiles_m = (m + p.bm - 1) / p.bm;
   p.tiles_n = (n + p.bn - 1) / p.bn;
   const int tiles = p.tiles_m * p.tiles_n, slots = sms * per_sm[p.kind];
-  int splits = 1;  // as many K slices as fill the resident slots in one wave
-  if (tiles * 2 <= slots && k >= 1024) splits = std::max(1, std::min(slots / tiles, k / 256));
+  // As many K slices as fill the resident slots in one wave, of at least 128: one 128 x 128 tile alone takes 106 us at
+  // k = 966 (an SM's whole FP64 rate), seven slices and their sum 25.
+  int splits = 1;
+  if (tiles * 2 <= slots && k >= 256) splits = std::max(1, std::min(slots / tiles, k / 128));
   int kchunk = (k + splits - 1) / splits;
   kchunk = std::max(kBK, (kchunk + kBK - 1) / kBK * kBK);
   p.splits = std::max(1, (k + kchunk - 1) / kchunk);

@@ -631,8 +631,7 @@ class LargeSolver {
     large::pack_density_kernel<<<gN, large::kBlock, 0, c_->stream>>>(m_, Pt, B_.dpk.as<double>(), B_.jacc.as<double>());
     const long long np = (long long)N_ * (N_ - 1) / 2;
     const int gp = grid_for((size_t)std::max<long long>(np, 1));
-    const int ga = (N_ + large::kBlock / 32 - 1) / (large::kBlock / 32);  // one warp per atom
-    large::coulomb_atoms_kernel<<<ga, large::kBlock, 0, c_->stream>>>(m_, B_.W.as<double>(), B_.dpk.as<double>(),
+    large::coulomb_atoms_kernel<<<N_, large::kBlock, 0, c_->stream>>>(m_, B_.W.as<double>(), B_.dpk.as<double>(),
                                                                       B_.jacc.as<double>());
     ++c_->launches;
     if (Pb)

@@ -194,15 +194,15 @@ __global__ void __launch_bounds__(kBlock) pack_density_kernel(Mol m, const doubl
   }
 }
 // Two-centre Coulomb sums of the Fock build, J_x[p] = sum_{y != x} sum_q (x p | y q) Pbar_y[q]
-// (fock.rs:106-159), one warp per atom x, lanes over the partners in a fixed order (the pair
-// kernel leaves them out), so the Fock matrix does not depend on timing. Pair blocks are stored
+// (fock.rs:106-159), one block per atom x, threads over the partners in a fixed order (the pair
+// kernel leaves them out), so the Fock matrix does not depend on timing (483 atoms: one warp an atom took 314 us, each lane
+// 15 partners one after another). Pair blocks are stored
 // in (a, b) orientation, a the atom with more orbitals (the first one on a tie).
 __global__ void __launch_bounds__(kBlock) coulomb_atoms_kernel(Mol m, const double* W, const double* dpk, double* jacc) {
-  const int lane = threadIdx.x & 31, x = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
-  if (x >= m.N) return;  // whole warps
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, x = blockIdx.x;
   const int sx = m.sprow[x + 1] - m.sprow[x];
   double acc[10] = {};
-  for (int y = lane; y < m.N; y += 32) {
+  for (int y = threadIdx.x; y < m.N; y += kBlock) {
     if (y == x) continue;
     const int sy = m.sprow[y + 1] - m.sprow[y];
     const int u = min(x, y), v = max(x, y);
@@ -222,10 +222,17 @@ __global__ void __launch_bounds__(kBlock) coulomb_atoms_kernel(Mol m, const doub
       acc[p] += t;
     }
   }
+  __shared__ double red[10][kBlock / 32];
 #pragma unroll
   for (int p = 0; p < 10; ++p) {
     const double t = warp_sum(acc[p]);
-    if (lane == 0 && p < sx) jacc[10 * (size_t)x + p] = t;
+    if (lane == 0) red[p][warp] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < sx) {
+    double t = 0.0;
+    for (int w = 0; w < kBlock / 32; ++w) t += red[threadIdx.x][w];
+    jacc[10 * (size_t)x + threadIdx.x] = t;
   }
 }
 template <bool UHF>
