@@ -207,32 +207,13 @@ __device__ __forceinline__ int tri_cols(double (&a)[kRegB * (kRegB + 1) / 2], co
   const int end = min(base + 16 * (B0 + 1), c.M - 2);
   for (; i < end; ++i) {
     const Refl h = reflector(c, i);
-    constexpr int R = NB > 3 ? 8 : (NB > 1 ? 4 : 2);  // row sums and, in the last place, v^T A v
     {
-      double vc[NB], pc[NB], py[R], dot = 0.0;
+      double vc[NB], pc[NB], dot = 0.0;
 #pragma unroll
       for (int k = 0; k < NB; ++k) {
         vc[k] = c.xs[base + 16 * (B0 + k) + tx];
         pc[k] = 0.0;
       }
-#pragma unroll
-      for (int I = 0; I < NB; ++I) {
-        const double vr = c.xs[base + 16 * (B0 + I) + ty];
-        double acc = 0.0;
-#pragma unroll
-        for (int J = 0; J <= I; ++J) {
-          const double x = a[rblk(B0 + I, B0 + J)];
-          acc = fma(x, vc[J], acc);
-          if (J < I) pc[J] = fma(x, vr, pc[J]);
-        }
-        dot = fma(acc, vr, dot);
-        py[I] = acc;
-      }
-#pragma unroll
-      for (int J = 0; J < NB; ++J) dot = fma(pc[J], vc[J], dot);
-#pragma unroll
-      for (int I = NB; I < R - 1; ++I) py[I] = 0.0;
-      py[R - 1] = dot;
       // the next column's present values
       if (tx == ((i + 1) & 15)) {
         const bool nextb = tx == 0;
@@ -243,24 +224,53 @@ __device__ __forceinline__ int tri_cols(double (&a)[kRegB * (kRegB + 1) / 2], co
           c.raw[base + 16 * (B0 + I) + ty] = x;
         }
       }
+      // rows four blocks at a time: their sums over the 16 lanes of a row, and with the last ones x^T A x
+#pragma unroll
+      for (int I0 = 0; I0 < NB; I0 += 4) {
+        constexpr bool kFull = (NB & 3) == 0;  // no free place beside the last rows
+        double py[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int I = I0 + k;
+          double acc = 0.0;
+          if (I < NB) {
+            const double vr = c.xs[base + 16 * (B0 + I) + ty];
+#pragma unroll
+            for (int J = 0; J <= I; ++J) {
+              const double x = a[rblk(B0 + I, B0 + J)];
+              acc = fma(x, vc[J], acc);
+              if (J < I) pc[J] = fma(x, vr, pc[J]);
+            }
+            dot = fma(acc, vr, dot);
+          }
+          py[k] = acc;
+        }
+        const bool last = I0 + 4 >= NB;
+        if (last) {
+#pragma unroll
+          for (int J = 0; J < NB; ++J) dot = fma(pc[J], vc[J], dot);
+          if (!kFull) py[3] = dot;
+        }
+        const double sum = sum16_of4(py, lane);
+        const int I = I0 + ((lane & 15) >> 2);
+        if ((lane & 3) == 0 && I < NB) c.rsum[base + 16 * (B0 + I) + ty] = sum;
+        if (last) {
+          double q = sum;  // lane 12 of each half
+          if (kFull) {
+            q = dot;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+          }
+          q += __shfl_xor_sync(0xffffffffu, q, 16);
+          if (lane == 12) c.dpart[tid >> 5] = q;
+        }
+      }
       // column sums over this warp's two rows of threads, then one partial per warp
 #pragma unroll
       for (int J = 0; J < NB; ++J) pc[J] += __shfl_xor_sync(0xffffffffu, pc[J], 16);
       if (lane < 16) {
 #pragma unroll
         for (int J = 0; J < NB; ++J) c.cpart[(base + 16 * (B0 + J) + tx) * kPart + (tid >> 5)] = pc[J];
-      }
-      // row sums over the 16 lanes of a row
-      double sum;
-      if constexpr (R == 8) sum = sum16_of8(py, lane);
-      else if constexpr (R == 4) sum = sum16_of4(py, lane);
-      else sum = sum16_of2(py, lane);
-      constexpr int S = 16 / R;  // lanes that share a sum
-      const int I = (lane & 15) / S;
-      const double both = sum + __shfl_xor_sync(0xffffffffu, sum, 16);
-      if ((lane & (S - 1)) == 0) {
-        if (I < NB) c.rsum[base + 16 * (B0 + I) + ty] = sum;
-        if (I == R - 1 && lane < 16) c.dpart[tid >> 5] = both;
       }
     }
     __syncthreads();
@@ -340,9 +350,6 @@ __device__ __forceinline__ int tri_mem_cols(double (&a)[kRegB * (kRegB + 1) / 2]
         for (int J = 0; J < kRegB; ++J) c.cpart[(base + 16 * J + tx) * kPart + (tid >> 5)] = pc[J];
       }
     }
-    double vr[kRegB];
-#pragma unroll
-    for (int k = 0; k < kRegB; ++k) vr[k] = c.xs[base + 16 * k + ty];
     for (int J = B; J < mb; ++J) {
       const double vcj = c.xs[16 * J + tx];
       double pcj = 0.0;
@@ -352,7 +359,7 @@ __device__ __forceinline__ int tri_mem_cols(double (&a)[kRegB * (kRegB + 1) / 2]
       for (int k = 0; k < kRegB; ++k, q += kThreads) {
         const double x = *q;
         py[k] = fma(x, vcj, py[k]);
-        pcj = fma(x, vr[k], pcj);
+        pcj = fma(x, c.xs[base + 16 * k + ty], pcj);
       }
       dot = fma(pcj, vcj, dot);
       const double s = pcj + __shfl_xor_sync(0xffffffffu, pcj, 16);
@@ -367,7 +374,7 @@ __device__ __forceinline__ int tri_mem_cols(double (&a)[kRegB * (kRegB + 1) / 2]
       if ((lane & 15) == 0) c.rsum[16 * I + ty] = acc;
     }
 #pragma unroll
-    for (int I = 0; I < kRegB; ++I) dot = fma(py[I], vr[I], dot);
+    for (int I = 0; I < kRegB; ++I) dot = fma(py[I], c.xs[base + 16 * I + ty], dot);
     py[7] = dot;
     {
       const double s = sum16_of8(py, lane);
@@ -391,7 +398,7 @@ __device__ __forceinline__ int tri_mem_cols(double (&a)[kRegB * (kRegB + 1) / 2]
     tri_rows(c, 16 * B, i, h);
     __syncthreads();
     store_reflector(c, 16 * B, i);
-    double wr[kRegB];
+    double wr[kRegB], vr[kRegB];
 #pragma unroll
     for (int k = 0; k < kRegB; ++k) {
       wr[k] = c.ws[base + 16 * k + ty];
@@ -427,13 +434,6 @@ struct SymInput {
   size_t stride;
   const double* proj;
   double shift;
-  __device__ __forceinline__ double at(size_t ix, bool diag) const {
-    double v = 0.0;
-    if (len == 0) v = X[ix];
-    for (int l = 0; l < len; ++l) v = fma(coef[l], hist[(size_t)((head + l) % depth) * stride + ix], v);
-    if (shift != 0.0) v += shift * ((diag ? 1.0 : 0.0) - proj[ix]);
-    return v;
-  }
 };
 
 // Householder reduction of the n x n symmetric matrix: diagonals to s.d, s.e,
@@ -464,59 +464,74 @@ __device__ __noinline__ void tridiagonalize(int n, const SymInput& in, double* V
   m.cap = max(0, (s.sh_doubles - 15 * M) / kThreads);
   m.nbt = nbt;
   m.mb = mb;
-  // element (row, col) of a block at this thread, as an index into the lower triangle; -1 in the padding
-  auto index = [&](int I, int J) -> int {
-    const int r = 16 * I + ty - off, q = 16 * J + tx - off;
-    return min(r, q) >= 0 ? max(r, q) * n + min(r, q) : -1;
-  };
+  // Elements of the blocks at this thread, as indices into the lower triangle: affine in the block's coordinates, with other
+  // constants on the diagonal (where both triangles are held). Negative columns are padding.
+  const int r0 = ty - off, q0 = tx - off, hi0 = max(r0, q0), lo0 = min(r0, q0);
+  auto col = [&](int I, int J) { return 16 * J + (I == J ? lo0 : q0); };
+  auto index = [&](int I, int J) { return (16 * I + (I == J ? hi0 : r0)) * n + col(I, J); };
+  const int terms = max(in.len, 1);
+  auto source = [&](int l) { return in.len ? in.hist + (size_t)((in.head + l) % in.depth) * in.stride : in.X; };
+  auto factor = [&](int l) { return in.len ? in.coef[l] : 1.0; };
+  auto shifted = [&](int I, int J) { return in.shift * ((I == J && tx == ty ? 1.0 : 0.0) - in.proj[index(I, J)]); };
+  // the memory blocks, 14 at a time: all their loads of one history matrix in flight together
+  for (int J = 0; J < mb; ++J)
+    for (int I0 = J; I0 < nbt; I0 += 14) {
+      double x[14];
+#pragma unroll
+      for (int k = 0; k < 14; ++k) x[k] = 0.0;
+      for (int l = 0; l < terms; ++l) {
+        const double* __restrict__ src = source(l);
+        const double cf = factor(l);
+#pragma unroll
+        for (int k = 0; k < 14; ++k)
+          if (I0 + k < nbt && col(I0 + k, J) >= 0) x[k] = fma(cf, src[index(I0 + k, J)], x[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 14; ++k)
+        if (I0 + k < nbt) {
+          if (in.shift != 0.0 && col(I0 + k, J) >= 0) x[k] += shifted(I0 + k, J);
+          *m.at(I0 + k, J) = x[k];
+        }
+    }
   double a[kRegB * (kRegB + 1) / 2];
 #pragma unroll
   for (int k = 0; k < kRegB * (kRegB + 1) / 2; ++k) a[k] = 0.0;
-  // history matrices in groups, with all the group's loads in flight: four at a time when a thread has at
-  // most 6 elements, else one (28 loads of one matrix)
+  // The register blocks from block F on: history matrices in groups of U, with all the group's loads in flight.
   auto load = [&](auto first, auto group) {
     constexpr int F = decltype(first)::value, U = decltype(group)::value;
-    const int terms = max(in.len, 1);
     for (int l0 = 0; l0 < terms; l0 += U) {
       const double* src[U];
       double cf[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int l = min(l0 + u, terms - 1);
-        src[u] = in.len ? in.hist + (size_t)((in.head + l) % in.depth) * in.stride : in.X;
-        cf[u] = l0 + u >= terms ? 0.0 : (in.len ? in.coef[l] : 1.0);
+        src[u] = source(l);
+        cf[u] = l0 + u >= terms ? 0.0 : factor(l);
       }
 #pragma unroll
       for (int I = F; I < kRegB; ++I)
 #pragma unroll
-        for (int J = F; J <= I; ++J) {
-          const int ix = index(mb + I, mb + J);
-          if (ix >= 0) {
+        for (int J = F; J <= I; ++J)
+          if (col(mb + I, mb + J) >= 0) {
+            const int ix = index(mb + I, mb + J);
             double x[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) x[u] = src[u][ix];
 #pragma unroll
             for (int u = 0; u < U; ++u) a[rblk(I, J)] = fma(cf[u], x[u], a[rblk(I, J)]);
           }
-        }
     }
   };
   if (off >= 16 * (kRegB - 3)) load(std::integral_constant<int, kRegB - 3>{}, std::integral_constant<int, 4>{});
+  else if (off >= 16 * (kRegB - 5)) load(std::integral_constant<int, kRegB - 5>{}, std::integral_constant<int, 2>{});
   else load(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
   if (in.shift != 0.0) {
 #pragma unroll
     for (int I = 0; I < kRegB; ++I)
 #pragma unroll
-      for (int J = 0; J <= I; ++J) {
-        const int ix = index(mb + I, mb + J);
-        if (ix >= 0) a[rblk(I, J)] += in.shift * ((I == J && tx == ty ? 1.0 : 0.0) - in.proj[ix]);
-      }
+      for (int J = 0; J <= I; ++J)
+        if (col(mb + I, mb + J) >= 0) a[rblk(I, J)] += shifted(mb + I, mb + J);
   }
-  for (int J = 0; J < mb; ++J)
-    for (int I = J; I < nbt; ++I) {
-      const int ix = index(I, J);
-      *m.at(I, J) = ix >= 0 ? in.at(ix, I == J && tx == ty) : 0.0;
-    }
   // publish the first column
   const int B = off >> 4;
   if (tx == (off & 15)) {
@@ -709,7 +724,7 @@ __device__ __forceinline__ double multisect(const double* __restrict__ d, const 
   for (int it = 0; it < 160; ++it) {
     if (act) {
       const double mid = 0.5 * (lo + hi);
-      if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
+      if (hi - lo <= eps * (2.0 * fmax(fabs(lo), fabs(hi)) + tnorm) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
     }
     if (!__any_sync(0xffffffffu, act)) break;
     const double w = hi - lo;
@@ -719,7 +734,7 @@ __device__ __forceinline__ double multisect(const double* __restrict__ d, const 
     if (close) {
       const double a = fabs(flo), b = fabs(fhi);  // the one of the smaller scale counts as 0
       const double r = elo == ehi ? a / (a + b) : (elo > ehi ? 1.0 : 0.0);
-      const double xs = lo + w * r, tiny = eps * fmax(fabs(lo), fabs(hi));
+      const double xs = lo + w * r, tiny = 0.5 * eps * (fmax(fabs(lo), fabs(hi)) + 0.5 * tnorm);
 #pragma unroll
       for (int t = 0; t < kPts; ++t) {  // distances w/4 .. w/2^26 (w/16 for P = 2), below and above
         const int q = gl * kPts + t, k = q < g ? q : P - 1 - q;
