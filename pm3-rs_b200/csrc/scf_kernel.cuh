@@ -411,76 +411,124 @@ __device__ __forceinline__ void fock_pair(int n, int oa, int ob, const double* _
   }
 }
 
-// One pair of the per-CTA Fock build for one spin density X (times xs): the exchange block F_ab = H_ab - K_ab to both
-// triangles and, with kJ, the pair's Coulomb parts J_a[p] = sum_q W[p][q] d_b[q] and
-// J_b[q] = sum_p d_a[p] W[p][q] to sa and sb. The integrals stream through once, row by row with the next row's loads in
-// flight: element (mu nu | la si) adds to the up to four exchange elements that share it. Returns the
-// pair's part of sum P (H + F), both triangles.
-template <int NA, int NB, bool kJ>
-__device__ __forceinline__ double fock_item(int n, int oa, int ob, const double* __restrict__ w, size_t ws,
-                                            const double* da, const double* db, double* sa, double* sb,
-                                            const double* __restrict__ H, const double* __restrict__ X, double xs,
-                                            double* __restrict__ F) {
-  constexpr int PA = NA == 4 ? 10 : 1, PB = NB == 4 ? 10 : 1;
-  double x[NA][NB], k[NA][NB], jb[PB], wv[PB], wn[PB];
+// One pair with at most one heavy atom a (NA = 4 or 1) and a light atom b of the per-CTA Fock build, for one spin density X (times
+// xs): the exchange block F_ab = H_ab - K_ab to both triangles and, with kJ, the pair's Coulomb parts J_a[p] = W[p] d_b and
+// J_b = sum_p d_a[p] W[p] to sa and sb. Returns the pair's part of sum P (H + F), both triangles.
+template <int NA, bool kJ>
+__device__ __forceinline__ double light_item(int n, int oa, int ob, const double* __restrict__ w, int ws, const double* da,
+                                             double db, double* __restrict__ sa, double* __restrict__ sb,
+                                             const double* __restrict__ H, const double* __restrict__ X, double xs,
+                                             double* __restrict__ F) {
+  constexpr int PA = NA == 4 ? 10 : 1;
+  const int ab = oa * n + ob, ba = ob * n + oa;
+  double wv[PA], x[NA], h[NA];
 #pragma unroll
-  for (int q = 0; q < PB; ++q) wn[q] = w[q * ws];
+  for (int p = 0; p < PA; ++p) wv[p] = w[p * ws];
 #pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      x[i][j] = xs * X[(size_t)(oa + i) * n + ob + j];
-      k[i][j] = 0.0;
-    }
-#pragma unroll
-  for (int q = 0; q < PB; ++q) jb[q] = 0.0;
-#pragma unroll
-  for (int mu = 0; mu < NA; ++mu)
-#pragma unroll
-    for (int nu = 0; nu <= mu; ++nu) {
-      const int p = pk(mu, nu);
-#pragma unroll
-      for (int q = 0; q < PB; ++q) wv[q] = wn[q];
-      if (p + 1 < PA) {
-#pragma unroll
-        for (int q = 0; q < PB; ++q) wn[q] = w[((p + 1) * PB + q) * ws];
-      }
-      if (kJ) {
-        const double dp = da[p];
-        double acc = 0.0;
-#pragma unroll
-        for (int q = 0; q < PB; ++q) {
-          acc = fma(db[q], wv[q], acc);
-          jb[q] = fma(dp, wv[q], jb[q]);
-        }
-        sa[p] = acc;
-      }
-#pragma unroll
-      for (int la = 0; la < NB; ++la)
-#pragma unroll
-        for (int si = 0; si <= la; ++si) {
-          const double e = wv[pk(la, si)];
-          k[mu][la] = fma(x[nu][si], e, k[mu][la]);
-          if (mu != nu) k[nu][la] = fma(x[mu][si], e, k[nu][la]);
-          if (la != si) k[mu][si] = fma(x[nu][la], e, k[mu][si]);
-          if (mu != nu && la != si) k[nu][si] = fma(x[mu][la], e, k[nu][si]);
-        }
-    }
+  for (int i = 0; i < NA; ++i) {
+    x[i] = xs * X[ab + i * n];
+    h[i] = H[ab + i * n];
+  }
   if (kJ) {
+    double jb = 0.0;
 #pragma unroll
-    for (int q = 0; q < PB; ++q) sb[q] = jb[q];
+    for (int p = 0; p < PA; ++p) {
+      sa[p] = wv[p] * db;
+      jb = fma(da[p], wv[p], jb);
+    }
+    *sb = jb;
   }
   double en = 0.0;
 #pragma unroll
-  for (int mu = 0; mu < NA; ++mu)
+  for (int mu = 0; mu < NA; ++mu) {
+    double k = 0.0;
 #pragma unroll
-    for (int la = 0; la < NB; ++la) {
-      const double h = H[(size_t)(oa + mu) * n + ob + la], f = h - k[mu][la];
-      F[(size_t)(oa + mu) * n + ob + la] = f;
-      F[(size_t)(ob + la) * n + oa + mu] = f;
-      en = fma(x[mu][la], h + f, en);
-    }
+    for (int nu = 0; nu < NA; ++nu) k = fma(x[nu], wv[pk(mu, nu)], k);
+    const double f = h[mu] - k;
+    F[ab + mu * n] = f;
+    F[ba + mu] = f;
+    en = fma(x[mu], h[mu] + f, en);
+  }
   return 2.0 * en / xs;
+}
+
+// Row mu of a pair of heavy atoms, one of the four lanes that share the pair: the exchange elements F_mu,la and, with kJ, the
+// Coulomb parts of the table rows (mu, nu <= mu), J_b summed over the four lanes. A lane reads 40 of the 100 integrals. (With the whole
+// pair on one lane the few pairs of a small molecule were one warp's chain of 1500 instructions: 18k of the 35k cycles
+// of a Fock build at 11 atoms.) Whole warps call, with `on` false past the last pair.
+template <bool kJ>
+__device__ __forceinline__ double heavy_item(bool on, int n, int oa, int ob, int mu, const double* __restrict__ w, int ws,
+                                             const double* da, const double* db, double* __restrict__ sa,
+                                             double* __restrict__ sb, const double* __restrict__ H,
+                                             const double* __restrict__ X, double xs, double* __restrict__ F) {
+  const int ab = oa * n + ob;
+  double x[4][4], k[4] = {0.0, 0.0, 0.0, 0.0}, jb[12], d[10];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[i][j] = on ? X[ab + i * n + j] : 0.0;
+  if (kJ) {
+#pragma unroll
+    for (int q = 0; q < 12; ++q) jb[q] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 10; ++q) d[q] = db[q];
+  }
+#pragma unroll
+  for (int nu = 0; nu < 4; ++nu) {
+    const int p = mu >= nu ? mu * (mu + 1) / 2 + nu : nu * (nu + 1) / 2 + mu;
+    const double* wr = w + p * 10 * ws;
+    double wv[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) wv[q] = wr[q * ws];
+#pragma unroll
+    for (int la = 0; la < 4; ++la)
+#pragma unroll
+      for (int si = 0; si <= la; ++si) {
+        const double e = wv[pk(la, si)];
+        k[la] = fma(x[nu][si], e, k[la]);
+        if (la != si) k[si] = fma(x[nu][la], e, k[si]);
+      }
+    if (kJ) {
+      const bool mine = on && nu <= mu;
+      const double dp = mine ? da[p] : 0.0;
+      double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+      for (int q = 0; q < 10; q += 2) {
+        a0 = fma(d[q], wv[q], a0);
+        a1 = fma(d[q + 1], wv[q + 1], a1);
+        jb[q] = fma(dp, wv[q], jb[q]);
+        jb[q + 1] = fma(dp, wv[q + 1], jb[q + 1]);
+      }
+      if (mine) sa[p] = a0 + a1;
+    }
+  }
+  if (kJ) {  // twelve places over four lanes: three sums each
+    const bool b1 = mu & 2, b0 = mu & 1;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const double send = b1 ? jb[q] : jb[q + 6], keep = b1 ? jb[q + 6] : jb[q];
+      jb[q] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double send = b0 ? jb[q] : jb[q + 3], keep = b0 ? jb[q + 3] : jb[q];
+      const double t = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+      const int at = (b1 ? 6 : 0) + (b0 ? 3 : 0) + q;
+      if (on && at < 10) sb[at] = t;
+    }
+  }
+  if (!on) return 0.0;
+  double en = 0.0;
+  const int row = ab + mu * n, colm = ob * n + oa + mu;
+#pragma unroll
+  for (int la = 0; la < 4; ++la) {
+    const double h = H[row + la], f = fma(-xs, k[la], h);
+    F[row + la] = f;
+    F[colm + la * n] = f;
+    const double xm = mu == 0 ? x[0][la] : (mu == 1 ? x[1][la] : (mu == 2 ? x[2][la] : x[3][la]));
+    en = fma(xm, h + f, en);
+  }
+  return 2.0 * en;
 }
 
 // The off-diagonal blocks of one spin's Fock matrix over all pairs of the molecule; with kJ also every pair's Coulomb
@@ -495,20 +543,35 @@ __device__ __noinline__ double fock_pairs(const Ctx& c, const double* dpk_, doub
   const double* __restrict__ W = c.W;
   const double* __restrict__ H = c.H;
   double en = 0.0;
-  auto run = [&](auto na, auto nb, int t) {
-    int ia, ib, ws;
-    size_t w0;
-    pair_item(K, t, ia, ib, w0, ws);
-    const int ra = K.row(ia), rb = K.row(ib);
-    en += fock_item<decltype(na)::value, decltype(nb)::value, kJ>(n, soff[order[ia]], soff[order[ib]], W + w0, ws, dpk + ra, dpk + rb,
-                                                                 S + (size_t)ib * K.rows + ra, S + (size_t)ia * K.rows + rb, H, X, xs, F);
-  };
-  using I4 = std::integral_constant<int, 4>;
-  using I1 = std::integral_constant<int, 1>;
-  for (int t = tid; t < K.nhh; t += kThreads) run(I4{}, I4{}, t);
+  const int mu = tid & 3;
+#pragma unroll 1
+  for (int t0 = 0; t0 < 4 * K.nhh; t0 += kThreads) {
+    const int t = (t0 + tid) >> 2;
+    const bool on = t < K.nhh;
+    int ia, ib;
+    pair_uv_short(K.nh, on ? t : 0, ia, ib);
+    en += heavy_item<kJ>(on, n, soff[order[ia]], soff[order[ib]], mu, W + (on ? t : 0), K.nhh, dpk + 10 * ia, dpk + 10 * ib,
+                         S + ib * K.rows + 10 * ia, S + ia * K.rows + 10 * ib, H, X, xs, F);
+  }
   // the other kinds from the last thread on: the warps that had one heavy pair less begin first
-  for (int t = kThreads - 1 - tid; t < K.nhl; t += kThreads) run(I4{}, I1{}, K.nhh + t);
-  for (int t = kThreads - 1 - tid; t < K.nll; t += kThreads) run(I1{}, I1{}, K.nhh + K.nhl + t);
+  const double* Wl = W + (size_t)100 * K.nhh;
+#pragma unroll 1
+  for (int t = kThreads - 1 - tid; t < K.nhl; t += kThreads) {
+    const int ia = t / K.nl, ib = K.nh + t - ia * K.nl, rb = K.row(ib);
+    en += light_item<4, kJ>(n, soff[order[ia]], soff[order[ib]], Wl + t, K.nhl, dpk + 10 * ia, dpk[rb], S + ib * K.rows + 10 * ia,
+                            S + ia * K.rows + rb, H, X, xs, F);
+  }
+  Wl += (size_t)10 * K.nhl;
+#pragma unroll 1
+  for (int t = kThreads - 1 - tid; t < K.nll; t += kThreads) {
+    int ia, ib;
+    pair_uv_short(K.nl, t, ia, ib);
+    ia += K.nh;
+    ib += K.nh;
+    const int ra = K.row(ia), rb = K.row(ib);
+    en += light_item<1, kJ>(n, soff[order[ia]], soff[order[ib]], Wl + t, K.nll, dpk + ra, dpk[rb], S + ib * K.rows + ra,
+                            S + ia * K.rows + rb, H, X, xs, F);
+  }
   return en;
 }
 
