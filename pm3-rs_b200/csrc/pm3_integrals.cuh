@@ -1,6 +1,6 @@
 // Two-centre NDDO quantities of one atom pair, for device (and host) code, templated on the
-// scalar: `double` for energies, `D3` (value + three partials along the displacement) for the
-// analytic gradient.
+// scalar: `double` for energies, `D1` (value + derivative along the pair's axis) for the analytic
+// gradient.
 //
 // Physics follows pm3-rs (which follows MOPAC):
 //   - frame rotation onto the pair axis:        src/integrals.rs:25-59
@@ -24,28 +24,26 @@
 namespace pm3gpu {
 
 // ------------------------------------------------------------------------------------ scalars
-struct D3 {
-  double v, g[3];
+struct D1 {
+  double v, g;
 };
 PM3_HD double vof(double x) { return x; }
-PM3_HD double vof(const D3& x) { return x.v; }
+PM3_HD double vof(const D1& x) { return x.v; }
 template <class S> PM3_HD S mk(double x);
 template <> PM3_HD double mk<double>(double x) { return x; }
-template <> PM3_HD D3 mk<D3>(double x) { return D3{x, {0.0, 0.0, 0.0}}; }
+template <> PM3_HD D1 mk<D1>(double x) { return D1{x, 0.0}; }
 
-PM3_HD D3 operator+(const D3& a, const D3& b) { return {a.v + b.v, {a.g[0] + b.g[0], a.g[1] + b.g[1], a.g[2] + b.g[2]}}; }
-PM3_HD D3 operator-(const D3& a, const D3& b) { return {a.v - b.v, {a.g[0] - b.g[0], a.g[1] - b.g[1], a.g[2] - b.g[2]}}; }
-PM3_HD D3 operator-(const D3& a) { return {-a.v, {-a.g[0], -a.g[1], -a.g[2]}}; }
-PM3_HD D3 operator*(const D3& a, const D3& b) {
-  return {a.v * b.v, {a.g[0] * b.v + a.v * b.g[0], a.g[1] * b.v + a.v * b.g[1], a.g[2] * b.v + a.v * b.g[2]}};
-}
-PM3_HD D3 operator+(const D3& a, double b) { return {a.v + b, {a.g[0], a.g[1], a.g[2]}}; }
-PM3_HD D3 operator+(double b, const D3& a) { return {a.v + b, {a.g[0], a.g[1], a.g[2]}}; }
-PM3_HD D3 operator-(const D3& a, double b) { return {a.v - b, {a.g[0], a.g[1], a.g[2]}}; }
-PM3_HD D3 operator-(double b, const D3& a) { return {b - a.v, {-a.g[0], -a.g[1], -a.g[2]}}; }
-PM3_HD D3 operator*(const D3& a, double b) { return {a.v * b, {a.g[0] * b, a.g[1] * b, a.g[2] * b}}; }
-PM3_HD D3 operator*(double b, const D3& a) { return a * b; }
-PM3_HD D3 lift(const D3& a, double f, double df) { return {f, {a.g[0] * df, a.g[1] * df, a.g[2] * df}}; }
+PM3_HD D1 operator+(const D1& a, const D1& b) { return {a.v + b.v, a.g + b.g}; }
+PM3_HD D1 operator-(const D1& a, const D1& b) { return {a.v - b.v, a.g - b.g}; }
+PM3_HD D1 operator-(const D1& a) { return {-a.v, -a.g}; }
+PM3_HD D1 operator*(const D1& a, const D1& b) { return {a.v * b.v, a.g * b.v + a.v * b.g}; }
+PM3_HD D1 operator+(const D1& a, double b) { return {a.v + b, a.g}; }
+PM3_HD D1 operator+(double b, const D1& a) { return {a.v + b, a.g}; }
+PM3_HD D1 operator-(const D1& a, double b) { return {a.v - b, a.g}; }
+PM3_HD D1 operator-(double b, const D1& a) { return {b - a.v, -a.g}; }
+PM3_HD D1 operator*(const D1& a, double b) { return {a.v * b, a.g * b}; }
+PM3_HD D1 operator*(double b, const D1& a) { return a * b; }
+PM3_HD D1 lift(const D1& a, double f, double df) { return {f, a.g * df}; }
 
 // 1/sqrt(x)
 PM3_HD double rsq(double x) {
@@ -55,22 +53,22 @@ PM3_HD double rsq(double x) {
   return 1.0 / std::sqrt(x);
 #endif
 }
-PM3_HD D3 rsq(const D3& x) { double r = rsq(x.v); return lift(x, r, -0.5 * r * r * r); }
+PM3_HD D1 rsq(const D1& x) { double r = rsq(x.v); return lift(x, r, -0.5 * r * r * r); }
 PM3_HD double sq_rt(double x) { return sqrt(x); }
-PM3_HD D3 sq_rt(const D3& x) { double s = sqrt(x.v); return lift(x, s, 0.5 / s); }
+PM3_HD D1 sq_rt(const D1& x) { double s = sqrt(x.v); return lift(x, s, 0.5 / s); }
 PM3_HD double inv(double x) { return 1.0 / x; }
-PM3_HD D3 inv(const D3& x) { double r = 1.0 / x.v; return lift(x, r, -r * r); }
+PM3_HD D1 inv(const D1& x) { double r = 1.0 / x.v; return lift(x, r, -r * r); }
 PM3_HD double ex(double x) { return exp(x); }
-PM3_HD D3 ex(const D3& x) { double e = exp(x.v); return lift(x, e, e); }
+PM3_HD D1 ex(const D1& x) { double e = exp(x.v); return lift(x, e, e); }
 PM3_HD double pw(double x, double p) { return pow(x, p); }
-PM3_HD D3 pw(const D3& x, double p) { double f = pow(x.v, p); return lift(x, f, p * pow(x.v, p - 1.0)); }
+PM3_HD D1 pw(const D1& x, double p) { double f = pow(x.v, p); return lift(x, f, p * pow(x.v, p - 1.0)); }
 template <class S> PM3_HD S ipow(S x, int n) {
   S r = x;
   for (int i = 1; i < n; ++i) r = r * x;
   return r;
 }
 PM3_HD double ab(double x) { return fabs(x); }
-PM3_HD D3 ab(const D3& x) { return x.v < 0.0 ? -x : x; }
+PM3_HD D1 ab(const D1& x) { return x.v < 0.0 ? -x : x; }
 
 PM3_HD int pk(int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
 
@@ -270,6 +268,25 @@ template <class S> PM3_HD void aux_a(const S& x, S a[7], int kmax) {
   a[0] = ex(-x) * ix;
   for (int i = 1; i <= kmax; ++i) a[i] = a[0] + a[i - 1] * ix * (double)i;
 }
+#if defined(__CUDACC__)
+#define PM3_X(j) 2.0 / j
+__constant__ double kTwoOver[48] = {
+    0.0,       PM3_X(1),  PM3_X(2),  PM3_X(3),  PM3_X(4),  PM3_X(5),  PM3_X(6),  PM3_X(7),  PM3_X(8),  PM3_X(9),  PM3_X(10), PM3_X(11),
+    PM3_X(12), PM3_X(13), PM3_X(14), PM3_X(15), PM3_X(16), PM3_X(17), PM3_X(18), PM3_X(19), PM3_X(20), PM3_X(21), PM3_X(22), PM3_X(23),
+    PM3_X(24), PM3_X(25), PM3_X(26), PM3_X(27), PM3_X(28), PM3_X(29), PM3_X(30), PM3_X(31), PM3_X(32), PM3_X(33), PM3_X(34), PM3_X(35),
+    PM3_X(36), PM3_X(37), PM3_X(38), PM3_X(39), PM3_X(40), PM3_X(41), PM3_X(42), PM3_X(43), PM3_X(44), PM3_X(45), PM3_X(46), PM3_X(47)};
+#undef PM3_X
+#endif
+// 2 / j, 1 <= j < 48: read, not divided (the divisions were most of an overlap's time)
+PM3_HD double two_over(int j) {
+#if defined(__CUDA_ARCH__)
+  return kTwoOver[j];
+#else
+  return 2.0 / (double)j;
+#endif
+}
+PM3_HD bool differ(double a, double b) { return a != b; }
+PM3_HD bool differ(const D1& a, const D1& b) { return a.v != b.v || a.g != b.g; }
 template <class S> PM3_HD void aux_b(const S& x, S b[7], int kmax) {
   if (fabs(vof(x)) > 3.0) {
     const S ix = inv(x);
@@ -278,12 +295,23 @@ template <class S> PM3_HD void aux_b(const S& x, S b[7], int kmax) {
     b[0] = ep + em;
     for (int i = 1; i <= kmax; ++i) b[i] = ep * ((i & 1) ? -1.0 : 1.0) + em + b[i - 1] * ix * (double)i;
   } else {
-    // B_k(x) = 2 sum_{m: k+m even} (-x)^m / (m! (k+m+1)), absolutely convergent
+    // B_k(x) = 2 sum_{m: k+m even} (-x)^m / (m! (k+m+1)), absolutely convergent. From m = 4 on each term is less than half of
+    // the last of its parity, so two terms in a row that change nothing end the sum with the value of all 40.
     for (int i = 0; i <= kmax; ++i) b[i] = mk<S>(0.0);
     S term = mk<S>(1.0);
+    bool last = true;
     for (int m = 0; m < 40; ++m) {
-      for (int k = (m & 1); k <= kmax; k += 2) b[k] = b[k] + term * (2.0 / (double)(k + m + 1));
-      term = term * (-x) * (1.0 / (double)(m + 1));
+      bool changed = false;
+#pragma unroll
+      for (int k = 0; k < 7; ++k) {
+        if (k > kmax || ((k ^ m) & 1)) continue;
+        const S next = b[k] + term * two_over(k + m + 1);
+        changed = changed || differ(next, b[k]);
+        b[k] = next;
+      }
+      if (m > 4 && !changed && !last) break;
+      last = changed;
+      term = term * (-x) * (0.5 * two_over(m + 1));
     }
   }
 }

@@ -711,18 +711,32 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
   return PM3GPU_OK;
 }
 
+// First AO of each atom, and the atoms with those that have p orbitals first; returns how many those are.
+int gradient_order(const pm3gpu_ctx* c, const int32_t* z, int natom, int32_t* ao_off, int32_t* order) {
+  int off = 0, nh = 0;
+  for (int a = 0; a < natom; ++a) {
+    ao_off[a] = off;
+    off += c->h_elem[z[a]].norb;
+    if (c->h_elem[z[a]].norb == 4) order[nh++] = a;
+  }
+  for (int a = 0, k = nh; a < natom; ++a)
+    if (c->h_elem[z[a]].norb != 4) order[k++] = a;
+  return nh;
+}
+
 // Gradients of the selected states of `mols` (one thread per atom pair of the whole batch).
-int launch_gradients(pm3gpu_ctx* c, const std::vector<GradMol>& mols, const std::vector<int32_t>& ao_off,
+// `ao_order`: the atoms' first AOs, then per molecule its atoms with those that have p orbitals first.
+int launch_gradients(pm3gpu_ctx* c, const std::vector<GradMol>& mols, const std::vector<int32_t>& ao_order,
                      const int32_t* d_z, const double* d_xyz, size_t total_atoms, std::vector<double>& grads,
                      const double* dens = nullptr) {
   grads.assign(3 * total_atoms, 0.0);
   if (mols.empty()) return PM3GPU_OK;
   long long npairs = mols.back().pair0 + (long long)mols.back().natom * (mols.back().natom - 1) / 2;
   CUDA_TRY(c, c->gmols.ensure(sizeof(GradMol) * mols.size()));
-  CUDA_TRY(c, c->aooff.ensure(4 * std::max<size_t>(ao_off.size(), 1)));
+  CUDA_TRY(c, c->aooff.ensure(4 * std::max<size_t>(ao_order.size(), 1)));
   CUDA_TRY(c, c->grads.ensure(24 * std::max<size_t>(total_atoms, 1)));
   CUDA_TRY(c, cudaMemcpyAsync(c->gmols.p, mols.data(), sizeof(GradMol) * mols.size(), cudaMemcpyHostToDevice, c->stream));
-  CUDA_TRY(c, cudaMemcpyAsync(c->aooff.p, ao_off.data(), 4 * ao_off.size(), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(c->aooff.p, ao_order.data(), 4 * ao_order.size(), cudaMemcpyHostToDevice, c->stream));
   CUDA_TRY(c, cudaMemsetAsync(c->grads.p, 0, 24 * total_atoms, c->stream));
   if (npairs > 0) {
     GradArgs g{};
@@ -731,19 +745,20 @@ int launch_gradients(pm3gpu_ctx* c, const std::vector<GradMol>& mols, const std:
     g.z = d_z;
     g.xyz = d_xyz;
     g.ao_off = c->aooff.as<int>();
+    g.order = g.ao_off + total_atoms;
     g.mols = c->gmols.as<GradMol>();
     g.nmol = (int)mols.size();
     g.npairs = npairs;
     g.dens = dens ? dens : c->dens.as<double>();
     g.grad = c->grads.as<double>();
-    const long long blocks = std::min<long long>((npairs + 127) / 128, (long long)c->sms * 16);
-    gradient_kernel<<<(unsigned)blocks, 128, 0, c->stream>>>(g);
+    const long long blocks = std::min<long long>((npairs + kGradThreads - 1) / kGradThreads, (long long)c->sms * 32);
+    gradient_kernel<<<(unsigned)blocks, kGradThreads, 0, c->stream>>>(g);
     c->launches += 1;
     CUDA_TRY(c, cudaGetLastError());
   }
   CUDA_TRY(c, cudaMemcpyAsync(grads.data(), c->grads.p, 24 * total_atoms, cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  c->h2d += (long long)(sizeof(GradMol) * mols.size() + 4 * ao_off.size());
+  c->h2d += (long long)(sizeof(GradMol) * mols.size() + 4 * ao_order.size());
   c->d2h += (long long)(24 * total_atoms);
   return PM3GPU_OK;
 }
@@ -875,12 +890,9 @@ int run_large(pm3gpu_ctx* c, const MolPlan& p, const int32_t* hz, const int32_t*
     std::memcpy(mo_energies, all.data(), 8 * (size_t)p.nao);
   }
   if (want.grad && gradient && so.converged) {
-    std::vector<int32_t> ao_off(p.natom);
-    for (int a = 0, off = 0; a < p.natom; ++a) {
-      ao_off[a] = off;
-      off += c->h_elem[hz[a]].norb;
-    }
+    std::vector<int32_t> ao_order(2 * (size_t)p.natom);
     GradMol g{};
+    g.nh = gradient_order(c, hz, p.natom, ao_order.data(), ao_order.data() + p.natom);
     g.atom0 = 0;
     g.natom = p.natom;
     g.nao = p.nao;
@@ -889,7 +901,7 @@ int run_large(pm3gpu_ctx* c, const MolPlan& p, const int32_t* hz, const int32_t*
     g.pair0 = 0;
     g.dens_off = 0;
     std::vector<double> gr;
-    rc = launch_gradients(c, {g}, ao_off, dz, dxyz, (size_t)p.natom, gr, c->lsel.as<double>());
+    rc = launch_gradients(c, {g}, ao_order, dz, dxyz, (size_t)p.natom, gr, c->lsel.as<double>());
     if (rc != PM3GPU_OK) return rc;
     std::memcpy(gradient, gr.data(), 24 * (size_t)p.natom);
   }
@@ -1330,17 +1342,13 @@ int run_batch(pm3gpu_ctx* c, int n_mol, const int32_t* h_offs, const int32_t* h_
   // ---------------------------------------------------------------- analytic gradients
   if (want.grad && gradients) {
     std::vector<GradMol> gm;
-    std::vector<int32_t> ao_off(total_atoms, 0);
+    std::vector<int32_t> ao_order(2 * (size_t)total_atoms, 0);
     long long pair0 = 0;
     for (int m = 0; m < n_mol; ++m) {
       const MolPlan& p = plans[m];
       if (p.status != PM3GPU_OK || p.large || !chosen[m].o.converged) continue;
-      int off = 0;
-      for (int a = 0; a < p.natom; ++a) {
-        ao_off[p.atom0 + a] = off;
-        off += c->h_elem[h_z[p.atom0 + a]].norb;
-      }
       GradMol g{};
+      g.nh = gradient_order(c, h_z + p.atom0, p.natom, ao_order.data() + p.atom0, ao_order.data() + total_atoms + p.atom0);
       g.atom0 = p.atom0;
       g.natom = p.natom;
       g.nao = p.nao;
@@ -1353,7 +1361,7 @@ int run_batch(pm3gpu_ctx* c, int n_mol, const int32_t* h_offs, const int32_t* h_
       gm.push_back(g);
     }
     std::vector<double> gr;
-    rc = launch_gradients(c, gm, ao_off, dz, dxyz, (size_t)total_atoms, gr);
+    rc = launch_gradients(c, gm, ao_order, dz, dxyz, (size_t)total_atoms, gr);
     if (rc != PM3GPU_OK) return rc;
     for (int m = 0; m < n_mol; ++m) {
       const MolPlan& p = plans[m];

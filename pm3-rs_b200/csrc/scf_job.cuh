@@ -487,7 +487,6 @@ __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
   c.n = J.nao;
   c.N = J.natom;
   const int n = c.n, nb = J.n_beta;
-  const size_t nn = (size_t)n * n;
   setup_job(c);
   double* own_vb = c.Vb;
   double* own_vt = c.Vt;
