@@ -618,15 +618,15 @@ __device__ __forceinline__ double pow2(int ex) {  // 2^ex for normal results, 0 
 template <int M>
 __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const double* __restrict__ e2, int n,
                                             const double (&x)[M], int (&cnt)[M], double (&val)[M], int (&ex)[M]) {
-  constexpr double kBig = 0x1p256, kSmall = 0x1p-256;
+  constexpr int kOne = 1023 << 20, kBig = (1023 + 256) << 20, kSmall = (1023 - 256) << 20;  // upper halves of 1, 2^256, 2^-256
   double p[M], pm[M];
-  unsigned sg[M];
+  unsigned sg[M];  // sign bits, the newest last
 #pragma unroll
   for (int t = 0; t < M; ++t) {
     pm[t] = 1.0;
     ex[t] = 0;
     p[t] = d[0] - x[t];
-    sg[t] = __double_as_longlong(p[t]) < 0 ? 1u : 0u;
+    sg[t] = (unsigned)__double2hiint(p[t]) >> 31;
     cnt[t] = (int)sg[t];
   }
   int i = 1;
@@ -637,34 +637,35 @@ __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const 
 #pragma unroll
       for (int t = 0; t < M; ++t) {
         const double pn = fma(di - x[t], p[t], -ei * pm[t]);
-        const unsigned s = __double_as_longlong(pn) < 0 ? 1u : 0u;
-        cnt[t] += (int)(s ^ sg[t]);
-        sg[t] = s;
+        sg[t] = __funnelshift_l((unsigned)__double2hiint(pn), sg[t], 1);
         pm[t] = p[t];
         p[t] = pn;
       }
     }
 #pragma unroll
     for (int t = 0; t < M; ++t) {
-      const double m = fmax(fabs(p[t]), fabs(pm[t]));
-      const double sc = m > kBig ? kSmall : (m < kSmall ? kBig : 1.0);
-      ex[t] += m > kBig ? 1 : (m < kSmall ? -1 : 0);
+      cnt[t] += __popc((sg[t] ^ (sg[t] >> 1)) & 0xffu);
+      const int m = max(__double2hiint(p[t]) & 0x7fffffff, __double2hiint(pm[t]) & 0x7fffffff);  // the larger magnitude's upper half
+      const int up = m > kBig ? 1 : (m < kSmall ? -1 : 0);
+      const double sc = __hiloint2double(kOne - up * (256 << 20), 0);
+      ex[t] += up;
       p[t] *= sc;
       pm[t] *= sc;
     }
   }
+  const unsigned left = (1u << (n - i)) - 1u;
   for (; i < n; ++i) {
     const double di = d[i], ei = e2[i - 1];
 #pragma unroll
     for (int t = 0; t < M; ++t) {
       const double pn = fma(di - x[t], p[t], -ei * pm[t]);
-      const unsigned s = __double_as_longlong(pn) < 0 ? 1u : 0u;
-      cnt[t] += (int)(s ^ sg[t]);
-      sg[t] = s;
+      sg[t] = __funnelshift_l((unsigned)__double2hiint(pn), sg[t], 1);
       pm[t] = p[t];
       p[t] = pn;
     }
   }
+#pragma unroll
+  for (int t = 0; t < M; ++t) cnt[t] += __popc((sg[t] ^ (sg[t] >> 1)) & left);
 #pragma unroll
   for (int t = 0; t < M; ++t) val[t] = p[t];
 }
@@ -676,7 +677,7 @@ __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const 
 // secant estimate of the characteristic polynomial's root, whose values the counts yield on the way; the counts
 // still decide, and a step that gained less than a factor of 4 is followed by an even one.
 // What bounds it: the recurrence, about 40 cycles a row and step; steps from a cold start at n = 64, k = 33:
-// 17 when all were even.
+// 17 when all were even, 9 now.
 // With `prev` (eigenvalue j of the previous SCF iteration) and `dprev` (its last change) the search starts from a
 // bracket around prev[j] once two counts confirm it. Whole warps call; lanes without an eigenvalue pass
 // active = false.

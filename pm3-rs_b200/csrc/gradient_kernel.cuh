@@ -190,7 +190,7 @@ __device__ __noinline__ void pair_force(const ElemDev& ea, const ElemDev& eb, co
     if (blk == 0) {  // P_ab (beta_i + beta_j) S_ab, both off-diagonal blocks
       const bool swap = ea.npq < eb.npq;
       D1 o[5];
-      if (overlap_local(swap ? eb : ea, swap ? ea : eb, r, o)) {
+      if (dist >= 1.0e-8 && overlap_local(swap ? eb : ea, swap ? ea : eb, r, o)) {  // constant below, as in overlap_block
         const double ss = ea.bs + eb.bs, ps = ea.bp + eb.bs, sp = ea.bs + eb.bp, p2 = ea.bp + eb.bp;
         A[0][0] = ss * o[0].v;
         de = fma(ss * o[0].g, X[0][0], de);

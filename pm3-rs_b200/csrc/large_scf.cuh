@@ -693,8 +693,9 @@ __global__ void __launch_bounds__(kBlock) block_v_kernel(const double* A, int n,
 // T (kWy x kWy, row-major, upper triangular) of H(p) ... H(p+b-1) = I - V T V^T from the Gram
 // G = V^T V (b x b) and tau: T[k][k] = tau_k, T[m][k] = -tau_k sum_{m <= l < k} T[m][l] G[l][k]. The 16 x 16 diagonal
 // blocks are formed row by row (a row depends only on its own earlier entries), then neighbours are
-// joined three times, [T1, -T1 G12 T2; 0, T2], by products in shared memory. One CTA; forming whole rows of 128 one
-// thread each took most of the back-transformation (3.6 of 3.7 ms at n = 966, against 0.6).
+// joined three times, [T1, -T1 G12 T2; 0, T2], by products in shared memory. One CTA, bound by the latency of the
+// 16 x 16 chains and the joins: 46 us a factor at n = 966; with whole rows of 128 formed one thread each the
+// back-transformation of an iteration took 3.6 ms, 2.0 with this.
 constexpr int kTld = kWy + 1;
 constexpr int kTGs = 64 * 65;  // G12 of a level, all pairs: at most 64 (s + 1)
 constexpr int kTSmem = (kWy * kTld + 2 * kTGs) * 8;

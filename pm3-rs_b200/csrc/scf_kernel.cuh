@@ -649,7 +649,8 @@ __device__ __noinline__ double build_fock(Ctx& c, const double* Pt, const double
 }
 
 // The lower triangle of E = F P - P F (scf.rs:1039-1054), which is antisymmetric: nothing reads the other half. The
-// transposed subtraction of a full product F P cost as much as the product (n = 148: 550k cycles before, 150k now).
+// transposed subtraction of a full product F P cost as much as the product (n = 148: 550k cycles before, 180k now, FP64
+// issue).
 __device__ __noinline__ void commutator(Ctx& c, const double* Fm, const double* Pm, double* E) {
   const int n = c.n;
   lower_product<true>(n, n, Fm, Pm, in_shared(c.tile),
