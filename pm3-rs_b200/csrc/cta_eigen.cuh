@@ -1289,9 +1289,10 @@ __device__ __forceinline__ void back_transform_t(int n, int kvec, const double* 
 }
 
 // Split by size: the n x kvec block of vectors is spread over the CTA's registers, in as few passes as
-// they allow. Shared scratch: 16 rows of G RT doubles.
+// they allow. Beyond 160 the rows a lane holds follow n (12, 14, 16), since two vectors and a reflector of 16 rows no longer fit the
+// registers: a molecule of n = 168 takes 13.0 ms against 14.1 with 16 rows, n = 222 29.0 against 30.1. Shared scratch: 16 rows of G RT doubles.
 __host__ __device__ constexpr int back_scratch(int n) {
-  return 16 * (n <= 32 ? 32 : n <= 64 ? 64 : n <= 96 ? 96 : n <= 128 ? 128 : n <= 160 ? 160 : 256);
+  return 16 * (n <= 32 ? 32 : n <= 64 ? 64 : n <= 96 ? 96 : n <= 128 ? 128 : n <= 160 ? 160 : n <= 192 ? 192 : n <= 224 ? 224 : 256);
 }
 __device__ __noinline__ void back_transform(int n, int kvec, const double* __restrict__ V, const double* __restrict__ Yt,
                                             double* Y, const EigenScratch& s_) {
@@ -1304,6 +1305,8 @@ __device__ __noinline__ void back_transform(int n, int kvec, const double* __res
   else if (n <= 128 && kvec > 64) back_transform_t<16, 8, 4>(n, kvec, V, Yt, Y, tau, sh);
   else if (n <= 128) back_transform_t<8, 16, 2>(n, kvec, V, Yt, Y, tau, sh);
   else if (n <= 160) back_transform_t<16, 10, 3>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 192) back_transform_t<16, 12, 2>(n, kvec, V, Yt, Y, tau, sh);
+  else if (n <= 224) back_transform_t<16, 14, 2>(n, kvec, V, Yt, Y, tau, sh);
   else back_transform_t<16, 16, 2>(n, kvec, V, Yt, Y, tau, sh);
 }
 

@@ -20,8 +20,10 @@ HOF_TOL = 1e-6
 Q_TOL = 1e-5
 GRAD_TOL = 1e-6 * 0.0433641043 / 1.8897261246
 D = ctypes.POINTER(ctypes.c_double)
-UNITS = {"w": ([8, 1, 1], [[0.0, 0.0, 0.0], [0.957, 0.0, 0.0], [-0.24, 0.927, 0.0]]), "h": ([1, 1], [[0.0, 0.0, 0.0], [0.74, 0.0, 0.0]]),
-         "n": ([7, 7], [[0.0, 0.0, 0.0], [1.1, 0.0, 0.0]]), "r": ([6, 1, 1, 1], [[0.0, 0.0, 0.05], [1.12, 0.0, 0.0], [-0.55, 0.95, 0.0], [-0.55, -0.95, 0.0]])}
+UNITS = {"w": ([8, 1, 1], [[0.0, 0.0, 0.0], [0.957, 0.0, 0.0], [-0.24, 0.927, 0.0]]),
+         "h": ([1, 1], [[0.0, 0.0, 0.0], [0.74, 0.0, 0.0]]),
+         "n": ([7, 7], [[0.0, 0.0, 0.0], [1.1, 0.0, 0.0]]),
+         "r": ([6, 1, 1, 1], [[0.0, 0.0, 0.05], [1.12, 0.0, 0.0], [-0.55, 0.95, 0.0], [-0.55, -0.95, 0.0]])}
 
 
 def cluster(w=0, h=0, n=0, r=0, seed=0):
@@ -61,7 +63,8 @@ def _close(got, ref):
 
 @pytest.mark.parametrize("unit", [
     dict(h=1), dict(w=2, h=2), dict(w=3), dict(w=5, h=1), dict(w=18, h=2), dict(w=19), dict(w=21, h=1), dict(w=21, h=2), dict(w=26, h=2),
-    dict(w=27), dict(w=29, h=1), dict(w=42, h=2), dict(h=9), dict(h=57), dict(n=2), dict(n=14), dict(n=8, h=25)])
+    dict(w=27), dict(w=29, h=1), dict(w=32), dict(w=32, h=1), dict(w=37, h=1), dict(w=37, h=2), dict(w=42, h=2),
+    dict(h=9), dict(h=57), dict(n=2), dict(n=14), dict(n=8, h=25)])
 def test_per_cta_sizes_match_oracle(ctx, unit):
     z, xyz = cluster(**unit)
     opts = dict(p_tol=1e-8)
