@@ -8,8 +8,9 @@
 // integrals out of it. Along the axis the integrals change: dual numbers in the distance. Across it only the frame turns:
 // with A = dE/dP the derivative by the turning angle is <A, [G, P]>, G mixing sigma with one pi. (The energy does not change when
 // the frame turns about the axis.) With every integral a dual number of three partials in the molecular frame a heavy pair was
-// 100 rotations of four-fold products: 1000 organics of 10-35 atoms took 3.01 ms (pairs by kind included), 0.66 now, 24 atoms
-// 0.22 of 3.9 ms of a call, 0.11 now. Bound by the latency of one thread's chain and by its registers (a heavy pair holds some 100 doubles).
+// 100 rotations of four-fold products: 1000 organics of 10-35 atoms took 3.01 ms (pairs by kind included), 0.47 now, 24 atoms
+// 0.22 of 3.9 ms of a call, 0.11 now. Bound by instruction
+// fetch (half of the cycles between a warp's instructions: a heavy pair is one long straight run of code) and one thread's chain.
 #pragma once
 #include "pm3_integrals.cuh"
 

@@ -316,6 +316,20 @@ template <class S> PM3_HD void aux_b(const S& x, S b[7], int kmax) {
   }
 }
 
+// Both for the scaled distances x and y. The differentiated form is one function called in turn: a pair's gradient waits for
+// instruction fetch, and its copies in line cost 0.66 ms against 0.47 (1000 organics of 10-35 atoms).
+PM3_HD void aux_ab(double x, double y, double a[7], double b[7], int kmax) {
+  aux_a(x, a, kmax);
+  aux_b(y, b, kmax);
+}
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__
+#endif
+inline void aux_ab(const D1& x, const D1& y, D1 a[7], D1 b[7], int kmax) {
+  aux_a(x, a, kmax);
+  aux_b(y, b, kmax);
+}
+
 // Local overlaps (s s sigma, p_a s sigma, s p_b sigma, p p sigma, p p pi) for ea the atom with
 // the larger principal quantum number. Returns false when no closed form exists.
 template <class S> PM3_HD bool overlap_local(const ElemDev& ea, const ElemDev& eb, const S& r, S o[5]) {
@@ -338,16 +352,14 @@ template <class S> PM3_HD bool overlap_local(const ElemDev& ea, const ElemDev& e
   if (lo < 1.0e300 && vof(r) * (0.5 * lo) > 300.0) return true;
   const int km = (na + nb + 1 < 6) ? na + nb + 1 : 6;
   S a11[7], b11[7];
-  aux_a(r * (0.5 * (za0 + zb0)), a11, km);
-  aux_b(r * (0.5 * (za0 - zb0)), b11, km);
+  aux_ab(r * (0.5 * (za0 + zb0)), r * (0.5 * (za0 - zb0)), a11, b11, km);
   const double s3 = sqrt(3.0);
   if (j == 11) {
     o[0] = pw(r * r * (za0 * zb0), 1.5) * (a11[2] * b11[0] - b11[2] * a11[0]) * 0.25;
     return true;
   }
   S a21[7], b21[7];
-  aux_a(r * (0.5 * (za1 + zb0)), a21, km);
-  aux_b(r * (0.5 * (za1 - zb0)), b21, km);
+  aux_ab(r * (0.5 * (za1 + zb0)), r * (0.5 * (za1 - zb0)), a21, b21, km);
   if (j == 21) {
     const S r4 = ipow(r, 4);
     o[0] = r4 * (pow(zb0, 1.5) * pow(za0, 2.5)) * (a11[3] * b11[0] - b11[3] * a11[0] + a11[2] * b11[1] - b11[2] * a11[1]) * (1.0 / (s3 * 8.0));
@@ -364,10 +376,8 @@ template <class S> PM3_HD bool overlap_local(const ElemDev& ea, const ElemDev& e
     return true;
   }
   S a12[7], b12[7], a22[7], b22[7];
-  aux_a(r * (0.5 * (za0 + zb1)), a12, km);
-  aux_b(r * (0.5 * (za0 - zb1)), b12, km);
-  aux_a(r * (0.5 * (za1 + zb1)), a22, km);
-  aux_b(r * (0.5 * (za1 - zb1)), b22, km);
+  aux_ab(r * (0.5 * (za0 + zb1)), r * (0.5 * (za0 - zb1)), a12, b12, km);
+  aux_ab(r * (0.5 * (za1 + zb1)), r * (0.5 * (za1 - zb1)), a22, b22, km);
   if (j == 22) {
     const S r5 = ipow(r, 5);
     o[0] = r5 * pow(zb0 * za0, 2.5) * (a11[4] * b11[0] + b11[4] * a11[0] - a11[2] * b11[2] * 2.0) * (1.0 / 48.0);
