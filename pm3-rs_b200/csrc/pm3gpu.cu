@@ -396,6 +396,13 @@ void plan_molecule(const pm3gpu_ctx* c, const int32_t* z, const double* xyz, int
   m.steered = o->level_shift_ev != 0.0 || o->damping != 0.0;
 }
 
+// Whether a solve asks for what the reference tightens second derivatives to (hessian.rs:169-175). Its result is one end of a
+// difference, so it runs on the sums of scf_tight.cuh (there: why, and what it costs).
+template <class T>
+bool second_derivative_tolerances(const T& o) {
+  return o.e_tol <= 1.0e-12 && o.p_tol <= 1.0e-11 && o.max_scf >= 500;
+}
+
 // run_scf of run_pm3 (scf.rs:531-555) as a job: resolve the accelerator the loop will use.
 JobDesc make_job(const MolPlan& m, int guess, int accel, double shift, double damp, bool force_uhf, int extra_flags) {
   const pm3gpu_options& o = *m.o;
@@ -496,20 +503,21 @@ int g_scf_static_smem = 1024;
 // ctas: 0 = choose (two CTAs per SM when at least 90% of the batch keeps its packed eigen input
 // in the smaller layout), 1 or 2 = the autotuner's measured choice.
 // wcap: doubles of the launch's largest pair table; the union is widened to hold it when two CTAs per SM allow.
+// tight: the layout of scf_tight_kernel, which holds the packed matrix itself.
 SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const std::vector<int>* naos = nullptr,
-                       int ctas = 0, long long wcap = 0) {
+                       int ctas = 0, long long wcap = 0, bool tight = false) {
   SmemLayout L{};
   L.amax = amax;
   auto align = [](int b) { return (b + 15) & ~15; };
   int off = 0;
   L.off_int = off;
-  off += align((3 * amax + 1 + 16) * 4);
+  off += align(((tight ? 4 : 3) * amax + 1 + 16) * 4);
   L.off_dbl = off;
   off += align(((3 * amax + 1) / 2 * 2 + 4 * kMaxDepth * kWarps + 4 * kMaxDepth + 2 * kMaxDepth * kMaxDepth + kMaxDepth + 8) * 8);
   L.off_eig = off;
   off += align(7 * nmax * 8 + (2 * nmax + 2) * 4);
   L.off_union = off;
-  const int fixed_union = union_keep(nmax);
+  const int fixed_union = tight ? std::max(20 * amax, tight::kGemmScratch) : union_keep(nmax);
   auto fit = [&](int budget) {
     int nsm = nmax;
     for (; nsm > 0; --nsm)
@@ -532,7 +540,7 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
   }
   L.nsm = nsm;
   L.uni = std::max(fixed_union, nsm * (nsm + 1) / 2);
-  if (smem_per_sm > 0 && wcap > 0) {
+  if (smem_per_sm > 0 && wcap > 0 && !tight) {
     const long long want = fixed_union + wcap;
     if (off + want * 8 <= smem_per_sm / 2 - 1024 - g_scf_static_smem) L.uni = std::max(L.uni, (int)want);
   }
@@ -592,9 +600,16 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
     }
   for (const JobDesc& j : jobs) naos.push_back(j.nao);
   const int ctas = c->force_ctas ? c->force_ctas : tune_lookup(c->tune_batch, nmax, 0);
-  const SmemLayout L = make_layout(amax, nmax, c->smem_optin, c->smem_per_sm, &naos, ctas, wcap);
+  // Launches of second-derivative solves alone; a launch that mixes them with others, or may hand a spin to a helper, is the common one.
+  bool tight = true;
+  for (const std::vector<JobDesc>* L : {&jobs, &rjobs})
+    for (const JobDesc& j : *L)
+      tight &= second_derivative_tolerances(j) && !(j.flags & (kJobCoreOnly | kJobFockOnly)) &&
+               !(c->tail_helpers && (j.flags & kJobUhf));
+  const SmemLayout L = make_layout(amax, nmax, c->smem_optin, c->smem_per_sm, &naos, ctas, wcap, tight);
+  const auto kernel = tight ? scf_tight_kernel : scf_batch_kernel;
   int per_sm = 0;
-  CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scf_batch_kernel, kThreads, L.bytes));
+  CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, L.bytes));
   if (per_sm < 1) return fail(c, PM3GPU_RESOURCE_LIMIT, "SCF kernel does not fit on an SM");
   c->last_ctas = per_sm;
   c->last_nsm = L.nsm;
@@ -657,7 +672,7 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
   a.wcap = wcap;
   a.queue = c->queue.as<int>();
   a.prof = nullptr;
-  a.help = c->tail_helpers ? c->help.as<HelpRec>() : nullptr;
+  a.help = c->tail_helpers && !tight ? c->help.as<HelpRec>() : nullptr;
   // With tail helpers, up to 32 idle CTAs stay for late stability rungs and unrestricted jobs to
   // help; otherwise idle CTAs exit and free their SM for the next batch in flight.
   a.max_waiters = c->tail_helpers ? 32 : 0;
@@ -669,7 +684,7 @@ int launch_jobs(pm3gpu_ctx* c, const std::vector<JobDesc>& jobs, const std::vect
   }
   a.sm = L;
   CUDA_TRY(c, cudaEventRecord(c->kev[0], c->stream));
-  scf_batch_kernel<<<(unsigned)grid, kThreads, L.bytes, c->stream>>>(a);
+  kernel<<<(unsigned)grid, kThreads, L.bytes, c->stream>>>(a);
   c->launches += 1;
   CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaEventRecord(c->kev[1], c->stream));
@@ -1174,7 +1189,8 @@ int run_batch(pm3gpu_ctx* c, int n_mol, const int32_t* h_offs, const int32_t* h_
     // they spread, over that kernel's whole range (n = 204: 23 against 45 ms; n = 252: 44 against 60). The whole-GPU
     // path still takes it where only that path has what was asked for.
     if (n_mol == 1 && !c->large_set && p.status == PM3GPU_OK && !p.large && p.nao >= kSingleWholeNao &&
-        o->guess != PM3GPU_GUESS_LEARNED && (c->precision == PM3GPU_PRECISION_MIXED || c->large_checks))
+        o->guess != PM3GPU_GUESS_LEARNED &&
+        (c->precision == PM3GPU_PRECISION_MIXED || c->large_checks || second_derivative_tolerances(*o)))
       p.large = true;
     if (p.status != PM3GPU_OK || p.large) continue;  // large molecules: whole-GPU path below
     JobDesc j = p.steered ? make_job(p, o->guess, o->accelerator, o->level_shift_ev, o->damping, false, 0)
@@ -1522,12 +1538,15 @@ int pm3gpu_context_create(int device, pm3gpu_ctx** out) {
   // asks for its own layout's bytes, which make_layout keeps within the same budget).
   cudaFuncAttributes fa{};
   if ((e = cudaFuncGetAttributes(&fa, scf_batch_kernel)) != cudaSuccess) return bail(e);
-  c->smem_optin = (int)prop.sharedMemPerBlockOptin - (int)fa.sharedSizeBytes;
-  g_scf_static_smem = std::max(512, (int)fa.sharedSizeBytes);
+  cudaFuncAttributes ft{};
+  if ((e = cudaFuncGetAttributes(&ft, scf_tight_kernel)) != cudaSuccess) return bail(e);
+  const int fixed = (int)std::max(fa.sharedSizeBytes, ft.sharedSizeBytes);
+  c->smem_optin = (int)prop.sharedMemPerBlockOptin - fixed;
+  g_scf_static_smem = std::max(512, fixed);
   c->smem_per_sm = (int)prop.sharedMemPerMultiprocessor;
-  if ((e = cudaFuncSetAttribute(scf_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin)) !=
-      cudaSuccess)
-    return bail(e);
+  for (const auto kernel : {scf_batch_kernel, scf_tight_kernel})
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin)) != cudaSuccess)
+      return bail(e);
   if ((e = cudaHostAlloc(reinterpret_cast<void**>(&c->h_gerr), sizeof(int), cudaHostAllocDefault)) != cudaSuccess)
     return bail(e);
   *c->h_gerr = 0;

@@ -3,6 +3,7 @@
 // (src/gradient.rs:306-599, src/repulsion.rs:30-49).
 #pragma once
 #include "scf_kernel.cuh"
+#include "scf_tight.cuh"
 
 namespace pm3gpu {
 
@@ -115,11 +116,39 @@ __device__ __noinline__ bool diis_step(Ctx& c, const JobDesc& J, bool uhf, bool 
   return iv[0] != 0;
 }
 
+// The numerics of a job: scf_kernel.cuh's, or (kTight) scf_tight.cuh's.
+template <bool kTight>
+struct Numerics {
+  static __device__ __forceinline__ void solve(Ctx& c, const SymInput& in, int kval, int kvec, double* Y, double* lam, double* tri,
+                                               bool warm = false, double* dlam = nullptr) {
+    if constexpr (kTight) tight::eigensolve(c, in, kval, kvec, Y, lam, tri, warm, dlam);
+    else eigensolve(c, in, kval, kvec, Y, lam, tri, warm, dlam);
+  }
+  static __device__ __forceinline__ double density(Ctx& c, const double* Y, int k, double w, const double* Pold, double* Pnew,
+                                                   double damp) {
+    if constexpr (kTight) return tight::density(c, Y, k, w, Pold, Pnew, damp);
+    else return pm3gpu::density(c, Y, k, w, Pold, Pnew, damp);
+  }
+  static __device__ __forceinline__ void all_eigenvalues(int n, const double* tri, double* out, const EigenScratch& s) {
+    if constexpr (kTight) tight::all_eigenvalues(n, tri, tri + n, out, s);
+    else pm3gpu::all_eigenvalues(n, tri, tri + n, out, s);
+  }
+  // The Fock matrices of a density (spins P and Q, or P alone) and twice its electronic energy. `sum`: P + Q where it is at hand,
+  // n^2 doubles to form it in for kTight. G null with Q given (not for kTight): the first spin alone.
+  static __device__ __forceinline__ double fock(Ctx& c, bool uhf, double* sum, const double* P, const double* Q, double* F, double* G) {
+    if constexpr (kTight) return 2.0 * tight::fock_energy(c, uhf, P, Q, sum, F, G);
+    else return uhf ? build_fock(c, sum, P, Q, F, G) : build_fock(c, P, nullptr, nullptr, F, nullptr);
+  }
+};
+
+// One job. kTight: by the numerics of scf_tight.cuh, where no other CTA helps.
+template <bool kTight>
 __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, int jidx = -1) {
   const KernelArgs& A = *c.A;
   c.job = job;
   c.out = out;
   const JobDesc& J = c.job;
+  using Num = Numerics<kTight>;
   c.n = J.nao;
   c.N = J.natom;
   const int n = c.n, tid = threadIdx.x;
@@ -133,10 +162,15 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
   o.pad = 0;
 
   c.tmark = clock64();
-  setup_job(c);
-  o.core = build_core(c);
+  if constexpr (kTight) {
+    tight::setup_job(c);
+    o.core = tight::build_core(c);
+  } else {
+    setup_job(c);
+    o.core = build_core(c);
+  }
   mark(c, kPhCore);
-  if (J.flags & (kJobCoreOnly | kJobFockOnly)) {
+  if (!kTight && (J.flags & (kJobCoreOnly | kJobFockOnly))) {
     double* io = A.densities + J.dens_off;
     if (J.flags & kJobCoreOnly) {
       for (size_t k = tid; k < nn; k += kThreads) io[k] = c.H[k];
@@ -156,9 +190,9 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
   double* Pb = c.Q[0];
   if (J.guess == 2) {  // core-Hamiltonian orbitals, aufbau (scf.rs:929-932, 969-975)
     const int kv = uhf ? na : na;  // na >= nb
-    eigensolve(c, sym_input(c.H, nullptr, 0.0), n < kv + 1 ? n : kv + 1, kv, c.Vt, c.tri_a + 2 * n, nullptr);
-    density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
-    if (uhf) density(c, c.Vt, nb, 1.0, Pb, Pb, 0.0);
+    Num::solve(c, sym_input(c.H, nullptr, 0.0), n < kv + 1 ? n : kv + 1, kv, c.Vt, c.tri_a + 2 * n, nullptr);
+    Num::density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
+    if (uhf) Num::density(c, c.Vt, nb, 1.0, Pb, Pb, 0.0);
   } else if (J.guess == 4) {  // given (learned) density, scaled to the electron count
     const double* G0 = A.guess_dens + J.guess_off;
     double tr = 0.0;
@@ -176,16 +210,12 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
     // The prediction is not an idempotent density, and A-DIIS would treat it as one. One
     // Roothaan step turns it into an aufbau density (as the core guess does with H): its Fock
     // matrix, diagonalised, gives the occupied orbitals the iteration starts from.
-    if (!uhf) {
-      build_fock(c, Pa, nullptr, nullptr, c.F, nullptr);
-    } else {
-      build_fock(c, nullptr, Pa, Pb, c.F, c.G);
-    }
-    eigensolve(c, sym_input(c.F, nullptr, 0.0), n < na + 1 ? n : na + 1, na, c.Vt, c.tri_a + 2 * n, nullptr);
-    density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
+    Num::fock(c, uhf, kTight ? c.Vb + nn : nullptr, Pa, Pb, c.F, c.G);
+    Num::solve(c, sym_input(c.F, nullptr, 0.0), n < na + 1 ? n : na + 1, na, c.Vt, c.tri_a + 2 * n, nullptr);
+    Num::density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pa, Pa, 0.0);
     if (uhf) {
-      eigensolve(c, sym_input(c.G, nullptr, 0.0), n < nb + 1 ? n : nb + 1, nb, c.Vb, c.tri_b + 2 * n, nullptr);
-      density(c, c.Vb, nb, 1.0, Pb, Pb, 0.0);
+      Num::solve(c, sym_input(c.G, nullptr, 0.0), n < nb + 1 ? n : nb + 1, nb, c.Vb, c.tri_b + 2 * n, nullptr);
+      Num::density(c, c.Vb, nb, 1.0, Pb, Pb, 0.0);
     }
   } else {
     double fa = 1.0, fb = 0.0;
@@ -278,18 +308,24 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
       }
     }
     // twice the electronic energy; paired: the helper builds F_beta and returns its part
-    double e_elec = uhf ? build_fock(c, nullptr, Pc, Qc, Fa, paired ? nullptr : Fb)
-                        : build_fock(c, Pc, nullptr, nullptr, Fa, nullptr);
+    double e_elec = Num::fock(c, uhf, kTight ? c.Vb + nn : nullptr, Pc, Qc, Fa, paired ? nullptr : Fb);
     if (!paired) e_elec *= 0.5;
     mark(c, kPhFock);
 
     // ---- accelerator (scf.rs:1240-1259 RHF; 1398-1413 UHF)
     bool use_hist = false;
     if (J.accel != 0) {
-      commutator(c, Fa, Pc, Ea);
-      if (uhf) commutator(c, Fb, Qc, Eb);
-      mark(c, kPhCommutator);
-      use_hist = diis_step(c, J, uhf, keep, len, head, depth, slot_mats, Fa, Fb, Ea, Eb, Dh, Pc);
+      if constexpr (kTight) {
+        tight::commutator(c, Fa, Pc, Ea);
+        if (uhf) tight::commutator(c, Fb, Qc, Eb);
+        mark(c, kPhCommutator);
+        use_hist = tight::diis_step(c, uhf, keep, len, head, depth, slot_mats, Fa, Ea, Eb, Dh, Pc);
+      } else {
+        commutator(c, Fa, Pc, Ea);
+        if (uhf) commutator(c, Fb, Qc, Eb);
+        mark(c, kPhCommutator);
+        use_hist = diis_step(c, J, uhf, keep, len, head, depth, slot_mats, Fa, Fb, Ea, Eb, Dh, Pc);
+      }
       ++len;
       mark(c, kPhDiisSolve);
     }
@@ -309,12 +345,12 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
           in.stride = slot_mats * nn;
         }
         if (spin == 0) {
-          eigensolve(c, in, kva, na, c.Vt, eps_a, c.tri_a, iter > 0, c.tri_a + 3 * n);
-          sq_a = density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pc, Pn, uhf ? J.damping : 0.0);
+          Num::solve(c, in, kva, na, c.Vt, eps_a, c.tri_a, iter > 0, c.tri_a + 3 * n);
+          sq_a = Num::density(c, c.Vt, na, uhf ? 1.0 : 2.0, Pc, Pn, uhf ? J.damping : 0.0);
           mark(c, kPhDensity);
         } else {
-          eigensolve(c, in, kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
-          sq_b = density(c, c.Vb, nb, 1.0, Qc, Qn, J.damping);
+          Num::solve(c, in, kvb, nb, c.Vb, eps_b, c.tri_b, iter > 0, c.tri_b + 3 * n);
+          sq_b = Num::density(c, c.Vb, nb, 1.0, Qc, Qn, J.damping);
           mark(c, kPhDensity);
         }
       }
@@ -358,7 +394,7 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
   double* Qf = c.Q[c.cur];
   double* Pt = Pf;
   if (!uhf) {
-    o.electronic = 0.5 * build_fock(c, Pf, nullptr, nullptr, c.F, nullptr);
+    o.electronic = 0.5 * Num::fock(c, uhf, nullptr, Pf, nullptr, c.F, nullptr);
     o.spin_max = 0.0;
   } else {
     Pt = c.Vb + nn;
@@ -368,7 +404,7 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
       mx = fmax(mx, fabs(Pf[k] - Qf[k]));
     }
     o.spin_max = block_max(mx, c.red);
-    o.electronic = 0.5 * build_fock(c, Pt, Pf, Qf, c.F, c.G);
+    o.electronic = 0.5 * Num::fock(c, uhf, Pt, Pf, Qf, c.F, c.G);
   }
   o.converged = converged ? 1 : 0;
   o.iterations = iterations;
@@ -407,8 +443,8 @@ __device__ void run_job(Ctx& c, const JobDesc& job, JobOut* out, int kind = -1, 
       }
   }
   if (J.flags & kJobEps) {
-    all_eigenvalues(n, c.tri_a, c.tri_a + n, A.eps + J.eps_off, c.es);
-    if (uhf) all_eigenvalues(n, c.tri_b, c.tri_b + n, A.eps + J.eps_off + n, c.es);
+    Num::all_eigenvalues(n, c.tri_a, A.eps + J.eps_off, c.es);
+    if (uhf) Num::all_eigenvalues(n, c.tri_b, A.eps + J.eps_off + n, c.es);
   }
   __syncthreads();
   mark(c, kPhFinal);
@@ -543,7 +579,8 @@ __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
 
 // ----------------------------------------------------------------------- the kernel
 
-__global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args) {
+template <bool kTight>
+__device__ __forceinline__ void scf_batch(const KernelArgs& args) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_job;
   Ctx c;
@@ -553,8 +590,9 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
   int* ip = reinterpret_cast<int*>(smem + L.off_int);
   c.sz = ip;
   c.soff = ip + amax;
-  c.order = ip + 2 * amax;
+  c.order = c.sprow = ip + 2 * amax;
   c.iv = ip + 3 * amax + 1;
+  c.sroff = c.iv + 16;
   double* dp = reinterpret_cast<double*>(smem + L.off_dbl);
   c.sxyz = dp;
   dp += (3 * amax + 1) & ~1;  // the reduction scratch is read 16 bytes at a time
@@ -585,6 +623,8 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
   double* up = reinterpret_cast<double*>(smem + L.off_union);
   c.tile = up;
   c.es.sh = up;
+  c.dpk = up;
+  c.jacc = up + 10 * amax;
 
   slot_ptrs(c, args.work + (size_t)blockIdx.x * args.slot, args.nmax);
 
@@ -672,21 +712,25 @@ __global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args)
     const int kind = s_kind, jid = s_job, hg = s_hgen;
     __syncthreads();
     if (kind < 0) break;
-    if (kind == 2) {
+    if (!kTight && kind == 2) {
       help_job(c, jid, hg);
     } else if (kind == 0) {
-      run_job(c, args.jobs[jid], args.out + jid, 0, jid);
+      run_job<kTight>(c, args.jobs[jid], args.out + jid, 0, jid);
       if (threadIdx.x == 0) {  // after its rungs (if any) are queued
         __threadfence();
         atomicAdd(&q[4], 1);
         if (args.tjob) args.tjob[jid] = globaltimer_ns();
       }
     } else {
-      run_job(c, args.rjobs[jid], args.rout + jid, 1, jid);
+      run_job<kTight>(c, args.rjobs[jid], args.rout + jid, 1, jid);
     }
   }
   if (args.prof && threadIdx.x < kPhases) atomicAdd(&args.prof[threadIdx.x], s_ph[threadIdx.x]);
 }
+
+__global__ void __launch_bounds__(kThreads, 2) scf_batch_kernel(KernelArgs args) { scf_batch<false>(args); }
+// Launches whose every solve asks for second-derivative tolerances (scf_tight.cuh); args.help is null.
+__global__ void __launch_bounds__(kThreads, 2) scf_tight_kernel(KernelArgs args) { scf_batch<true>(args); }
 
 inline long long slot_doubles(int nmax, long long wcap) {
   const long long nn = (long long)nmax * nmax;

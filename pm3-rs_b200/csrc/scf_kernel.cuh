@@ -143,6 +143,7 @@ struct Ctx {
   int* sz;              // [amax] Z of each atom
   int* soff;            // [amax] first AO
   int* order;           // [amax] atoms with p orbitals first, then the others, each in the molecule's order
+  int *sprow, *sroff;   // scf_tight_kernel: [amax + 1] prefix of packed sizes, [amax] pair-table row offsets
   int nh;               // atoms with p orbitals
   double* sxyz;         // [3 amax]
   double* red;          // reduction scratch
@@ -151,6 +152,7 @@ struct Ctx {
   double* mg;           // [8*8] <D_i,F_j>
   double* coef;         // [kMaxDepth+1]
   int* iv;              // small ints
+  double *dpk, *jacc;   // scf_tight_kernel: [10 amax] packed densities, [10 amax] Coulomb accumulators (in the union)
   double* tile;         // the union: GEMM tiles, the Fock build's packed rows, the eigensolver's scratch
   EigenScratch es;
   unsigned long long* ph;  // [kPhases] shared accumulators
@@ -243,10 +245,11 @@ __device__ void setup_job(Ctx& c) {
 }
 
 // One atom pair of H_core (hamiltonian.rs:191-344): both atoms' electron-core attraction blocks
-// (stored to hacc_a, hacc_b), the pair table block W in (a, b) orientation (a
+// (stored to hacc_a, hacc_b; kAdd: added to them atomically), the pair table block W in (a, b) orientation (a
 // the atom with more orbitals; consecutive integrals ws apart), and the resonance block H_ab = (beta_i + beta_j)/2 S_ij written to
 // both triangles of H (row stride n). Returns the pair's core-core energy (repulsion.rs:57-120),
 // evaluated with the atoms in the caller's (u, v) order.
+template <bool kAdd = false>
 __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb, const ElemDev& eu, const ElemDev& ev,
                                             const PairDev& pp, const double* xa, const double* xb, int oa, int ob,
                                             size_t n, double* hacc_a, double* hacc_b, double* w, int ws,
@@ -258,9 +261,15 @@ __device__ __forceinline__ double core_pair(const ElemDev& ea, const ElemDev& eb
   if (hacc_a) {  // null: the caller adds the electron-core blocks per atom itself
     double blk[10];
     core_attraction(ea, eb, dv, blk);
-    for (int k = 0; k < (ea.norb == 4 ? 10 : 1); ++k) hacc_a[k] = blk[k];
+    for (int k = 0; k < (ea.norb == 4 ? 10 : 1); ++k) {
+      if (kAdd) atomicAdd(&hacc_a[k], blk[k]);
+      else hacc_a[k] = blk[k];
+    }
     core_attraction(eb, ea, mdv, blk);
-    for (int k = 0; k < (eb.norb == 4 ? 10 : 1); ++k) hacc_b[k] = blk[k];
+    for (int k = 0; k < (eb.norb == 4 ? 10 : 1); ++k) {
+      if (kAdd) atomicAdd(&hacc_b[k], blk[k]);
+      else hacc_b[k] = blk[k];
+    }
   }
   const double ir = 1.0 / r;
   double R[9];
@@ -658,8 +667,8 @@ __device__ __noinline__ void commutator(Ctx& c, const double* Fm, const double* 
 }
 
 // ------------------------------------------------------------ small dense solves
-// Pulay coefficients from the Gram matrix (scf.rs:1544-1630), on the host; false = singular / unusable.
-inline bool cdiis_coeffs(int m, const double* gram, double* x) {
+// Pulay coefficients from the Gram matrix (scf.rs:1544-1630), on one thread; false = singular / unusable.
+__host__ __device__ inline bool cdiis_coeffs(int m, const double* gram, double* x) {
   if (m < 2) return false;
   double scale = 0.0;
   for (int i = 0; i < m * m; ++i) scale = fmax(scale, fabs(gram[(i / m) * kMaxDepth + i % m]));
