@@ -675,7 +675,8 @@ __device__ __forceinline__ void sturm_multi(const double* __restrict__ d, const 
 // Invariant: count(lo) <= j < count(hi). The points are evenly spaced (the bracket shrinks by P + 1) until
 // the interval holds this eigenvalue alone. From then on they close in geometrically on the
 // secant estimate of the characteristic polynomial's root, whose values the counts yield on the way; the counts
-// still decide, and a step that gained less than a factor of 4 is followed by an even one.
+// still decide, and a step that gained less than a factor of 4 is followed by an even one. The search ends at an interval of
+// 2 eps |lambda|, whatever the norm.
 // What bounds it: the recurrence, about 40 cycles a row and step; steps from a cold start at n = 64, k = 33:
 // 17 when all were even, 9 now.
 // With `prev` (eigenvalue j of the previous SCF iteration) and `dprev` (its last change) the search starts from a
@@ -725,7 +726,7 @@ __device__ __forceinline__ double multisect(const double* __restrict__ d, const 
   for (int it = 0; it < 160; ++it) {
     if (act) {
       const double mid = 0.5 * (lo + hi);
-      if (hi - lo <= eps * (2.0 * fmax(fabs(lo), fabs(hi)) + tnorm) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
+      if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + 4.0 * pivmin || !(mid > lo && mid < hi)) act = false;
     }
     if (!__any_sync(0xffffffffu, act)) break;
     const double w = hi - lo;
@@ -735,7 +736,7 @@ __device__ __forceinline__ double multisect(const double* __restrict__ d, const 
     if (close) {
       const double a = fabs(flo), b = fabs(fhi);  // the one of the smaller scale counts as 0
       const double r = elo == ehi ? a / (a + b) : (elo > ehi ? 1.0 : 0.0);
-      const double xs = lo + w * r, tiny = 0.5 * eps * (fmax(fabs(lo), fabs(hi)) + 0.5 * tnorm);
+      const double xs = lo + w * r, tiny = eps * fmax(fabs(lo), fabs(hi));
 #pragma unroll
       for (int t = 0; t < kPts; ++t) {  // distances w/4 .. w/2^26 (w/16 for P = 2), below and above
         const int q = gl * kPts + t, k = q < g ? q : P - 1 - q;
