@@ -39,3 +39,34 @@ extern "C" int probe_eigenvalues(int n, int kval, const double* d, const double*
   cudaFree(b);
   return rc;
 }
+
+// Largest differences, in units of the last place, of sqrt_newton and rcp_newton from CUDA's square root and division: every
+// exponent from -797 to 796 (1e-240 to 1e239), `each` random mantissas of one and the two ends of the binade.
+__global__ void roots_kernel(int each, unsigned long long* out) {
+  const int ex = (int)blockIdx.x - 797;
+  unsigned long long s = 0x9e3779b97f4a7c15ull * (blockIdx.x * blockDim.x + threadIdx.x + 1), m0 = 0, m1 = 0;
+  for (int i = threadIdx.x; i < each + 4; i += blockDim.x) {
+    s = s * 6364136223846793005ull + 1442695040888963407ull;
+    unsigned long long t = s ^ (s >> 29);
+    t = (t * 0xbf58476d1ce4e5b9ull) >> 12;  // 52 bits
+    if (i < 4) t = i < 2 ? (unsigned long long)i : (1ull << 52) - (unsigned long long)(i - 1);
+    const double x = __longlong_as_double(((long long)(ex + 1023) << 52) | (long long)t);
+    const long long a = __double_as_longlong(sqrt_newton(x)) - __double_as_longlong(sqrt(x));
+    const long long b = __double_as_longlong(rcp_newton(x)) - __double_as_longlong(1.0 / x);
+    m0 = max(m0, (unsigned long long)llabs(a));
+    m1 = max(m1, (unsigned long long)llabs(b));
+  }
+  atomicMax(out, m0);
+  atomicMax(out + 1, m1);
+}
+
+extern "C" int probe_roots(int each, unsigned long long* out) {
+  unsigned long long* b = nullptr;
+  if (cudaMalloc(&b, 16) != cudaSuccess) return 1;
+  cudaMemset(b, 0, 16);
+  roots_kernel<<<797 + 797, 256>>>(each, b);
+  cudaMemcpy(out, b, 16, cudaMemcpyDeviceToHost);
+  const int rc = (int)cudaDeviceSynchronize();
+  cudaFree(b);
+  return rc;
+}

@@ -37,3 +37,11 @@ def test_eigenvalues_to_their_own_last_bits(probe, n, kval):
     assert probe.probe_eigenvalues(n, kval, _p(d), _p(np.zeros(n)), _p(lam)) == 0
     want = np.sort(d)[:kval]
     assert (np.abs(lam - want) <= 2 * EPS * np.abs(want)).all()
+
+
+def test_root_and_reciprocal_of_the_reflectors(probe):
+    """Newton-Raphson from a 20-bit approximation: the last step's fma rounds a value whose error is far below an ulp, so the
+    results are the neighbours of the exact ones and within one unit of CUDA's correctly rounded functions."""
+    worst = (ctypes.c_ulonglong * 2)()
+    assert probe.probe_roots(20000, worst) == 0
+    assert worst[0] <= 1 and worst[1] <= 1, list(worst)
