@@ -320,8 +320,8 @@ int pm3gpu_last_transfer_bytes(pm3gpu_ctx* ctx, long long* h2d, long long* d2h);
 int pm3gpu_last_kernel_launches(pm3gpu_ctx* ctx);
 
 /* Shape of the last batched SCF launch (no counterpart in the reference): CTAs resident per SM and
- * the largest basis size whose eigensolver keeps the matrix in registers and shared memory; larger
- * molecules of that launch keep its first block columns in global memory. */
+ * a basis size up to which the eigensolver keeps the matrix in registers and shared memory (the
+ * layout guarantees it); larger molecules of that launch may keep its first block columns in global memory. */
 int pm3gpu_last_launch_layout(pm3gpu_ctx* ctx, int* ctas_per_sm, int* smem_matrix_n);
 
 /* Molecules with at least `nao` basis functions are solved one at a time on the whole GPU

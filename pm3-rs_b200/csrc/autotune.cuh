@@ -4,7 +4,7 @@
 //
 // Two choices are measured, each between variants that give the same results:
 //   batch  CTAs per SM of the persistent SCF launch. One CTA per SM gives each molecule the
-//          largest shared-memory eigen workspace (the packed matrix of up to ~230 basis functions
+//          largest shared-memory eigen workspace (the matrix of up to 224 basis functions
 //          stays on chip); two CTAs per SM halve it but double the molecules in flight. The
 //          bucket is the batch's largest basis size (the layout is sized for it).
 //   large  the whole-GPU Householder reduction as one cooperative launch per panel or as five

@@ -69,6 +69,11 @@ constexpr int kRegRows = 16 * kRegB;
 __host__ __device__ constexpr int frame_rows(int n) { return n <= kRegRows ? kRegRows : (n + 15) / 16 * 16; }
 // doubles of shared scratch `tridiagonalize` needs for bases up to n (vectors; memory blocks go after them)
 __host__ __device__ constexpr int tri_scratch(int n) { return 15 * frame_rows(n); }
+// the same with every memory block in shared memory: kThreads doubles for each of the (nb - J) blocks of the columns J < nb - kRegB
+__host__ __device__ constexpr int tri_resident(int n) {
+  const int nb = frame_rows(n) / 16, mb = nb - kRegB;
+  return tri_scratch(n) + kThreads * (mb * nb - mb * (mb - 1) / 2);
+}
 
 constexpr int kPart = 10;
 struct TriCtx {

@@ -497,11 +497,13 @@ long long pair_table_doubles(const pm3gpu_ctx* c, const int32_t* z, int natom) {
 // Static shared memory of scf_batch_kernel (set when a context is created).
 int g_scf_static_smem = 1024;
 
-// Shared-memory carve-up of one launch. The packed eigen input lives in shared memory for
-// bases up to `nsm` (global memory above). When `naos` is given, the layout is shrunk to let
-// two CTAs share an SM as long as at least 90% of the launch's jobs still fit in shared memory.
-// ctas: 0 = choose (two CTAs per SM when at least 90% of the batch keeps its packed eigen input
-// in the smaller layout), 1 or 2 = the autotuner's measured choice.
+// Shared-memory carve-up of one launch. For bases up to `nsm` the eigensolver's matrix stays on chip (registers and shared
+// memory); larger ones keep block columns in global memory. When `naos` is given, the layout is shrunk to let
+// two CTAs share an SM as long as at least 90% of the launch's jobs are at most nsm in the smaller layout.
+// ctas: 0 = choose so, 1 or 2 = the autotuner's measured choice.
+// The union holds what the eigensolver takes at nsm (tri_resident), and n (n + 1) / 2 doubles: the packed triangle of
+// scf_tight_kernel, and the measure by which the 90% rule was set. For the common kernel that second term is a margin:
+// at two CTAs and nmax = 252 it ends nsm at 149, where the blocks of sizes up to 160 fit the same union.
 // wcap: doubles of the launch's largest pair table; the union is widened to hold it when two CTAs per SM allow.
 // tight: the layout of scf_tight_kernel, which holds the packed matrix itself.
 SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const std::vector<int>* naos = nullptr,
@@ -518,10 +520,11 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
   off += align(7 * nmax * 8 + (2 * nmax + 2) * 4);
   L.off_union = off;
   const int fixed_union = tight ? std::max(20 * amax, tight::kGemmScratch) : union_keep(nmax);
+  auto matrix = [&](int n) { return std::max(n * (n + 1) / 2, tight ? 0 : tri_resident(n)); };
   auto fit = [&](int budget) {
     int nsm = nmax;
     for (; nsm > 0; --nsm)
-      if (off + std::max(fixed_union, nsm * (nsm + 1) / 2) * 8 <= budget) break;
+      if (off + std::max(fixed_union, matrix(nsm)) * 8 <= budget) break;
     return nsm;
   };
   int nsm = fit(optin);
@@ -539,7 +542,7 @@ SmemLayout make_layout(int amax, int nmax, int optin, int smem_per_sm = 0, const
     }
   }
   L.nsm = nsm;
-  L.uni = std::max(fixed_union, nsm * (nsm + 1) / 2);
+  L.uni = std::max(fixed_union, nsm > 0 ? matrix(nsm) : 0);
   if (smem_per_sm > 0 && wcap > 0 && !tight) {
     const long long want = fixed_union + wcap;
     if (off + want * 8 <= smem_per_sm / 2 - 1024 - g_scf_static_smem) L.uni = std::max(L.uni, (int)want);

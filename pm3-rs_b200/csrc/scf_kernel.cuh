@@ -68,7 +68,7 @@ struct JobOut {
 // Byte offsets of the dynamic shared-memory carve-up (computed on the host).
 struct SmemLayout {
   int amax;      // atoms per molecule this launch supports
-  int nsm;       // largest n whose packed matrix would fit the union
+  int nsm;       // size up to which the eigensolver's matrix is certain to stay on chip (make_layout)
   int uni;       // doubles in the union of the phases' scratch
   int off_int, off_dbl, off_eig, off_union;
   int bytes;
@@ -238,7 +238,7 @@ __device__ void setup_job(Ctx& c) {
   // helpers another CTA may have to read it, from global memory.
   const PairKinds K(c.nh, c.N);
   const int wsize = 100 * K.nhh + 10 * K.nhl + K.nll;
-  const bool near = A.help == nullptr && union_keep(c.n) + wsize <= A.sm.uni;
+  const bool near = A.help == nullptr && max(union_keep(c.n), tri_resident(c.n)) + wsize <= A.sm.uni;
   c.W = near ? c.tile + (A.sm.uni - wsize) : c.Wg;
   c.es.sh_doubles = near ? A.sm.uni - wsize : A.sm.uni;
   __syncthreads();
