@@ -2367,15 +2367,19 @@ int noalloc_run(pm3gpu_ctx* c, int n_atoms, const int32_t* z, const double* xyz,
     c->err = p.msg;
     return p.status;
   }
-  // the whole-GPU algorithm needs allocations: by the context's threshold, or (none set) the size from which
-  // this entry has always left molecules to it
-  const bool lone_whole = !c->large_set && p.nao >= kSingleWholeNao && o->guess != PM3GPU_GUESS_LEARNED;
-  if (p.large || lone_whole) {
+  // Molecules of the whole-GPU path, which needs allocations; and, while no threshold is set, this entry's own limit.
+  if (p.large || (!c->large_set && p.nao >= kSingleWholeNao)) {
     char msg[220];
-    std::snprintf(msg, sizeof msg,
-                  "molecule (nao=%d) is at or above the whole-GPU threshold (%d) of a single-molecule call; the "
-                  "allocation-free path runs only the one-CTA-per-molecule kernel",
-                  p.nao, p.large ? c->large_min : kSingleWholeNao);
+    if (p.large)
+      std::snprintf(msg, sizeof msg,
+                    "molecule (nao=%d) belongs to the whole-GPU path (from %d basis functions here); the "
+                    "allocation-free path runs only the one-CTA-per-molecule kernel",
+                    p.nao, std::min(c->large_min, kMaxN + 1));
+    else
+      std::snprintf(msg, sizeof msg,
+                    "molecule (nao=%d): the allocation-free path takes fewer than %d basis functions while no whole-GPU "
+                    "threshold is set",
+                    p.nao, kSingleWholeNao);
     return fail(c, PM3GPU_RESOURCE_LIMIT, msg);
   }
   // the first pass and the stability rungs run_pm3 would try, in its order (scf.rs:599-715)
