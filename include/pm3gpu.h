@@ -337,12 +337,13 @@ int pm3gpu_set_large_threshold(pm3gpu_ctx* ctx, int nao);
  * (atom_offsets / z / xyz as in pm3gpu_batch), the two launch choices that trade off against each
  * other, and keeps the faster per size bucket in the context: CTAs per SM of the batched SCF
  * launch (bucket: the batch's largest basis size) and, for molecules on the whole-GPU path, the
- * Householder reduction as one cooperative launch per panel or as five launches per column
- * (bucket: basis size). Both variants of each choice give the same results. When cache_path is
+ * Householder reduction in its cooperative form (one launch on register tiles up to 1472, one per panel
+ * beyond) or as five launches per column (bucket: basis size; a choice measured with one cooperative form is not
+ * applied to the sizes of the other). Both variants of each choice give the same results. When cache_path is
  * not NULL the table is written there as JSON; pm3gpu_load_tuning reads such a file into another
  * context (with ctx = NULL it only checks the file and returns its status).
  * pm3gpu_tuning_choice returns the choice a size would get (kind 0: CTAs per SM for a
- * batch whose largest basis is `size`; kind 1: 1 = cooperative panels for basis `size`), or -1
+ * batch whose largest basis is `size`; kind 1: 1 = cooperative for basis `size`), or -1
  * when no tuned bucket covers it. */
 /* What pm3gpu_autotune minimises for the batched launch: PM3GPU_TUNE_BATCH_TIME (default), the time
  * of one whole batch, tail included (one batch at a time); PM3GPU_TUNE_THROUGHPUT, the time until

@@ -7,10 +7,11 @@
 //          largest shared-memory eigen workspace (the matrix of up to 224 basis functions
 //          stays on chip); two CTAs per SM halve it but double the molecules in flight. The
 //          bucket is the batch's largest basis size (the layout is sized for it).
-//   large  the whole-GPU Householder reduction as one cooperative launch per panel or as five
-//          launches per column replayed from a CUDA graph; bucket = basis size.
+//   large  the whole-GPU Householder reduction as one cooperative launch (register tiles) or one per panel, whichever the
+//          size takes, or as five launches per column replayed from a CUDA graph; bucket = basis size, entries of the two
+//          cooperative forms apart ("tiles" in the file).
 // A bucket covers sizes up to its bound; lookups take the smallest tuned bucket that covers the
-// size and fall back to the built-in choice (the 90% rule of make_layout, cooperative panels).
+// size and fall back to the built-in choice (the 90% rule of make_layout, the cooperative reduction).
 
 constexpr int kTuneBatchBuckets[] = {64, 128, 256};  // coarse: a sample and its full batch share a bucket
 constexpr int kTuneLargeBuckets[] = {512, 1024, 2048, 4096, 8192, 16384, 32768, 65536, 131072};
@@ -24,7 +25,7 @@ int tune_bucket(const int (&b)[N], int v) {
 
 void tune_store(std::vector<pm3gpu_ctx::Tune>& t, const pm3gpu_ctx::Tune& e) {
   for (pm3gpu_ctx::Tune& x : t)
-    if (x.le == e.le) {
+    if (x.le == e.le && x.tiles == e.tiles) {
       x = e;
       return;
     }
@@ -93,14 +94,14 @@ int tune_batch_part(pm3gpu_ctx* c, int n_mol, const int32_t* offs, const int32_t
 // The reduction choice for each size bucket met by the sample's large molecules (first molecule
 // per bucket): one Householder reduction of its H_core per candidate.
 int tune_large_part(pm3gpu_ctx* c, int n_mol, const int32_t* offs, const int32_t* z, const double* xyz) {
-  std::vector<int> done;
+  std::vector<std::pair<int, int>> done;
   for (int m = 0; m < n_mol; ++m) {
     const int na = offs[m + 1] - offs[m];
     const int nao = tune_nao(c, z + offs[m], na);
     if (nao < c->large_min || nao < 3) continue;
-    const int b = tune_bucket(kTuneLargeBuckets, nao);
-    if (std::find(done.begin(), done.end(), b) != done.end()) continue;
-    done.push_back(b);
+    const int b = tune_bucket(kTuneLargeBuckets, nao), tiles = tile_sized(c, nao) ? 1 : 0;
+    if (std::find(done.begin(), done.end(), std::make_pair(b, tiles)) != done.end()) continue;
+    done.push_back({b, tiles});
     CUDA_TRY(c, dgemm_ready(c->device));
     if (!c->lbuf) c->lbuf = new LargeBufs();
     CUDA_TRY(c, c->z.ensure(4 * (size_t)na));
@@ -114,7 +115,7 @@ int tune_large_part(pm3gpu_ctx* c, int n_mol, const int32_t* offs, const int32_t
     if (rc == PM3GPU_OK) rc = S.time_reduction(0, &t_multi);
     c->force_coop = -1;
     if (rc != PM3GPU_OK) return rc;
-    tune_store(c->tune_large, {b, t_coop <= t_multi ? 1 : 0, t_coop, t_multi});
+    tune_store(c->tune_large, {b, t_coop <= t_multi ? 1 : 0, t_coop, t_multi, tiles});
   }
   return PM3GPU_OK;
 }
@@ -134,8 +135,8 @@ int write_tuning(pm3gpu_ctx* c, const char* path) {
   std::fprintf(f, "\n  ],\n  \"large\": [");
   for (size_t k = 0; k < c->tune_large.size(); ++k) {
     const pm3gpu_ctx::Tune& e = c->tune_large[k];
-    std::fprintf(f, "%s\n    {\"n_le\": %d, \"coop\": %d, \"ms_coop\": %.6f, \"ms_multi\": %.6f}", k ? "," : "", e.le,
-                 e.choice, e.ms_a, e.ms_b);
+    std::fprintf(f, "%s\n    {\"n_le\": %d, \"tiles\": %d, \"coop\": %d, \"ms_coop\": %.6f, \"ms_multi\": %.6f}", k ? "," : "",
+                 e.le, e.tiles, e.choice, e.ms_a, e.ms_b);
   }
   std::fprintf(f, "\n  ]\n}\n");
   const bool ok = std::fclose(f) == 0;
@@ -181,7 +182,10 @@ int read_tuning(pm3gpu_ctx* c, const char* path) {
       num("ms_coop", &a);
       num("ms_multi", &b);
       if (ch != 0.0 && ch != 1.0) return fail(c, PM3GPU_INVALID_INPUT, "tuning file: coop must be 0 or 1");
-      tl.push_back({(int)le, (int)ch, a, b});
+      double tiles = 0.0;  // not there in older files: panels
+      num("tiles", &tiles);
+      if (tiles != 0.0 && tiles != 1.0) return fail(c, PM3GPU_INVALID_INPUT, "tuning file: tiles must be 0 or 1");
+      tl.push_back({(int)le, (int)ch, a, b, (int)tiles});
     }
   }
   if (tb.empty() && tl.empty()) return fail(c, PM3GPU_INVALID_INPUT, std::string("no tuning entries in ") + path);

@@ -542,7 +542,7 @@ class LargeSolver {
     return eigenvalues(n_, out, none, false);
   }
 
-  // Autotuner: device time of one Householder reduction of H_core with the cooperative panels
+  // Autotuner: device time of one Householder reduction of H_core in the cooperative form of its size
   // (coop = 1) or the multi-launch path (coop = 0); the second of two runs is timed.
   int time_reduction(int coop, double* ms) {
     int rc = prepare_reduction();
@@ -787,12 +787,16 @@ class LargeSolver {
     return PM3GPU_OK;
   }
 
+  // Whether this matrix takes a cooperative reduction: the switch, and what was measured or is being measured for its size.
+  bool cooperative() const {
+    return c_->coop_panels && (c_->force_coop >= 0 ? c_->force_coop : tune_large_lookup(c_, n_, 1)) != 0;
+  }
+
   // Grid of the cooperative panel kernel for this matrix size, 0 when the multi-launch path runs
   // instead (no cooperative launch, PM3GPU_COOP_PANELS=0, or more 64-row stripes than blocks:
   // each block owns one stripe).
   int coop_grid() {
-    if (!c_->coop_panels) return 0;
-    if ((c_->force_coop >= 0 ? c_->force_coop : tune_lookup(c_->tune_large, n_, 1)) == 0) return 0;
+    if (!cooperative()) return 0;
     if (coop_g_ < 0) {
       int occ = 0, coop = 0;
       if (cudaFuncSetAttribute(large::panel_coop_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -818,21 +822,21 @@ class LargeSolver {
   static constexpr int kCoopSmallN = 512;  // at most 8 stripes of 64 rows
 
   // Grid of the register-tile reduction (tile_reduce.cuh), 0 when the matrix has more tiles than can be resident (two CTAs per
-  // SM: n > 1472 on 148 SMs) or the cooperative reductions are off. Up to there it beats the panels at every size
-  // (n = 966: 4.6 against 12.7 ms).
+  // SM: n > 1472 on 148 SMs), the device has no cooperative launch, or the tiles (PM3GPU_TILE_REDUCE=0) or the cooperative
+  // reductions are off. Up to there it beats the panels at every size (n = 966: 4.6 against 12.7 ms).
   int tile_grid() {
-    if (n_ < 3 || coop_grid() <= 0) return 0;
+    if (!tile_sized(c_, n_) || !cooperative()) return 0;
     if (tile_g_ < 0) {
-      int occ = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large::tile_reduce_kernel, large::kBlock, 0) != cudaSuccess) {
+      int occ = 0, coop = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large::tile_reduce_kernel, large::kBlock, 0) != cudaSuccess ||
+          cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c_->device) != cudaSuccess) {
         (void)cudaGetLastError();
-        occ = 0;
+        occ = coop = 0;
       }
-      tile_g_ = std::min(occ, 2) * c_->sms;
+      tile_g_ = coop ? std::min(occ, 2) * c_->sms : 0;
     }
-    const int nts = large::tile_stripes(n_);
-    const long long tiles = (long long)nts * (nts + 1) / 2;
-    return nts <= large::kTileMaxStripes && tiles <= tile_g_ ? (int)tiles : 0;
+    const int nts = large::tile_stripes(n_), tiles = nts * (nts + 1) / 2;
+    return tiles <= tile_g_ ? tiles : 0;
   }
   // The barrier record of the reduction that run_tridiag takes, null for the multi-launch one.
   const void* reduction_sync() { return tile_grid() > 0 ? B_.tsync.p : (coop_grid() > 0 ? B_.gsync.p : nullptr); }

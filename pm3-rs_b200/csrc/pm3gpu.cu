@@ -125,13 +125,15 @@ struct pm3gpu_ctx {
   // autotuner: measured choices per size bucket (autotune.cuh); forced values while it measures
   struct Tune {
     int le;      // bucket: largest basis size it covers
-    int choice;  // batch: CTAs per SM (1 or 2); large: 1 cooperative panels, 0 multi-launch
+    int choice;  // batch: CTAs per SM (1 or 2); large: 1 cooperative, 0 multi-launch
     double ms_a, ms_b;  // measured times of the two candidates (batch: 1 and 2 CTAs; large: coop, multi)
+    int tiles = 0;      // large: the cooperative candidate was the register-tile reduction (1) or the panels (0)
   };
   std::vector<Tune> tune_batch, tune_large;
   int force_ctas = 0, force_coop = -1;
   int precision = PM3GPU_PRECISION_FP64;  // arithmetic of the whole-GPU path's dense products
-  bool coop_panels = true;    // Householder panels as cooperative launches (PM3GPU_COOP_PANELS=0: off)
+  bool coop_panels = true;    // Householder reduction as cooperative launches (PM3GPU_COOP_PANELS=0: off)
+  bool tile_reduce = true;    // on register tiles where the size allows (PM3GPU_TILE_REDUCE=0: panels)
   std::vector<double> ltrace;  // per-iteration record of the last whole-GPU solve (5 per row)
   DevBuf tcbuf[7];             // pm3gpu_split_gemm: A, B (FP64), A hi / lo, B hi / lo, C; tcerr (pm3gpu_dgemm: A, B, C, split-K work)
   bool large_checks = false;   // whole-GPU path: eigen residual of every eigensolve (one more DGEMM)
@@ -154,6 +156,22 @@ namespace {
 int tune_lookup(const std::vector<pm3gpu_ctx::Tune>& t, int size, int dflt) {
   for (const pm3gpu_ctx::Tune& e : t)
     if (size <= e.le) return e.choice;
+  return dflt;
+}
+
+// Sizes that the register-tile reduction takes (tile_reduce.cuh) when it is on.
+bool tile_sized(const pm3gpu_ctx* c, int n) {
+  const long long nts = large::tile_stripes(n);
+  return c->tile_reduce && n >= 3 && nts <= large::kTileMaxStripes && nts * (nts + 1) / 2 <= 2LL * c->sms;
+}
+
+// The cooperative (1) or multi-launch (0) reduction for a matrix of n: the smallest tuned bucket that covers n and
+// was measured with the form that n takes. One measured with the panels (every entry of a file older than the tiles) says nothing
+// about the sizes on tiles, and the other way round.
+int tune_large_lookup(const pm3gpu_ctx* c, int n, int dflt) {
+  const int tiles = tile_sized(c, n) ? 1 : 0;
+  for (const pm3gpu_ctx::Tune& e : c->tune_large)
+    if (n <= e.le && e.tiles == tiles) return e.choice;
   return dflt;
 }
 
@@ -1560,6 +1578,8 @@ int pm3gpu_context_create(int device, pm3gpu_ctx** out) {
     c->profile = pe && pe[0] && pe[0] != '0';
     const char* pc = std::getenv("PM3GPU_COOP_PANELS");
     c->coop_panels = !(pc && pc[0] == '0');
+    const char* pt = std::getenv("PM3GPU_TILE_REDUCE");
+    c->tile_reduce = !(pt && pt[0] == '0');
   }
   if ((e = c->elem.ensure(sizeof(c->h_elem))) != cudaSuccess) return bail(e);
   if ((e = c->pairs.ensure(sizeof(PairDev))) != cudaSuccess) return bail(e);
@@ -2151,7 +2171,7 @@ int pm3gpu_tuning_choice(pm3gpu_ctx* c, int kind, int size) {
   if (!c) return -1;
   std::lock_guard<std::mutex> lk(c->mu);
   if (kind == 0) return tune_lookup(c->tune_batch, size, -1);
-  if (kind == 1) return tune_lookup(c->tune_large, size, -1);
+  if (kind == 1) return tune_large_lookup(c, size, -1);
   return -1;
 }
 
