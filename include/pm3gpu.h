@@ -254,7 +254,8 @@ int pm3gpu_optimize_batch(pm3gpu_ctx* ctx, int n_mol, const int32_t* atom_offset
  * reference's numerical_hessian (src/hessian.rs:268-319). Column j of molecule m is
  * (g(x + step e_j) - g(x - step e_j)) / (2 step) with j = 3 * atom + axis, then the matrix is averaged
  * with its transpose. The SCF is tightened as the reference does for second derivatives
- * (src/hessian.rs:169-175: e_tol <= 1e-12 eV, p_tol <= 1e-11, max_scf >= 500). Every displaced
+ * (src/hessian.rs:169-175: e_tol <= 1e-12 eV, p_tol <= 1e-11, max_scf >= 500), and such solves run on sums of their own, so
+ * that the values, which depend on the path of the SCFs to about 4e-9 relative, stay what they were. Every displaced
  * geometry of every molecule runs in the batched SCF + gradient launch. hessians receives each
  * molecule's (3 n_m) x (3 n_m) row-major block in eV/Bohr^2, packed molecule after molecule;
  * status[m] is PM3GPU_OK or the run_pm3 status of the molecule's first failing displacement (its
@@ -328,7 +329,8 @@ int pm3gpu_last_launch_layout(pm3gpu_ctx* ctx, int* ctas_per_sm, int* smem_matri
  * (grid-wide integral and Fock kernels, blocked eigensolver, the library's FP64 tensor-core GEMM for
  * the dense products) instead of one CTA each. Default and maximum 257: every molecule beyond one CTA's
  * 256 basis functions; by default a call with a single molecule also sends it there from 192 basis
- * functions when mixed precision or the eigensolver checks are on (setting a threshold replaces that rule). Lower values send
+ * functions when mixed precision or the eigensolver checks are on, or under second-derivative tolerances
+ * (e_tol <= 1e-12, p_tol <= 1e-11, max_scf >= 500); setting a threshold replaces that rule. Lower values send
  * smaller molecules to that path too (one molecule at a time, all SMs on it). Same run_pm3
  * semantics either way (no reference counterpart: the reference has one CPU path). */
 int pm3gpu_set_large_threshold(pm3gpu_ctx* ctx, int nao);

@@ -62,8 +62,10 @@ struct EigenScratch {
 // partial sums of A x, forms w, and applies the column's update to the next column in advance (its
 // old values were published with the partial sums), so that the next reflector is known when the
 // rest of the matrix is updated.
-// What bounds it: the chain of two barriers, shuffles and shared-memory round trips up to
-// n = 64 or so (about 1500 cycles a column), FP64 issue above (4 FMAs per element and column).
+// What bounds it: latency, the chain of two barriers, shuffles and shared-memory round trips that 8 warps a CTA do not hide:
+// about 1500 cycles a column up to n = 64 or so; at n = 112 2.2k alone and 3.0k with two CTAs on the SM, where the four
+// FMAs an element and column are 131 cycles of the FP64 pipe (5.8 % busy over a launch). Beyond 112 the memory blocks' traffic adds to it
+// (n = 148: 4.9k).
 constexpr int kRegB = 7;                        // block columns held in registers: 28 values a thread
 constexpr int kRegRows = 16 * kRegB;
 __host__ __device__ constexpr int frame_rows(int n) { return n <= kRegRows ? kRegRows : (n + 15) / 16 * 16; }
@@ -973,7 +975,7 @@ __device__ double* tridiag_vectors(int n, int kvec, double* tf, const EigenScrat
     for (int g = share; lo + 8 * g <= hi; g += shares) {
       const int t0 = 8 * g + (g > 0 ? 1 : 0), t1 = min(8 * g + 8, hi - lo);  // rows t0 .. t1 of the block
       const int ef = EF[g * kvec + j];
-      // g's rows hi - i: at most three of its groups meet nine rows
+      // g's rows hi - i: nine consecutive rows meet at most two of its groups
       const int gb = max(hi - lo - t1 - 1, 0) >> 3;
       const int e0 = EG[gb * kvec + j], e1 = EG[min(gb + 1, (n + 7) / 8 - 1) * kvec + j];
       double p[9];

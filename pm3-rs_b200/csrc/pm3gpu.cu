@@ -1206,9 +1206,11 @@ int run_batch(pm3gpu_ctx* c, int n_mol, const int32_t* h_offs, const int32_t* h_
     if (na < 0) return fail(c, PM3GPU_INVALID_INPUT, "atom_offsets must be non-decreasing");
     const pm3gpu_options* o = per_mol ? opts + m : opts;
     plan_molecule(c, h_z + p.atom0, h_xyz ? h_xyz + 3 * (size_t)p.atom0 : nullptr, na, o, p);
-    // A lone molecule finishes sooner on the one CTA the batched kernel gives it than on all SMs, whose grid barriers cost more than
-    // they spread, over that kernel's whole range (n = 204: 23 against 45 ms; n = 252: 44 against 60). The whole-GPU
-    // path still takes it where only that path has what was asked for.
+    // A lone molecule stays on the one CTA the batched kernel gives it, over that kernel's whole range. The other side is near from
+    // 192 on (one CTA against all SMs, ms: n = 192 17.3 and 17.7, 204 21.6 and 19.5, 228 29.9 and 21.3, 252 43.2 and 24.9;
+    // unrestricted 199 77 and 85, 211 93 and 93, 247 149 and 104): below about 200 one CTA is ahead, above it all SMs. The
+    // whole-GPU path takes it where only that path has what was asked for, and under second-derivative tolerances, whose
+    // kernel is slower still (180 ms at 252).
     if (n_mol == 1 && !c->large_set && p.status == PM3GPU_OK && !p.large && p.nao >= kSingleWholeNao &&
         o->guess != PM3GPU_GUESS_LEARNED &&
         (c->precision == PM3GPU_PRECISION_MIXED || c->large_checks || second_derivative_tolerances(*o)))

@@ -491,7 +491,7 @@ __device__ __forceinline__ void slot_ptrs(Ctx& c, double* slot, int nmax) {
 // CTA), iteration by iteration on L's workspace: F_beta = H + J(P_t) - K(P_beta), its eigensolve
 // (warm-started from L's saved beta eigenvalues) and the new P_beta, then the energy part and the
 // squared density change for L, which decides convergence. Own shared memory and own scratch
-// (packed eigen input, eigenvector scratch, total density) stay with this CTA. Every wait is
+// (reflectors, eigenvectors and their scratch) stay with this CTA. Every wait is
 // bounded; a wait that runs out raises the launch's error flag.
 __device__ __noinline__ void help_job(Ctx& c, int L, int mygen) {
   const KernelArgs& A = *c.A;
