@@ -6,9 +6,10 @@
 // passes or fails by their rounding: where it passes the state lands within 1e-15, where it fails the iteration stops with
 // up to 1e-11 left. So another order of the same sums is another Hessian. scf_kernel.cuh's sums moved those of an 8-atom organic
 // by up to 1.8e-9 relative (24 geometries, 7 of them beyond 1e-9); those kept here, every product, reduction and division in its
-// order and form, give them back to 2e-12. Molecules of up to 32 atom pairs (one warp's) repeat to 1e-14; with more, the order of the atomic
-// sums between warps varies, and two runs of an 11-atom molecule differ by up to 3e-9. The cost: 5.4 ms against 3.1 for three
-// molecules of 8-14 atoms (198 solves).
+// order and form, give them back to 2e-12. The dipole derivatives of the same molecule moved by up to 1.2e-6 and are equal
+// again. Molecules of up to 32 atom pairs (one warp's) repeat to 1e-14; with more, the order of the atomic sums between warps
+// varies, and two runs of an 11-atom molecule differ by up to 3e-9. The cost: 5.4 ms against 3.1 for three molecules of 8-14 atoms
+// (198 solves).
 //
 // The eigensolver is the same chain as in cta_eigen.cuh (Householder, multisection, twisted vectors, back-transformation) on a
 // packed lower triangle (row-major: element (r, c), r >= c, at r(r+1)/2 + c) in shared memory, or in global memory when it does not fit.

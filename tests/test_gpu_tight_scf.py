@@ -35,6 +35,16 @@ def test_hessians_keep_their_values(k):
     assert np.linalg.norm(got - ref) < 1e-10 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("k", range(len(KEPT)))
+def test_dipole_derivatives_keep_their_values(k):
+    """The same for the dipole, whose rounding (charges of a few e Bohr, 1e-15 each) over 2e-3 Bohr is 1e-12."""
+    z, xyz = np.array(KEPT[k]["z"], np.int32), np.array(KEPT[k]["xyz_bohr"])
+    with open(os.path.join(os.path.dirname(__file__), "golden", "dipole_derivatives_8_atoms.json")) as f:
+        ref = np.array(json.load(f)["derivatives"][k])
+    got = native.dipole_derivatives_batch(np.array([0, len(z)], np.int32), z, xyz)["derivatives"][0]
+    assert np.linalg.norm(got - ref) < 1e-10 * np.linalg.norm(ref)
+
+
 def _check(res, m, z, xyz_bohr, **opts):
     ref = O.single_point(z, xyz_bohr, **opts)
     assert res.status[m] == 0 and res.unrestricted[m] == ref["unrestricted"]
